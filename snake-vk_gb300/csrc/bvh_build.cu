@@ -419,22 +419,59 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 }
 
 // ---- treelet restructuring -----------------------------------------------------
+// Bound by latency: a climb towards the root is a chain of treelets, each of which
+// waits for the one below it (about 20 on the way up a 131,072-triangle tree).  So a
+// warp works one treelet out with all its lanes and as few dependent loads as there
+// are levels in it: lane k holds treelet leaf k (box, cost, count, children), an
+// opened leaf's two children are fetched by two lanes at once, the subsets of each
+// size are costed one per lane (four lanes share a subset of six leaves), and the
+// six rewritten nodes are stored by six lanes.  Subtrees below seven primitives only
+// need their cost, which each lane works out for its own node.
 constexpr int TL_LEAVES = 7;
 constexpr int TL_SUBSETS = 1 << TL_LEAVES;
 constexpr int TL_WARPS = BLK / 32;
 constexpr float SAH_CI = 1.2f;   // binary internal node
 constexpr float SAH_CT = 1.0f;   // primitive
 
+// the subsets of 2 to 6 treelet leaves, by size
+struct SubsetTable { uint8_t v[120]; };
+constexpr SubsetTable make_subsets() {
+    SubsetTable t{};
+    int n = 0;
+    for (int size = 2; size <= 6; size++)
+        for (int s = 1; s < TL_SUBSETS; s++) {
+            int c = 0;
+            for (int k = 0; k < TL_LEAVES; k++) c += (s >> k) & 1;
+            if (c == size) t.v[n++] = (uint8_t)s;
+        }
+    return t;
+}
+__device__ const SubsetTable TL_SUBS = make_subsets();
+constexpr int TL_AT2 = 0, TL_AT3 = 21, TL_AT4 = 56, TL_AT5 = 91, TL_AT6 = 112;   // 21, 35, 35, 21 and 7 subsets
+
+// the subsets a lane works out (0: none): one or two of each size, a quarter of one of size 6
+struct TreeletLane { uint32_t s2, s3, s3b, s4, s4b, s5, s6; };
+__device__ __forceinline__ TreeletLane treelet_lane() {
+    const int lane = threadIdx.x & 31;
+    const uint8_t* v = TL_SUBS.v;
+    TreeletLane t;
+    t.s2 = lane < 21 ? __ldg(v + TL_AT2 + lane) : 0u;
+    t.s3 = __ldg(v + TL_AT3 + lane);
+    t.s3b = lane < 3 ? __ldg(v + TL_AT3 + 32 + lane) : 0u;
+    t.s4 = __ldg(v + TL_AT4 + lane);
+    t.s4b = lane < 3 ? __ldg(v + TL_AT4 + 32 + lane) : 0u;
+    t.s5 = lane < 21 ? __ldg(v + TL_AT5 + lane) : 0u;
+    t.s6 = lane < 28 ? __ldg(v + TL_AT6 + (lane >> 2)) : 0u;
+    return t;
+}
+
 struct TreeletSmem {
     float area[TL_SUBSETS];
     float cost[TL_SUBSETS];
     uint32_t count[TL_SUBSETS];
     uint8_t part[TL_SUBSETS];
-    float4 lo[TL_LEAVES], hi[TL_LEAVES];
-    float leaf_cost[TL_LEAVES];
-    uint32_t leaf_cnt[TL_LEAVES];
+    float4 lo[TL_LEAVES], hi[TL_LEAVES];   // leaf boxes (lo.w: cost, hi.w: primitive count)
     int leaf[TL_LEAVES];
-    int inner[TL_LEAVES - 1];
 };
 
 // subtrees of at most leaf_max primitives become leaves of the wide BVH
@@ -442,181 +479,240 @@ __device__ __forceinline__ float node_cost(float area, uint32_t cnt, float split
     return cnt <= leaf_max ? SAH_CT * area * (float)cnt : SAH_CI * area + split_cost;
 }
 
-// Optimises the treelet rooted at `root` (all 32 lanes of the warp call this).
+// The best of the PARTS unordered 2-partitions of subset sub (the part that holds its
+// lowest leaf is enumerated, from the largest down: of equal costs the lowest part wins)
+template <int PARTS>
+__device__ __forceinline__ void treelet_subset(TreeletSmem& T, uint32_t sub, uint32_t leaf_max) {
+    if (sub == 0u) return;
+    const uint32_t low = sub & (0u - sub), rest = sub ^ low;
+    uint32_t q = (rest - 1u) & rest, bp = low | q;
+    float best = T.cost[bp] + T.cost[sub ^ bp];
+#pragma unroll
+    for (int i = 1; i < PARTS; i++) {
+        q = (q - 1u) & rest;
+        const uint32_t P = low | q;
+        const float c = T.cost[P] + T.cost[sub ^ P];
+        if (c <= best) { best = c; bp = P; }
+    }
+    T.cost[sub] = node_cost(T.area[sub], T.count[sub], best, leaf_max);
+    T.part[sub] = (uint8_t)bp;
+}
+
+// minimum of (cost, part) over the lanes that differ in the lane bits up to `lanes`
+__device__ __forceinline__ void treelet_min(float& best, uint32_t& bp, int lanes) {
+    for (int o = lanes >> 1; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+        const uint32_t op = __shfl_xor_sync(0xFFFFFFFFu, bp, o);
+        if (ob < best || (ob == best && op < bp)) { best = ob; bp = op; }
+    }
+}
+
+// Optimises the treelet rooted at `root`, a subtree of at least TL_LEAVES primitives
+// (all 32 lanes of the warp call this).  Internal nodes have ids below nl.
 template <bool G>
 __device__ void treelet_optimise(int root, int nl, int2* children, int* parent, float4* node_lo, float4* node_hi,
-                                 uint32_t* leaf_count, float* cost, TreeletSmem& T, uint32_t leaf_max) {
+                                 uint32_t* leaf_count, float* cost, TreeletSmem& T, const TreeletLane& mine,
+                                 uint32_t leaf_max) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
-    const uint32_t total = ldx<G>(&leaf_count[root]);
-    if (total < (uint32_t)TL_LEAVES) {
-        // small subtree: only its cost (boxes and counts are already final)
-        if (lane == 0) {
-            int2 ch = ldx<G>(&children[root]);
-            float c = ldx<G>(&cost[ch.x]) + ldx<G>(&cost[ch.y]);
-            cost[root] = node_cost(half_area(ldx<G>(&node_lo[root]), ldx<G>(&node_hi[root])), total, c, leaf_max);
-        }
-        __syncwarp();
-        return;
+    // grow: open the largest treelet leaf until there are seven.  A leaf's children are
+    // fetched with its box, so each step waits for one round of loads.
+    int id = 0, inner = root;   // lane k: treelet leaf k / internal node k
+    float area = 0.0f;
+    int2 ch = make_int2(0, 0);
+    float4 lo, hi;
+    auto fetch = [&](int c) {
+        id = c;
+        lo = ldx<G>(&node_lo[c]);
+        hi = ldx<G>(&node_hi[c]);
+        const float k = ldx<G>(&cost[c]);
+        const uint32_t n = ldx<G>(&leaf_count[c]);
+        if (c < nl) ch = ldx<G>(&children[c]);
+        area = half_area(lo, hi);
+        lo.w = k;
+        hi.w = __uint_as_float(n);
+    };
+    const int2 rc = ldx<G>(&children[root]);
+    if (lane < 2) fetch(lane == 0 ? rc.x : rc.y);
+#pragma unroll
+    for (int nleaf = 2; nleaf < TL_LEAVES; nleaf++) {
+        // (a subtree of >= 7 primitives always has an internal node to open; areas are >= 0)
+        const unsigned key = (lane < nleaf && id < nl) ? __float_as_uint(area) + 1u : 0u;
+        const unsigned mx = __reduce_max_sync(FULL, key);
+        const int best = __ffs(__ballot_sync(FULL, key == mx)) - 1;
+        const int bx = __shfl_sync(FULL, ch.x, best), by = __shfl_sync(FULL, ch.y, best);
+        const int opened = __shfl_sync(FULL, id, best);
+        if (lane == nleaf - 1) inner = opened;
+        if (lane == best || lane == nleaf) fetch(lane == best ? bx : by);
     }
-    if (lane == 0) {
-        int2 ch = ldx<G>(&children[root]);
-        int L[TL_LEAVES];
-        float A[TL_LEAVES];
-        L[0] = ch.x; L[1] = ch.y;
-        A[0] = half_area(ldx<G>(&node_lo[ch.x]), ldx<G>(&node_hi[ch.x]));
-        A[1] = half_area(ldx<G>(&node_lo[ch.y]), ldx<G>(&node_hi[ch.y]));
-        T.inner[0] = root;
-        int nleaf = 2, ninner = 1;
-        while (nleaf < TL_LEAVES) {
-            int best = -1;
-            float ba = -1.0f;
-            for (int k = 0; k < nleaf; k++)
-                if (L[k] < nl && A[k] > ba) { ba = A[k]; best = k; }
-            // (a subtree of >= 7 primitives always has an internal node to open)
-            int2 c2 = ldx<G>(&children[L[best]]);
-            T.inner[ninner++] = L[best];
-            L[best] = c2.x;
-            A[best] = half_area(ldx<G>(&node_lo[c2.x]), ldx<G>(&node_hi[c2.x]));
-            L[nleaf] = c2.y;
-            A[nleaf] = half_area(ldx<G>(&node_lo[c2.y]), ldx<G>(&node_hi[c2.y]));
-            nleaf++;
-        }
-        for (int k = 0; k < TL_LEAVES; k++) {
-            T.leaf[k] = L[k];
-            T.lo[k] = ldx<G>(&node_lo[L[k]]);
-            T.hi[k] = ldx<G>(&node_hi[L[k]]);
-            T.leaf_cost[k] = ldx<G>(&cost[L[k]]);
-            T.leaf_cnt[k] = ldx<G>(&leaf_count[L[k]]);
-        }
+    if (lane < TL_LEAVES) {
+        T.lo[lane] = lo;
+        T.hi[lane] = hi;
+        T.leaf[lane] = id;
     }
     __syncwarp();
-    // subset areas and primitive counts
-    for (int sub = lane + 1; sub < TL_SUBSETS; sub += 32) {
-        float4 lo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), hi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
+    // areas and primitive counts of the subsets lane + 32 h: the union of the leaves
+    // 0..4 in `lane`, then with leaf 5, leaf 6 and both
+    {
+        float4 a = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), z = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
         uint32_t cnt = 0;
-        for (int k = 0; k < TL_LEAVES; k++) {
-            if (!(sub & (1 << k))) continue;
-            float4 a = T.lo[k], b = T.hi[k];
-            lo.x = fminf(lo.x, a.x); lo.y = fminf(lo.y, a.y); lo.z = fminf(lo.z, a.z);
-            hi.x = fmaxf(hi.x, b.x); hi.y = fmaxf(hi.y, b.y); hi.z = fmaxf(hi.z, b.z);
-            cnt += T.leaf_cnt[k];
+        auto add = [&](int k) {
+            const float4 l = T.lo[k], h = T.hi[k];
+            a.x = fminf(a.x, l.x); a.y = fminf(a.y, l.y); a.z = fminf(a.z, l.z);
+            z.x = fmaxf(z.x, h.x); z.y = fmaxf(z.y, h.y); z.z = fmaxf(z.z, h.z);
+            cnt += __float_as_uint(h.w);
+        };
+#pragma unroll
+        for (int k = 0; k < 5; k++)
+            if ((lane >> k) & 1) add(k);
+        const float4 a0 = a, z0 = z;
+        const uint32_t c0 = cnt;
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            a = a0; z = z0; cnt = c0;
+            if (h & 1) add(5);
+            if (h & 2) add(6);
+            const int sub = lane + 32 * h;
+            T.area[sub] = half_area(a, z);
+            T.count[sub] = cnt;
+            if (__popc(sub) == 1) T.cost[sub] = T.lo[__ffs(sub) - 1].w;
         }
-        T.area[sub] = half_area(lo, hi);
-        T.count[sub] = cnt;
-        if (__popc(sub) == 1) { T.cost[sub] = T.leaf_cost[__ffs(sub) - 1]; T.part[sub] = 0; }
     }
     __syncwarp();
-    // subsets of 2..6 leaves, by size; every unordered 2-partition (the part that
-    // holds the lowest leaf is enumerated)
-    for (int size = 2; size < TL_LEAVES; size++) {
-        for (int sub = lane + 1; sub < TL_SUBSETS; sub += 32) {
-            if (__popc(sub) != size) continue;
-            const int low = sub & -sub, rest = sub ^ low;
-            float best = 3.4e38f;
-            int bp = 0;
-            // P = low | q over the proper subsets q of rest (q = rest would be all of sub)
-            for (int q = (rest - 1) & rest;; q = (q - 1) & rest) {
-                const int P = low | q;
-                float c = T.cost[P] + T.cost[sub ^ P];
-                if (c < best || (c == best && P < bp)) { best = c; bp = P; }
-                if (q == 0) break;
+    treelet_subset<1>(T, mine.s2, leaf_max);
+    __syncwarp();
+    treelet_subset<3>(T, mine.s3, leaf_max);
+    treelet_subset<3>(T, mine.s3b, leaf_max);
+    __syncwarp();
+    treelet_subset<7>(T, mine.s4, leaf_max);
+    treelet_subset<7>(T, mine.s4b, leaf_max);
+    __syncwarp();
+    treelet_subset<15>(T, mine.s5, leaf_max);
+    __syncwarp();
+    {   // size 6: lanes 4 j .. 4 j + 3 share subset j's 31 partitions
+        const uint32_t sub = mine.s6;
+        float best = 3.4e38f;
+        uint32_t bp = 0xFFFFFFFFu;
+        if (sub) {
+            const int gap = __ffs(sub ^ (TL_SUBSETS - 1)) - 1;   // the leaf it leaves out
+            const uint32_t low = gap == 0 ? 2u : 1u, keep = gap == 0 ? 0u : (1u << gap) - 1u;
+#pragma unroll
+            for (uint32_t i = 0; i < 8; i++) {
+                const uint32_t k = 4u * i + (uint32_t)(lane & 3), t = k << 1;
+                if (k == 31u) break;   // (all of sub)
+                const uint32_t P = low | (t & keep) | ((t & ~keep) << 1);
+                const float c = T.cost[P] + T.cost[sub ^ P];
+                if (c < best || (c == best && P < bp) || bp == 0xFFFFFFFFu) { best = c; bp = P; }
             }
+        }
+        treelet_min(best, bp, 4);
+        if (sub && (lane & 3) == 0) {
             T.cost[sub] = node_cost(T.area[sub], T.count[sub], best, leaf_max);
             T.part[sub] = (uint8_t)bp;
         }
-        __syncwarp();
     }
-    // the full set: 63 partitions across the warp
-    {
-        const int full = TL_SUBSETS - 1;
-        float best = 3.4e38f;
-        int bp = 0;
-        for (int q = lane; q < (TL_SUBSETS >> 1) - 1; q += 32) {
-            int P = 1 | (q << 1);
-            float c = T.cost[P] + T.cost[full ^ P];
-            if (c < best || (c == best && P < bp)) { best = c; bp = P; }
+    __syncwarp();
+    {   // the full set: 63 partitions across the warp
+        const uint32_t full = TL_SUBSETS - 1;
+        uint32_t bp = 1u | ((uint32_t)lane << 1);
+        float best = T.cost[bp] + T.cost[full ^ bp];
+        if (lane < 31) {
+            const uint32_t P = bp + 64u;
+            const float c = T.cost[P] + T.cost[full ^ P];
+            if (c < best) { best = c; bp = P; }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            float ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            int op = __shfl_xor_sync(0xFFFFFFFFu, bp, o);
-            if (ob < best || (ob == best && op < bp)) { best = ob; bp = op; }
-        }
+        treelet_min(best, bp, 32);
         if (lane == 0) {
             T.cost[full] = node_cost(T.area[full], T.count[full], best, leaf_max);
             T.part[full] = (uint8_t)bp;
         }
     }
     __syncwarp();
-    // rewrite the treelet's internal nodes (lane 0; 6 nodes)
-    if (lane == 0) {
-        int stk_sub[TL_LEAVES], stk_node[TL_LEAVES];
-        int sp = 0, next = 1;
-        stk_sub[sp] = TL_SUBSETS - 1; stk_node[sp] = T.inner[0]; sp++;
-        while (sp > 0) {
-            --sp;
-            const int sub = stk_sub[sp], node = stk_node[sp];
-            const int P = T.part[sub], Q = sub ^ P;
-            int cidx[2];
-            const int halves[2] = {P, Q};
-            for (int h = 0; h < 2; h++) {
-                const int hs = halves[h];
-                if (__popc(hs) == 1) {
-                    cidx[h] = T.leaf[__ffs(hs) - 1];
-                } else {
-                    cidx[h] = T.inner[next++];
-                    stk_sub[sp] = hs; stk_node[sp] = cidx[h]; sp++;
-                }
-                parent[cidx[h]] = node;
+    // rewrite the treelet's six internal nodes: every lane follows the partitions,
+    // lane k keeps and stores node k
+    uint32_t sub = lane == 0 ? TL_SUBSETS - 1 : 0u;
+    int2 kids = make_int2(0, 0);
+    int next = 1;
+#pragma unroll
+    for (int k = 0; k < TL_LEAVES - 1; k++) {
+        const uint32_t s = __shfl_sync(FULL, sub, k);
+        const uint32_t half[2] = {T.part[s], s ^ T.part[s]};
+        int c[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (__popc(half[h]) == 1) {
+                c[h] = T.leaf[__ffs(half[h]) - 1];
+            } else {
+                if (lane == next) sub = half[h];
+                c[h] = __shfl_sync(FULL, inner, next);
+                next++;
             }
-            children[node] = make_int2(cidx[0], cidx[1]);
-            float4 lo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), hi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
-            for (int k = 0; k < TL_LEAVES; k++) {
-                if (!(sub & (1 << k))) continue;
-                float4 a = T.lo[k], b = T.hi[k];
-                lo.x = fminf(lo.x, a.x); lo.y = fminf(lo.y, a.y); lo.z = fminf(lo.z, a.z);
-                hi.x = fmaxf(hi.x, b.x); hi.y = fmaxf(hi.y, b.y); hi.z = fmaxf(hi.z, b.z);
-            }
-            node_lo[node] = lo;
-            node_hi[node] = hi;
-            leaf_count[node] = T.count[sub];
-            cost[node] = T.cost[sub];
         }
+        if (lane == k) kids = make_int2(c[0], c[1]);
+    }
+    if (lane < TL_LEAVES - 1) {
+        children[inner] = kids;
+        parent[kids.x] = inner;
+        parent[kids.y] = inner;
+        float4 a = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), z = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < TL_LEAVES; k++) {
+            if (!((sub >> k) & 1u)) continue;
+            const float4 l = T.lo[k], h = T.hi[k];
+            a.x = fminf(a.x, l.x); a.y = fminf(a.y, l.y); a.z = fminf(a.z, l.z);
+            z.x = fmaxf(z.x, h.x); z.y = fmaxf(z.y, h.y); z.z = fmaxf(z.z, h.z);
+        }
+        node_lo[inner] = a;
+        node_hi[inner] = z;
+        leaf_count[inner] = T.count[sub];
+        cost[inner] = T.cost[sub];
     }
     __syncwarp();
 }
 
 // One restructuring pass, leaf j of this thread (every lane of the warp calls
-// it): each thread climbs towards the root; the second thread to reach a node
-// hands that node's treelet to its whole warp.
+// it): each thread climbs towards the root; the second thread to reach a node costs
+// it, or hands its treelet to the whole warp when it holds at least seven
+// primitives.  Every pass adds 2 to the flag of each internal node.
 template <bool G>
 __device__ void treelet_climb(int j, int n, int2* children, int* parent, int* flags, float4* node_lo,
                               float4* node_hi, uint32_t* leaf_count, float* cost, TreeletSmem& T, uint32_t leaf_max) {
     const int nl = n - 1;
+    const TreeletLane mine = treelet_lane();
     bool active = j < n;
     int cur = nl + j;
     if (active) cost[cur] = SAH_CT * half_area(node_lo[cur], node_hi[cur]);
     while (true) {
         int p = -1;
-        bool ready = false;
+        bool ready = false, big = false;
         if (active) {
             p = ldx<G>(&parent[cur]);
             if (p < 0) {
                 active = false;
             } else {
                 mem_fence<G>();
-                if (atomicAdd(&flags[p], 1) == 0) active = false;
+                if ((atomicAdd(&flags[p], 1) & 1) == 0) active = false;
                 else ready = true;
                 mem_fence<G>();
             }
         }
-        unsigned m = __ballot_sync(0xFFFFFFFFu, ready);
+        if (ready) {
+            const uint32_t total = ldx<G>(&leaf_count[p]);
+            big = total >= (uint32_t)TL_LEAVES;
+            if (!big) {   // (box and count are already final)
+                const int2 ch = ldx<G>(&children[p]);
+                const float c = ldx<G>(&cost[ch.x]) + ldx<G>(&cost[ch.y]);
+                cost[p] = node_cost(half_area(ldx<G>(&node_lo[p]), ldx<G>(&node_hi[p])), total, c, leaf_max);
+            }
+        }
+        __syncwarp();
+        unsigned m = __ballot_sync(0xFFFFFFFFu, big);
         while (m) {
             const int l = __ffs(m) - 1;
             m &= m - 1;
             const int root = __shfl_sync(0xFFFFFFFFu, p, l);
-            treelet_optimise<G>(root, nl, children, parent, node_lo, node_hi, leaf_count, cost, T, leaf_max);
+            treelet_optimise<G>(root, nl, children, parent, node_lo, node_hi, leaf_count, cost, T, mine, leaf_max);
         }
-        mem_fence<G>();
         if (ready) cur = p;
         if (!__any_sync(0xFFFFFFFFu, active)) break;
     }

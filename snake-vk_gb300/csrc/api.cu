@@ -111,6 +111,8 @@ struct snk_pt_ctx {
     BuildScratch scratch;
     DBuf<float4> d_box_lo, d_box_hi;
     DBuf<uint32_t> d_prim_order, d_inst_list;
+    DBuf<uint32_t> d_trees;            // the meshes' trees: first primitives, then mesh indices
+    DBuf<SmallBuildOut> d_mesh_out;    // result record of the mesh build
 
     // frame buffers
     DBuf<float4> rays0, rays1, beta, L, srays, scontrib;
@@ -261,41 +263,68 @@ Status build_meshes(snk_pt_ctx* ctx) {
     SNK_TRY(upload(ctx->d_pos, pos.data(), pos.size(), st));
     SNK_TRY(upload(ctx->d_nrm, nrm.data(), nrm.size(), st));
     SNK_TRY(upload(ctx->d_idx, idx.data(), idx.size(), st));
-    size_t max_nt = 1;
-    for (auto& H : ctx->meshes) max_nt = std::max<size_t>(max_nt, H.nt);
-    SNK_TRY_CUDA(ctx->d_box_lo.reserve(max_nt));
-    SNK_TRY_CUDA(ctx->d_box_hi.reserve(max_nt));
-    SNK_TRY_CUDA(ctx->d_prim_order.reserve(max_nt));
+    SNK_TRY(upload(ctx->d_meshes, ctx->h_meshes.data(), ctx->h_meshes.size(), st));
     SNK_TRY_CUDA(ctx->d_blas.reserve(nt + ctx->meshes.size() + 1));
     SNK_TRY_CUDA(ctx->d_tris.reserve(nt ? nt : 1));
+    // One build makes the trees of consecutive meshes together, up to BATCH_PRIMS triangles
+    // (or one larger mesh): one scene usually is one build, and a huge one needs no more
+    // scratch than its largest batch.  Only a further batch waits for the node count of
+    // the one before.
+    constexpr uint32_t BATCH_PRIMS = 1u << 20;
+    const uint32_t leaf_max = leaf_size(ctx->tune.bvh_leaf_max, 1);
     uint32_t node_base = 0, prim_base = 0;
-    double sah_sum = 0.0, sah_w = 0.0;
-    for (size_t m = 0; m < ctx->meshes.size(); m++) {
-        MeshInfo& mi = ctx->h_meshes[m];
-        if (mi.num_triangles == 0) continue;
-        SNK_TRY(launch_triangle_boxes(ctx->d_pos.p, ctx->d_idx.p, mi.vertex_offset, mi.index_offset, mi.num_triangles,
-                                      ctx->d_box_lo.p, ctx->d_box_hi.p, st));
-        BuildResult br;
-        SNK_TRY(build_wide_bvh(ctx->scratch, ctx->d_box_lo.p, ctx->d_box_hi.p, mi.num_triangles, ctx->d_blas.p,
-                               node_base, prim_base, ctx->d_prim_order.p, st, &br,
-                               treelet_passes(ctx->tune.bvh_treelet_passes, 3), leaf_size(ctx->tune.bvh_leaf_max, 1),
-                               std::max(leaf_size(ctx->tune.bvh_leaf_pack, 1), leaf_size(ctx->tune.bvh_leaf_max, 1)),
-                               ctx->tune.bvh_collapse == 0));
-        SNK_TRY(launch_fill_triangles(ctx->d_prim_order.p, mi.num_triangles, ctx->d_pos.p, ctx->d_idx.p,
-                                      mi.vertex_offset, mi.index_offset, ctx->d_tris.p + prim_base, st));
-        mi.blas_root = node_base;
-        for (int a = 0; a < 3; a++) { mi.lo[a] = br.lo[a]; mi.hi[a] = br.hi[a]; }
-        node_base += br.num_nodes;
-        prim_base += mi.num_triangles;
-        sah_sum += br.sah * mi.num_triangles;
-        sah_w += mi.num_triangles;
+    double sah_sum = 0.0;
+    std::vector<uint32_t> first, tree_mesh;
+    for (size_t m = 0; m < ctx->meshes.size();) {
+        first.clear();
+        tree_mesh.clear();
+        uint32_t prims = 0, max_n = 0;
+        for (; m < ctx->meshes.size(); m++) {
+            const uint32_t n = ctx->h_meshes[m].num_triangles;
+            if (n == 0) continue;
+            if (prims && (uint64_t)prims + n > BATCH_PRIMS) break;
+            first.push_back(prims);
+            tree_mesh.push_back((uint32_t)m);
+            prims += n;
+            max_n = std::max(max_n, n);
+        }
+        if (prims == 0) break;
+        const uint32_t n_trees = (uint32_t)tree_mesh.size();
+        first.push_back(prims);
+        first.insert(first.end(), tree_mesh.begin(), tree_mesh.end());
+        SNK_TRY(upload(ctx->d_trees, first.data(), first.size(), st));
+        SNK_TRY_CUDA(ctx->d_box_lo.reserve(prims));
+        SNK_TRY_CUDA(ctx->d_box_hi.reserve(prims));
+        SNK_TRY_CUDA(ctx->d_prim_order.reserve(prims));
+        SNK_TRY_CUDA(ctx->d_mesh_out.reserve(1));
+        const BuildTrees B{ctx->d_trees.p, n_trees, prims};
+        const uint32_t* d_tree_mesh = ctx->d_trees.p + n_trees + 1;
+        SNK_TRY(launch_triangle_boxes(ctx->d_pos.p, ctx->d_idx.p, B, d_tree_mesh, ctx->d_meshes.p, ctx->d_box_lo.p,
+                                      ctx->d_box_hi.p, st));
+        SNK_TRY(build_wide_bvhs(ctx->scratch, ctx->d_box_lo.p, ctx->d_box_hi.p, B, max_n, ctx->d_blas.p, node_base,
+                                prim_base, ctx->d_prim_order.p, nullptr, st,
+                                treelet_passes(ctx->tune.bvh_treelet_passes, 3), leaf_max,
+                                std::max(leaf_size(ctx->tune.bvh_leaf_pack, 1), leaf_max), ctx->d_mesh_out.p, nullptr,
+                                ctx->tune.bvh_collapse == 0, true));
+        SNK_TRY(launch_fill_triangles(ctx->scratch, ctx->d_prim_order.p, B, d_tree_mesh, node_base, ctx->d_meshes.p,
+                                      ctx->d_pos.p, ctx->d_idx.p, ctx->d_tris.p + prim_base, st));
+        SmallBuildOut r{};
+        SNK_TRY_CUDA(cudaMemcpyAsync(&r, ctx->d_mesh_out.p, sizeof(r), cudaMemcpyDeviceToHost, st));
+        SNK_TRY_CUDA(cudaStreamSynchronize(st));
+        if (r.error) return Status::Err(SNK_ERR_LIMIT, "mesh BVH build exceeded its capacity");
+        node_base += r.num_nodes;
+        prim_base += prims;
+        sah_sum += r.sah;
     }
+    // the meshes' roots and bounds, for the host
+    if (!ctx->h_meshes.empty())
+        SNK_TRY_CUDA(cudaMemcpyAsync(ctx->h_meshes.data(), ctx->d_meshes.p, ctx->h_meshes.size() * sizeof(MeshInfo),
+                                     cudaMemcpyDeviceToHost, st));
+    SNK_TRY_CUDA(cudaStreamSynchronize(st));
     ctx->blas_nodes = node_base;
     ctx->total_tris = prim_base;
+    ctx->blas_sah = prim_base ? 1.0 + sah_sum / prim_base : 0.0;
     ctx->blas_leaf_single = leaf_size(ctx->tune.bvh_leaf_max, 1) == 1 && leaf_size(ctx->tune.bvh_leaf_pack, 1) <= 1;
-    ctx->blas_sah = sah_w > 0 ? sah_sum / sah_w : 0.0;
-    SNK_TRY(upload(ctx->d_meshes, ctx->h_meshes.data(), ctx->h_meshes.size(), st));
-    SNK_TRY_CUDA(cudaStreamSynchronize(st));
     return Status::Ok();
 }
 
@@ -479,10 +508,10 @@ Status build_instances(snk_pt_ctx* ctx) {
             return Status::Ok();
         } else {
             // multi-launch build, also without a host round trip (node count bounded by n + 1)
-            SNK_TRY(build_wide_bvh_device(ctx->scratch, ctx->d_box_lo.p, ctx->d_box_hi.p, n, ctx->d_tlas.p, 0u, 0u,
-                                          ctx->d_tlas_order.p, ctx->d_err.p, st, passes,
-                                          leaf_size(ctx->tune.tlas_leaf_max, 1), leaf_size(ctx->tune.tlas_leaf_max, 1),
-                                          ctx->d_small_out.p, ctx->d_tlas_depth.p, ctx->tune.bvh_collapse == 0));
+            SNK_TRY(build_wide_bvhs(ctx->scratch, ctx->d_box_lo.p, ctx->d_box_hi.p, BuildTrees{nullptr, 1u, n}, n,
+                                    ctx->d_tlas.p, 0u, 0u, ctx->d_tlas_order.p, ctx->d_err.p, st, passes,
+                                    leaf_size(ctx->tune.tlas_leaf_max, 1), leaf_size(ctx->tune.tlas_leaf_max, 1),
+                                    ctx->d_small_out.p, ctx->d_tlas_depth.p, ctx->tune.bvh_collapse == 0, false));
             ctx->tlas_nodes = n + 1;
             ctx->tlas_small = false;
             ctx->tlas_builds++;

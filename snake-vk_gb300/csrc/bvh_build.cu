@@ -5,25 +5,32 @@
 //   TLAS::BuildFromInstances     Core/src/resources/TLAS.cpp:10-87   (full rebuild every frame,
 //                                Core/src/scene/TlasSystem.cpp:16-20,27-49)
 //
-// Pipeline (all on the device, one stream):
-//   1. centroid bounds (block reduction + order-preserving atomics)
+// Pipeline (all on the device, one stream, no host round trip).  A build takes the
+// primitives of any number of trees (the meshes of a scene, one after another; the
+// instance BVH is one tree), so that loading many submeshes costs the launches and
+// the dependent steps of one (50 small meshes: 807 launches and 29.3 ms one mesh and
+// one host-read level at a time, 31 launches and 1.63 ms together; a 131,072-triangle
+// terrain and a sphere 3.66 and 2.46 ms):
+//   1. centroid bounds of each tree (block reduction + order-preserving atomics)
 //   2. 63-bit Morton codes of the centroids (21 bits per axis)
-//   3. sort of (code, primitive) pairs (project kernels below: a bitonic network
-//      in one CTA's shared memory up to 8192 pairs, an LSD radix sort in one CTA
-//      up to 65,536, three kernels per radix digit beyond)
-//   4. binary radix tree (Karras, HPG 2012): one thread per internal node
-//   5. bottom-up boxes and leaf counts (atomic arrival flags)
+//   3. sort of (tree, code, primitive) (project kernels below: a bitonic network in one
+//      CTA's shared memory for one small tree, else an LSD radix sort, one kernel per digit)
+//   4. binary radix trees (Karras, HPG 2012): one thread per internal node
+//   5. boxes and leaf counts, bottom-up (atomic arrival flags), in the first of the
+//      climbs below that runs
 //   5b. treelet restructuring (Karras & Aila, HPG 2013): bottom-up over the binary
 //      tree, every node whose subtree holds >= 7 primitives roots a treelet of 7
 //      leaves (grown by opening the largest-area treelet leaf); one warp finds the
 //      SAH-optimal binary topology of those 7 leaves by dynamic programming over
 //      all 127 leaf subsets and every 2-partition of each, and rewrites the
-//      treelet's 6 internal nodes in place.  Subtrees of <= 3 primitives are
-//      costed as the leaves the collapse will make of them.  Repeated for a few
+//      treelet's 6 internal nodes in place.  Subtrees of at most leaf_max primitives
+//      are costed as the leaves the collapse will make of them.  Repeated for a few
 //      passes; the result is deterministic (each treelet depends only on its
 //      finished subtrees, ties break on the lowest subset index).
-//   6. top-down collapse to 8-wide nodes, one thread per output node, level by
-//      level: a node's children start as its binary children; the internal child
+//   5c. least-SAH choice of every wide node's children (bottom-up)
+//   6. top-down collapse to 8-wide nodes, one warp per output node, level by
+//      level: a node's children are the least-SAH choice or, with greedy collapse,
+//      start as its binary children, of which the internal one
 //      with the largest surface area and more than leaf_max primitives is replaced
 //      by its two children until 8 children exist or none can be opened.  Children
 //      with <= leaf_pack primitives (leaf_max <= leaf_pack <= 4) become leaves: a
@@ -34,10 +41,15 @@
 //      are quantised outwards to 8 bits per plane.
 //   7. SAH cost of the result (for quality reporting).
 //
-// Mesh BVHs (built once, at load) take the multi-launch pipeline above.  The
-// per-frame instance BVH of up to 1024 instances is built by one single-CTA
+// Binary node ids: internal node i of the tree whose primitives start at f is f + i
+// (its root is f), the leaf at sorted position j is N + j, N the primitives of the
+// whole build.
+//
+// The per-frame instance BVH of up to 1024 instances is built by one single-CTA
 // launch instead (k_build_small: clustering in shared memory, then treelet passes
-// and the same collapse), so that a frame's rebuild costs no host round trip.
+// and the same collapse).
+
+#include <algorithm>
 
 #include "snk_host.h"
 
@@ -62,31 +74,58 @@ __device__ __forceinline__ T ldx(const T* p) {
     else return *p;
 }
 
-__global__ void k_init_bounds(unsigned* cb) {
-    if (threadIdx.x < 3) { cb[threadIdx.x] = 0xFFFFFFFFu; cb[3 + threadIdx.x] = 0u; }
+// the tree of primitive i / where tree t's primitives begin and end
+__device__ __forceinline__ uint32_t tree_of(const BuildTrees& B, uint32_t i) {
+    uint32_t lo = 0, hi = B.count - 1u;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1u) >> 1;
+        if (__ldg(B.first + mid) <= i) lo = mid;
+        else hi = mid - 1u;
+    }
+    return lo;
+}
+__device__ __forceinline__ uint32_t tree_begin(const BuildTrees& B, uint32_t t) {
+    return B.count == 1u ? 0u : __ldg(B.first + t);
+}
+__device__ __forceinline__ uint32_t tree_end(const BuildTrees& B, uint32_t t) {
+    return B.count == 1u ? B.total : __ldg(B.first + t + 1u);
 }
 
-__global__ void k_centroid_bounds(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n,
-                                  unsigned* cb) {
-    __shared__ unsigned smin[3][BLK], smax[3][BLK];
-    unsigned mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0u, 0u, 0u};
-    for (uint32_t i = blockIdx.x * BLK + threadIdx.x; i < n; i += gridDim.x * BLK) {
-        float4 a = lo[i], b = hi[i];
-        float c[3] = {0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z)};
-        for (int k = 0; k < 3; k++) { unsigned e = enc_f(c[k]); mn[k] = min(mn[k], e); mx[k] = max(mx[k], e); }
+// Centroid bounds of every tree, 6 words each (zero at the start): the largest ~enc of
+// x, y, z (whose complement is the smallest) and the largest enc.  A block inside one
+// tree reduces before its atomics.
+__global__ void __launch_bounds__(BLK) k_centroid_bounds(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                         BuildTrees B, unsigned* cb) {
+    __shared__ unsigned red[6][BLK / 32];
+    const uint32_t b0 = blockIdx.x * BLK, i = b0 + threadIdx.x;
+    const bool valid = i < B.total;
+    const uint32_t last = min(b0 + BLK, B.total) - 1u;
+    unsigned v[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    if (valid) {
+        const float4 a = lo[i], b = hi[i];
+        const float c[3] = {0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z)};
+        for (int k = 0; k < 3; k++) {
+            const unsigned e = enc_f(c[k]);
+            v[k] = ~e;
+            v[3 + k] = e;
+        }
     }
-    for (int k = 0; k < 3; k++) { smin[k][threadIdx.x] = mn[k]; smax[k][threadIdx.x] = mx[k]; }
-    __syncthreads();
-    for (int s = BLK / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-            for (int k = 0; k < 3; k++) {
-                smin[k][threadIdx.x] = min(smin[k][threadIdx.x], smin[k][threadIdx.x + s]);
-                smax[k][threadIdx.x] = max(smax[k][threadIdx.x], smax[k][threadIdx.x + s]);
-            }
+    const uint32_t t0 = tree_of(B, b0);
+    if (last < tree_end(B, t0)) {
+        for (int k = 0; k < 6; k++) {
+            const unsigned m = __reduce_max_sync(0xFFFFFFFFu, v[k]);
+            if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = m;
+        }
         __syncthreads();
+        if (threadIdx.x < 6) {
+            unsigned m = 0u;
+            for (int w = 0; w < BLK / 32; w++) m = max(m, red[threadIdx.x][w]);
+            atomicMax(&cb[6ull * t0 + threadIdx.x], m);
+        }
+    } else if (valid) {
+        unsigned* dst = cb + 6ull * tree_of(B, i);
+        for (int k = 0; k < 6; k++) atomicMax(&dst[k], v[k]);
     }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; k++) { atomicMin(&cb[k], smin[k][0]); atomicMax(&cb[3 + k], smax[k][0]); }
 }
 
 __device__ __forceinline__ unsigned long long spread21(unsigned long long x) {
@@ -113,14 +152,6 @@ __device__ __forceinline__ unsigned long long morton_of(float4 a, float4 b, cons
     return (spread21(q[0]) << 2) | (spread21(q[1]) << 1) | spread21(q[2]);
 }
 
-__global__ void k_morton(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n,
-                         const unsigned* cb, unsigned long long* keys, uint32_t* vals) {
-    uint32_t i = blockIdx.x * BLK + threadIdx.x;
-    if (i >= n) return;
-    keys[i] = morton_of(lo[i], hi[i], cb);
-    vals[i] = i;
-}
-
 __device__ __forceinline__ int delta(const unsigned long long* __restrict__ k, int n, int i, int j) {
     if (j < 0 || j >= n) return -1;
     unsigned long long a = k[i], b = k[j];
@@ -128,7 +159,8 @@ __device__ __forceinline__ int delta(const unsigned long long* __restrict__ k, i
     return __clzll(a ^ b);
 }
 
-__device__ void karras_node(int i, const unsigned long long* __restrict__ keys, int n, int2* children, int* parent) {
+__device__ __forceinline__ void karras_node(int i, const unsigned long long* __restrict__ keys, int n, uint32_t first,
+                                            uint32_t total, int2* children, int* parent) {
     int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
     int dmin = delta(keys, n, i, i - d);
     int lmax = 2;
@@ -144,31 +176,32 @@ __device__ void karras_node(int i, const unsigned long long* __restrict__ keys, 
         if (delta(keys, n, i, i + (s + t) * d) > dnode) s += t;
     } while (t > 1);
     int gamma = i + s * d + min(d, 0);
-    int left = (min(i, j) == gamma) ? (n - 1 + gamma) : gamma;
-    int right = (max(i, j) == gamma + 1) ? (n - 1 + gamma + 1) : gamma + 1;
-    children[i] = make_int2(left, right);
-    parent[left] = i;
-    parent[right] = i;
+    const int left = (int)first + gamma + (min(i, j) == gamma ? (int)total : 0);
+    const int right = (int)first + gamma + 1 + (max(i, j) == gamma + 1 ? (int)total : 0);
+    const int self = (int)first + i;
+    children[self] = make_int2(left, right);
+    parent[left] = self;
+    parent[right] = self;
 }
 
-// ---- radix sort of (63-bit Morton code, primitive) pairs ------------------------------
-// LSD radix sort with 8-bit digits.  Every pass is stable: the elements of one
-// digit keep their current order.  A CTA ranks a chunk of 1024 consecutive
-// elements at a time: lanes holding the same digit find each other with
-// __match_any_sync (their order within the warp is their lane order), every warp
-// counts its digits in shared memory, and an exclusive scan of those counts over
-// the warps gives each warp its start within the digit.  Up to SORT_SMALL_MAX
-// elements (sets above the bitonic sort's 8192) one CTA runs all passes in
-// one launch and skips the passes whose digit is the same for every key; larger
-// sets (mesh BVHs, at load time) take three launches per pass (per-tile digit
-// counts, their exclusive scan in digit-major order, the stable scatter).  The
-// result is always back in the first buffer pair.
+// ---- radix sort of (tree, 63-bit Morton code, primitive) ------------------------------
+// LSD radix sort with 8-bit digits, one kernel per digit: the code's eight, then the
+// digits of the tree's number when a build has several trees.  Every pass is stable:
+// the elements of one digit keep their current order.  A CTA owns a tile of the
+// input; it adds up the digit counts of the tiles before its own (and of all tiles,
+// for the digits' starts), then ranks a chunk of 1024 consecutive elements at a time:
+// lanes holding the same digit find each other with __match_any_sync (their order
+// within the warp is their lane order), every warp counts its digits in shared
+// memory, and an exclusive scan of those counts over the warps gives each warp its
+// start within the digit.  As it stores an element it counts the element's next digit
+// for the tile it lands in, so a pass needs no counting or scanning launch of its own.
+// Bound by latency at the sizes of a scene: tiles of 1024 put 131,072 elements on 128
+// SMs (tiles of 4096 and three launches per digit before).
 constexpr int SORT_THREADS = 1024;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
 constexpr int SORT_RADIX = 256;
-constexpr int SORT_PASSES = 8;                      // 64 bits (the codes use 63)
-constexpr uint32_t SORT_SMALL_MAX = 1u << 16;
-constexpr uint32_t SORT_TILE = 4u * SORT_THREADS;  // elements per CTA and pass (multi-CTA sort)
+constexpr int SORT_CODE_PASSES = 8;                // 64 bits (the codes use 63)
+constexpr uint32_t SORT_TILES = 160;               // tiles of a pass, about one per SM
 
 struct SortSmem {
     uint32_t wcnt[SORT_WARPS][SORT_RADIX];   // per-warp digit counts, then their exclusive scan
@@ -177,30 +210,24 @@ struct SortSmem {
     uint32_t warp_sum[SORT_RADIX / 32];
 };
 
-__device__ __forceinline__ uint32_t sort_digit(unsigned long long k, int shift) {
-    return (uint32_t)(k >> shift) & (SORT_RADIX - 1u);
+// digit `pass` of an element: of its code, or of its tree's number
+__device__ __forceinline__ uint32_t sort_digit(int pass, unsigned long long k, uint32_t v, const BuildTrees& B) {
+    if (pass < SORT_CODE_PASSES) return (uint32_t)(k >> (8 * pass)) & (SORT_RADIX - 1u);
+    return (tree_of(B, v) >> (8 * (pass - SORT_CODE_PASSES))) & (SORT_RADIX - 1u);
 }
 
-// threads 0..255: base[d] = sum of in[0..d) (in may alias base)
-__device__ __forceinline__ void scan_radix(SortSmem& S, const uint32_t* in) {
-    const int t = threadIdx.x, lane = t & 31;
-    uint32_t v = 0, incl = 0;
-    if (t < SORT_RADIX) {
-        v = in[t];
-        incl = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (lane == 31) S.warp_sum[t >> 5] = incl;
-    }
-    __syncthreads();
-    if (t < SORT_RADIX) {
-        uint32_t off = 0;
-        for (int w = 0; w < (t >> 5); w++) off += S.warp_sum[w];
-        S.base[t] = off + incl - v;
-    }
-    __syncthreads();
+// Morton codes within each tree's centroid bounds; hist: digit 0 of every tile (zero at
+// the start; null when the codes are not radix-sorted)
+__global__ void k_morton(const float4* __restrict__ lo, const float4* __restrict__ hi, BuildTrees B, const unsigned* cb,
+                         unsigned long long* keys, uint32_t* vals, uint32_t* hist, uint32_t tile_shift) {
+    const uint32_t i = blockIdx.x * BLK + threadIdx.x;
+    if (i >= B.total) return;
+    const unsigned* c = cb + 6ull * tree_of(B, i);
+    const unsigned bounds[6] = {~__ldg(c), ~__ldg(c + 1), ~__ldg(c + 2), __ldg(c + 3), __ldg(c + 4), __ldg(c + 5)};
+    const unsigned long long k = morton_of(lo[i], hi[i], bounds);
+    keys[i] = k;
+    vals[i] = i;
+    if (hist) atomicAdd(&hist[(size_t)(i >> tile_shift) * SORT_RADIX + sort_digit(0, k, i, B)], 1u);
 }
 
 // Output position of this thread's element (valid, digit d) in a chunk of one
@@ -216,6 +243,7 @@ __device__ __forceinline__ uint32_t rank_chunk(SortSmem& S, bool valid, uint32_t
     __syncthreads();
     if (t < SORT_RADIX) {
         uint32_t run = 0;
+#pragma unroll 8
         for (int w = 0; w < SORT_WARPS; w++) {
             const uint32_t c = S.wcnt[w][t];
             S.wcnt[w][t] = run;
@@ -230,50 +258,71 @@ __device__ __forceinline__ uint32_t rank_chunk(SortSmem& S, bool valid, uint32_t
     return pos;   // (the next chunk's first barrier orders the base update)
 }
 
-__global__ void __launch_bounds__(SORT_THREADS, 1) k_sort_small(unsigned long long* keys, uint32_t* vals,
-                                                              unsigned long long* keys_alt, uint32_t* vals_alt,
-                                                              uint32_t n) {
+// One digit of the sort.  hist: this digit's counts, 256 per tile; hist_next: the next
+// digit's, zero at the start (null at the last digit).  tile = 1 << tile_shift elements.
+__global__ void __launch_bounds__(SORT_THREADS, 1) k_sort_pass(const unsigned long long* __restrict__ sk,
+                                                             const uint32_t* __restrict__ sv, BuildTrees B, int pass,
+                                                             uint32_t tile_shift, const uint32_t* __restrict__ hist,
+                                                             uint32_t* hist_next, unsigned long long* dk, uint32_t* dv) {
     __shared__ SortSmem S;
-    __shared__ uint32_t hist[SORT_RADIX];
-    __shared__ int skip;
-    const int t = threadIdx.x;
-    unsigned long long* sk = keys;
-    uint32_t* sv = vals;
-    unsigned long long* dk = keys_alt;
-    uint32_t* dv = vals_alt;
-    for (int pass = 0; pass < SORT_PASSES; pass++) {
-        const int shift = 8 * pass;
-        if (t < SORT_RADIX) hist[t] = 0u;
-        __syncthreads();
-        for (uint32_t i = t; i < n; i += SORT_THREADS) atomicAdd(&hist[sort_digit(sk[i], shift)], 1u);
-        __syncthreads();
-        if (t == 0) skip = hist[sort_digit(sk[0], shift)] == n;   // every key has this digit
-        scan_radix(S, hist);
-        if (skip) continue;
-        for (uint32_t c = 0; c < n; c += SORT_THREADS) {
-            const uint32_t i = c + (uint32_t)t;
-            const bool valid = i < n;
-            const unsigned long long k = valid ? sk[i] : 0ull;
-            const uint32_t v = valid ? sv[i] : 0u;
-            const uint32_t pos = rank_chunk(S, valid, sort_digit(k, shift));
-            if (valid) { dk[pos] = k; dv[pos] = v; }
+    const uint32_t t = threadIdx.x, n = B.total;
+    {   // four rows of counts at a time: the tiles before this one, and all of them
+        const uint32_t d = t & (SORT_RADIX - 1u), group = t / SORT_RADIX;
+        uint32_t before = 0, all = 0;
+#pragma unroll 8
+        for (uint32_t r = group; r < gridDim.x; r += SORT_THREADS / SORT_RADIX) {
+            const uint32_t c = __ldg(&hist[(size_t)r * SORT_RADIX + d]);
+            all += c;
+            if (r < blockIdx.x) before += c;
         }
-        __syncthreads();
-        unsigned long long* tk = sk; sk = dk; dk = tk;
-        uint32_t* tv = sv; sv = dv; dv = tv;
+        S.wcnt[group][d] = before;
+        S.wcnt[SORT_THREADS / SORT_RADIX + group][d] = all;
     }
-    if (sk != keys) {   // an odd number of passes ran: the result goes back to the first pair
-        for (uint32_t i = t; i < n; i += SORT_THREADS) { keys[i] = sk[i]; vals[i] = sv[i]; }
+    __syncthreads();
+    const uint32_t lane = t & 31u;
+    uint32_t before = 0, sum = 0, incl = 0;
+    if (t < SORT_RADIX) {
+        for (int g = 0; g < SORT_THREADS / SORT_RADIX; g++) {
+            before += S.wcnt[g][t];
+            sum += S.wcnt[SORT_THREADS / SORT_RADIX + g][t];
+        }
+        incl = sum;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31u) S.warp_sum[t >> 5] = incl;
+    }
+    __syncthreads();
+    if (t < SORT_RADIX) {
+        uint32_t off = 0;
+        for (uint32_t w = 0; w < (t >> 5); w++) off += S.warp_sum[w];
+        S.base[t] = off + incl - sum + before;
+    }
+    __syncthreads();
+    const uint32_t b0 = blockIdx.x << tile_shift, b1 = min(b0 + (1u << tile_shift), n);
+    for (uint32_t c = b0; c < b1; c += SORT_THREADS) {
+        const uint32_t i = c + t;
+        const bool valid = i < b1;
+        const unsigned long long k = valid ? sk[i] : 0ull;
+        const uint32_t v = valid ? sv[i] : 0u;
+        const uint32_t pos = rank_chunk(S, valid, valid ? sort_digit(pass, k, v, B) : 0u);
+        if (valid) {
+            dk[pos] = k;
+            dv[pos] = v;
+            if (hist_next)
+                atomicAdd(&hist_next[(size_t)(pos >> tile_shift) * SORT_RADIX + sort_digit(pass + 1, k, v, B)], 1u);
+        }
     }
 }
 
-// Up to SORT_BITONIC_MAX pairs (the per-frame instance sets) one CTA sorts in shared
-// memory with a bitonic network: 91 barrier-separated compare-exchange stages for
-// 8192 entries instead of 8 radix passes over global memory.  The network is not
+// One tree of up to SORT_BITONIC_MAX primitives is sorted by one CTA in shared
+// memory with a bitonic network (66 barrier-separated compare-exchange stages for
+// 2048 entries, one launch instead of eight).  The network is not
 // stable by itself, so it orders by (key, value): the values are the primitives'
 // indices 0..n-1 in their input order, which makes the result the stable order.
 // Entries past n are padded with the largest pair.
-constexpr uint32_t SORT_BITONIC_MAX = 8192;
+constexpr uint32_t SORT_BITONIC_MAX = 2048;
 
 __global__ void __launch_bounds__(SORT_THREADS, 1) k_sort_bitonic(unsigned long long* keys, uint32_t* vals,
                                                                 uint32_t n) {
@@ -308,67 +357,15 @@ __global__ void __launch_bounds__(SORT_THREADS, 1) k_sort_bitonic(unsigned long 
     }
 }
 
-// multi-CTA pass, step 1: digit counts of each tile, digit-major (hist[d * tiles + tile])
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_hist(const unsigned long long* __restrict__ keys, uint32_t n,
-                                                            int shift, uint32_t* hist, uint32_t tiles) {
-    __shared__ uint32_t h[SORT_RADIX];
-    const int t = threadIdx.x;
-    if (t < SORT_RADIX) h[t] = 0u;
-    __syncthreads();
-    const uint32_t b0 = blockIdx.x * SORT_TILE, b1 = min(b0 + SORT_TILE, n);
-    for (uint32_t i = b0 + t; i < b1; i += SORT_THREADS) atomicAdd(&h[sort_digit(keys[i], shift)], 1u);
-    __syncthreads();
-    if (t < SORT_RADIX) hist[(size_t)t * tiles + blockIdx.x] = h[t];
-}
-
-// step 2: exclusive scan of the m = 256 x tiles counts in place (one CTA; each
-// thread scans a contiguous run, the runs' totals are scanned across the block)
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_scan(uint32_t* hist, uint32_t m) {
-    __shared__ uint32_t warp_tot[SORT_WARPS];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t per = (m + SORT_THREADS - 1) / SORT_THREADS;
-    const uint32_t b0 = min((uint32_t)t * per, m), b1 = min(b0 + per, m);
-    uint32_t sum = 0;
-    for (uint32_t i = b0; i < b1; i++) sum += hist[i];
-    uint32_t incl = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += u;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    uint32_t off = 0;
-    for (int w = 0; w < warp; w++) off += warp_tot[w];
-    uint32_t run = off + incl - sum;
-    for (uint32_t i = b0; i < b1; i++) {
-        const uint32_t c = hist[i];
-        hist[i] = run;
-        run += c;
-    }
-}
-
-// step 3: stable scatter of each tile from its digits' scanned starts
-__global__ void __launch_bounds__(SORT_THREADS, 1) k_sort_scatter(const unsigned long long* __restrict__ sk,
-                                                                const uint32_t* __restrict__ sv, uint32_t n, int shift,
-                                                                const uint32_t* __restrict__ hist, uint32_t tiles,
-                                                                unsigned long long* dk, uint32_t* dv) {
-    __shared__ SortSmem S;
-    const int t = threadIdx.x;
-    if (t < SORT_RADIX) S.base[t] = hist[(size_t)t * tiles + blockIdx.x];
-    const uint32_t b0 = blockIdx.x * SORT_TILE, b1 = min(b0 + SORT_TILE, n);
-    for (uint32_t c = b0; c < b1; c += SORT_THREADS) {
-        const uint32_t i = c + (uint32_t)t;
-        const bool valid = i < b1;
-        const unsigned long long k = valid ? sk[i] : 0ull;
-        const uint32_t v = valid ? sv[i] : 0u;
-        const uint32_t pos = rank_chunk(S, valid, sort_digit(k, shift));
-        if (valid) { dk[pos] = k; dv[pos] = v; }
-    }
-}
-
-__global__ void k_karras(const unsigned long long* __restrict__ keys, int n, int2* children, int* parent) {
-    int i = blockIdx.x * BLK + threadIdx.x;
-    if (i < n - 1) karras_node(i, keys, n, children, parent);
+// one thread per primitive: internal node i of its tree, i its place in the tree (the
+// last place has none); the root has no parent
+__global__ void k_karras(const unsigned long long* __restrict__ keys, BuildTrees B, int2* children, int* parent) {
+    const uint32_t g = blockIdx.x * BLK + threadIdx.x;
+    if (g >= B.total) return;
+    const uint32_t t = tree_of(B, g), first = tree_begin(B, t);
+    const int n = (int)(tree_end(B, t) - first), i = (int)(g - first);
+    if (i == 0) parent[n > 1 ? first : B.total + first] = -1;
+    if (i < n - 1) karras_node(i, keys + first, n, first, B.total, children, parent);
 }
 
 template <bool G>
@@ -377,40 +374,43 @@ __device__ __forceinline__ void mem_fence() {
     else __threadfence_block();
 }
 
-// boxes and primitive counts from leaf j to the root (the second thread to
-// arrive at a node completes it)
+// box and primitive count of internal node p from its two finished children; returns the count
 template <bool G>
-__device__ void bottom_up_leaf(int j, const uint32_t* __restrict__ sorted, const float4* __restrict__ plo,
-                               const float4* __restrict__ phi, int n, const int2* children, const int* parent,
-                               int* flags, float4* node_lo, float4* node_hi, uint32_t* leaf_count) {
-    int node = n - 1 + j;
-    uint32_t prim = sorted[j];
+__device__ __forceinline__ uint32_t join_children(int p, const int2* children, float4* node_lo, float4* node_hi,
+                                                  uint32_t* leaf_count) {
+    const int2 ch = children[p];
+    const float4 al = ldx<G>(&node_lo[ch.x]), ah = ldx<G>(&node_hi[ch.x]);
+    const float4 bl = ldx<G>(&node_lo[ch.y]), bh = ldx<G>(&node_hi[ch.y]);
+    const uint32_t cnt = ldx<G>(&leaf_count[ch.x]) + ldx<G>(&leaf_count[ch.y]);
+    node_lo[p] = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.0f);
+    node_hi[p] = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.0f);
+    leaf_count[p] = cnt;
+    return cnt;
+}
+__device__ __forceinline__ void init_leaf(int node, uint32_t prim, const float4* __restrict__ plo,
+                                          const float4* __restrict__ phi, float4* node_lo, float4* node_hi,
+                                          uint32_t* leaf_count) {
     node_lo[node] = plo[prim];
     node_hi[node] = phi[prim];
     leaf_count[node] = 1;
-    if (n == 1) return;
-    int p = parent[node];
-    while (p >= 0) {
-        mem_fence<G>();
-        if (atomicAdd(&flags[p], 1) == 0) return;
-        mem_fence<G>();
-        int2 ch = children[p];
-        float4 al = ldx<G>(&node_lo[ch.x]), ah = ldx<G>(&node_hi[ch.x]);
-        float4 bl = ldx<G>(&node_lo[ch.y]), bh = ldx<G>(&node_hi[ch.y]);
-        uint32_t ca = ldx<G>(&leaf_count[ch.x]), cb = ldx<G>(&leaf_count[ch.y]);
-        node_lo[p] = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.0f);
-        node_hi[p] = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.0f);
-        leaf_count[p] = ca + cb;
-        p = parent[p];
-    }
 }
 
+// Climbs from every leaf: the second thread to arrive at a node completes it.  Every
+// climb of a build adds 2 to the flag of each internal node, so the flags are zeroed
+// once.
 __global__ void k_bottom_up(const uint32_t* __restrict__ sorted, const float4* __restrict__ plo,
                             const float4* __restrict__ phi, int n, const int2* __restrict__ children,
                             const int* __restrict__ parent, int* flags, float4* node_lo, float4* node_hi,
                             uint32_t* leaf_count) {
-    int j = blockIdx.x * BLK + threadIdx.x;
-    if (j < n) bottom_up_leaf<true>(j, sorted, plo, phi, n, children, parent, flags, node_lo, node_hi, leaf_count);
+    const int j = blockIdx.x * BLK + threadIdx.x;
+    if (j >= n) return;
+    init_leaf(n + j, sorted[j], plo, phi, node_lo, node_hi, leaf_count);
+    for (int p = parent[n + j]; p >= 0; p = parent[p]) {
+        mem_fence<true>();
+        if ((atomicAdd(&flags[p], 1) & 1) == 0) return;
+        mem_fence<true>();
+        join_children<true>(p, children, node_lo, node_hi, leaf_count);
+    }
 }
 
 __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
@@ -673,11 +673,11 @@ __device__ void treelet_optimise(int root, int nl, int2* children, int* parent, 
 // One restructuring pass, leaf j of this thread (every lane of the warp calls
 // it): each thread climbs towards the root; the second thread to reach a node costs
 // it, or hands its treelet to the whole warp when it holds at least seven
-// primitives.  Every pass adds 2 to the flag of each internal node.
-template <bool G>
-__device__ void treelet_climb(int j, int n, int2* children, int* parent, int* flags, float4* node_lo,
+// primitives.  FIRST: the climb also makes the boxes and counts (the boxes and counts
+// of the leaves are in place).  Every pass adds 2 to the flag of each internal node.
+template <bool G, bool FIRST>
+__device__ void treelet_climb(int j, int n, int nl, int2* children, int* parent, int* flags, float4* node_lo,
                               float4* node_hi, uint32_t* leaf_count, float* cost, TreeletSmem& T, uint32_t leaf_max) {
-    const int nl = n - 1;
     const TreeletLane mine = treelet_lane();
     bool active = j < n;
     int cur = nl + j;
@@ -697,9 +697,10 @@ __device__ void treelet_climb(int j, int n, int2* children, int* parent, int* fl
             }
         }
         if (ready) {
-            const uint32_t total = ldx<G>(&leaf_count[p]);
+            const uint32_t total = FIRST ? join_children<G>(p, children, node_lo, node_hi, leaf_count)
+                                         : ldx<G>(&leaf_count[p]);
             big = total >= (uint32_t)TL_LEAVES;
-            if (!big) {   // (box and count are already final)
+            if (!big) {
                 const int2 ch = ldx<G>(&children[p]);
                 const float c = ldx<G>(&cost[ch.x]) + ldx<G>(&cost[ch.y]);
                 cost[p] = node_cost(half_area(ldx<G>(&node_lo[p]), ldx<G>(&node_hi[p])), total, c, leaf_max);
@@ -718,12 +719,17 @@ __device__ void treelet_climb(int j, int n, int2* children, int* parent, int* fl
     }
 }
 
-__global__ void __launch_bounds__(BLK) k_treelet_pass(int n, int2* children, int* parent, int* flags,
-                                                      float4* node_lo, float4* node_hi, uint32_t* leaf_count,
-                                                      float* cost, uint32_t leaf_max) {
+template <bool FIRST>
+__global__ void __launch_bounds__(BLK) k_treelet_pass(int n, const uint32_t* __restrict__ sorted,
+                                                      const float4* __restrict__ plo, const float4* __restrict__ phi,
+                                                      int2* children, int* parent, int* flags, float4* node_lo,
+                                                      float4* node_hi, uint32_t* leaf_count, float* cost,
+                                                      uint32_t leaf_max) {
     __shared__ TreeletSmem smem[TL_WARPS];
-    treelet_climb<true>(blockIdx.x * BLK + threadIdx.x, n, children, parent, flags, node_lo, node_hi, leaf_count,
-                        cost, smem[threadIdx.x >> 5], leaf_max);
+    const int j = blockIdx.x * BLK + threadIdx.x;
+    if (FIRST && j < n) init_leaf(n + j, sorted[j], plo, phi, node_lo, node_hi, leaf_count);
+    treelet_climb<true, FIRST>(j, n, n, children, parent, flags, node_lo, node_hi, leaf_count, cost,
+                               smem[threadIdx.x >> 5], leaf_max);
 }
 
 // smallest power-of-two exponent (biased) with 2^(e-127) >= x; at least 1
@@ -831,206 +837,70 @@ __device__ __forceinline__ void wide_cost_node(int p, int nl, const int2* childr
     wide_split[p] = split;
 }
 
-// bottom-up from leaf j of n (the second thread to arrive at a node completes it)
-template <bool G>
-__device__ void wide_cost_climb(int j, int n, const int2* children, const int* parent, int* flags,
-                                const float4* node_lo, const float4* node_hi, const uint32_t* leaf_count,
+// bottom-up from leaf j (the second thread to arrive at a node completes it; FIRST: with
+// its box and count)
+template <bool G, bool FIRST>
+__device__ void wide_cost_climb(int j, int nl, const int2* children, const int* parent, int* flags,
+                                float4* node_lo, float4* node_hi, uint32_t* leaf_count,
                                 float* wide_cost, uint32_t* wide_split, uint32_t leaf_max, uint32_t leaf_pack) {
-    if (n == 1) return;
-    const int nl = n - 1;
-    int p = parent[nl + j];
-    while (p >= 0) {
+    for (int p = parent[nl + j]; p >= 0; p = parent[p]) {
         mem_fence<G>();
-        if (atomicAdd(&flags[p], 1) == 0) return;
+        if ((atomicAdd(&flags[p], 1) & 1) == 0) return;
         mem_fence<G>();
+        if (FIRST) join_children<G>(p, children, node_lo, node_hi, leaf_count);
         wide_cost_node<G>(p, nl, children, node_lo, node_hi, leaf_count, wide_cost, wide_split, leaf_max, leaf_pack);
-        p = parent[p];
     }
 }
 
-__global__ void k_collapse_cost(int n, const int2* __restrict__ children, const int* __restrict__ parent, int* flags,
-                                const float4* __restrict__ node_lo, const float4* __restrict__ node_hi,
-                                const uint32_t* __restrict__ leaf_count, float* wide_cost, uint32_t* wide_split,
-                                uint32_t leaf_max, uint32_t leaf_pack) {
+template <bool FIRST>
+__global__ void k_collapse_cost(int n, const uint32_t* __restrict__ sorted, const float4* __restrict__ plo,
+                                const float4* __restrict__ phi, const int2* __restrict__ children,
+                                const int* __restrict__ parent, int* flags, float4* node_lo, float4* node_hi,
+                                uint32_t* leaf_count, float* wide_cost, uint32_t* wide_split, uint32_t leaf_max,
+                                uint32_t leaf_pack) {
     const int j = blockIdx.x * BLK + threadIdx.x;
-    if (j < n)
-        wide_cost_climb<true>(j, n, children, parent, flags, node_lo, node_hi, leaf_count, wide_cost, wide_split,
-                              leaf_max, leaf_pack);
+    if (j >= n) return;
+    if (FIRST) init_leaf(n + j, sorted[j], plo, phi, node_lo, node_hi, leaf_count);
+    wide_cost_climb<true, FIRST>(j, n, children, parent, flags, node_lo, node_hi, leaf_count, wide_cost, wide_split,
+                                 leaf_max, leaf_pack);
 }
 
-// the children of the wide node rooted at internal node b chosen by wide_split
-// (the least-SAH distribution of b's subtree over 8 slots); returns their number
+// The children of the wide node rooted at internal node b chosen by wide_split (the
+// least-SAH distribution of b's subtree over 8 slots), one per lane in the tree's
+// order; returns their number.  All open items expand in one round of loads (lane k
+// holds item k: a binary node and the slots it may fill; item: 8 entries of this
+// warp's shared memory).
 __device__ __forceinline__ int wide_children(int b, int nl, const int2* children, const uint32_t* wide_split,
-                                             int C[8]) {
-    int sn[8], ss[8], sp = 0, nc = 0;
+                                             int2* item, int* child) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
     const int2 ch = children[b];
     const int k8 = (int)(wide_split[b] & 15u);
-    sn[sp] = ch.y; ss[sp++] = 8 - k8;
-    sn[sp] = ch.x; ss[sp++] = k8;
-    while (sp > 0 && nc < 8) {
-        const int y = sn[--sp], slots = ss[sp];
-        const int k = (y >= nl || slots <= 1) ? 0 : (int)((wide_split[y] >> (4 * (slots - 1))) & 15u);
-        if (k == 0 || k >= slots || sp > 6) {
-            C[nc++] = y;
-        } else {
-            const int2 cy = children[y];
-            sn[sp] = cy.y; ss[sp++] = slots - k;
-            sn[sp] = cy.x; ss[sp++] = k;
+    int y = lane == 0 ? ch.x : ch.y, slots = lane == 0 ? k8 : 8 - k8, count = 2;
+    for (int round = 0; round < 7; round++) {
+        int k = 0;
+        int2 cy = make_int2(0, 0);
+        if (lane < count && y < nl && slots > 1) {
+            k = (int)((wide_split[y] >> (4 * (slots - 1))) & 15u);
+            cy = children[y];
+            if (k >= slots) k = 0;
         }
-    }
-    return sp > 0 ? -1 : nc;   // -1: more than 8 children (never with a consistent table)
-}
-
-// One output node: task = (binary node, wide node slot).  counters: [1] tasks
-// out, [2] wide nodes, [3] primitive slots, [4] capacity error bits.
-__device__ void collapse_task(uint2 task, uint32_t* counters, uint2* tasks_out, int n,
-                              const int2* __restrict__ children, const float4* __restrict__ node_lo,
-                              const float4* __restrict__ node_hi, const uint32_t* __restrict__ leaf_count,
-                              const uint32_t* __restrict__ sorted, WideNode* nodes, uint32_t node_base,
-                              uint32_t prim_base, uint32_t* prim_order, double* sah, float root_half_area,
-                              uint32_t leaf_max, uint32_t leaf_pack, const uint32_t* __restrict__ wide_split) {
-    int b = (int)task.x;
-    uint32_t w = task.y;
-    const int nl = n - 1;  // first leaf id
-    int C[8];
-    int nc;
-    if (b >= nl) { C[0] = b; nc = 1; }
-    else if (wide_split) {
-        nc = wide_children(b, nl, children, wide_split, C);
-        if (nc < 0) { atomicOr(&counters[4], 8u); return; }
-    }
-    else { int2 ch = children[b]; C[0] = ch.x; C[1] = ch.y; nc = 2; }
-    while (!wide_split && nc < 8) {
-        int best = -1;
-        float best_a = -1.0f;
-        for (int k = 0; k < nc; k++) {
-            int c = C[k];
-            if (c < nl && leaf_count[c] > leaf_max) {
-                float a = half_area(node_lo[c], node_hi[c]);
-                if (a > best_a) { best_a = a; best = k; }
-            }
+        const unsigned open = __ballot_sync(FULL, k > 0);
+        if (open == 0u) break;
+        const int total = count + __popc(open);
+        if (total > 8) return -1;   // (never with a consistent table)
+        if (lane < count) {
+            const int pos = lane + __popc(open & ((1u << lane) - 1u));
+            item[pos] = k > 0 ? make_int2(cy.x, k) : make_int2(y, slots);
+            if (k > 0) item[pos + 1] = make_int2(cy.y, slots - k);
         }
-        if (best < 0) break;
-        int2 ch = children[C[best]];
-        C[best] = ch.x;
-        C[nc++] = ch.y;
+        count = total;
+        __syncwarp();
+        if (lane < count) { y = item[lane].x; slots = item[lane].y; }
+        __syncwarp();
     }
-    // parent box and child centroids
-    float4 plo = node_lo[C[0]], phi = node_hi[C[0]];
-    for (int k = 1; k < nc; k++) {
-        float4 a = node_lo[C[k]], z = node_hi[C[k]];
-        plo.x = fminf(plo.x, a.x); plo.y = fminf(plo.y, a.y); plo.z = fminf(plo.z, a.z);
-        phi.x = fmaxf(phi.x, z.x); phi.y = fmaxf(phi.y, z.y); phi.z = fmaxf(phi.z, z.z);
-    }
-    float pcx = 0.5f * (plo.x + phi.x), pcy = 0.5f * (plo.y + phi.y), pcz = 0.5f * (plo.z + phi.z);
-    float ccx[8], ccy[8], ccz[8];
-    for (int k = 0; k < nc; k++) {
-        float4 a = node_lo[C[k]], z = node_hi[C[k]];
-        ccx[k] = 0.5f * (a.x + z.x) - pcx; ccy[k] = 0.5f * (a.y + z.y) - pcy; ccz[k] = 0.5f * (a.z + z.z) - pcz;
-    }
-    // greedy slot assignment: slot bit i set <=> the child lies on the + side of axis i
-    int slot_child[8];
-    for (int s = 0; s < 8; s++) slot_child[s] = -1;
-    uint32_t used_c = 0, used_s = 0;
-    for (int it = 0; it < nc; it++) {
-        float best = -3.4e38f;
-        int bk = -1, bs = -1;
-        for (int k = 0; k < nc; k++) {
-            if (used_c & (1u << k)) continue;
-            for (int s = 0; s < 8; s++) {
-                if (used_s & (1u << s)) continue;
-                float sc = ((s & 1) ? ccx[k] : -ccx[k]) + ((s & 2) ? ccy[k] : -ccy[k]) + ((s & 4) ? ccz[k] : -ccz[k]);
-                if (sc > best) { best = sc; bk = k; bs = s; }
-            }
-        }
-        used_c |= 1u << bk;
-        used_s |= 1u << bs;
-        slot_child[bs] = C[bk];
-    }
-    // classify and allocate
-    uint32_t n_int = 0, n_prims = 0;
-    for (int s = 0; s < 8; s++) {
-        int c = slot_child[s];
-        if (c < 0) continue;
-        if (c < nl && leaf_count[c] > leaf_pack) n_int++;
-        else n_prims += leaf_count[c];
-    }
-    uint32_t child_local = n_int ? atomicAdd(&counters[2], n_int) : 0u;
-    uint32_t prim_local = n_prims ? atomicAdd(&counters[3], n_prims) : 0u;
-    // capacity checks: n wide nodes, n primitive slots, n tasks (never exceeded by a
-    // correct tree; a violation is recorded and the node is not written)
-    if (child_local + n_int > (uint32_t)n + 1u || prim_local + n_prims > (uint32_t)n || w - node_base > (uint32_t)n) {
-        atomicOr(&counters[4], 1u);
-        return;
-    }
-    const QuantFrame F = quant_frame(plo, phi);
-    WideNode node;
-    node.px = plo.x; node.py = plo.y; node.pz = plo.z;
-    node.ex = (uint8_t)F.eb[0]; node.ey = (uint8_t)F.eb[1]; node.ez = (uint8_t)F.eb[2];
-    node.imask = 0;
-    node.child_base = node_base + child_local;
-    node.prim_base = prim_base + prim_local;
-    uint32_t rank = 0, off = 0;
-    double local_sah = 0.0;
-    for (int s = 0; s < 8; s++) {
-        int c = slot_child[s];
-        if (c < 0) {
-            node.meta[s] = 0;
-            for (int a = 0; a < 3; a++) { node.qlo[a][s] = 0; node.qhi[a][s] = 0; }
-            continue;
-        }
-        float4 a4 = node_lo[c], z4 = node_hi[c];
-        quant_child(F, a4, z4, node, s);
-        const float ha = sah ? half_area(a4, z4) / root_half_area : 0.0f;
-        if (c < nl && leaf_count[c] > leaf_pack) {
-            node.meta[s] = (uint8_t)META_INTERNAL;
-            node.imask |= (uint8_t)(1u << s);
-            uint32_t slot_out = atomicAdd(&counters[1], 1u);
-            if (slot_out < (uint32_t)n) tasks_out[slot_out] = make_uint2((uint32_t)c, node.child_base + rank);
-            else atomicOr(&counters[4], 2u);
-            rank++;
-            local_sah += (double)ha;   // one traversal step into the child
-        } else {
-            uint32_t cnt = leaf_count[c];
-            node.meta[s] = (uint8_t)((cnt << 5) | off);
-            // collect the (<= leaf_pack) leaves of subtree c in order
-            int stk[8];
-            int sp = 0;
-            stk[sp++] = c;
-            uint32_t k = 0;
-            while (sp > 0) {
-                int x = stk[--sp];
-                if (x >= nl) {
-                    if (k < cnt) prim_order[prim_local + off + k] = sorted[x - nl];
-                    k++;
-                } else if (sp < 7) {
-                    int2 ch = children[x];
-                    stk[sp++] = ch.y;
-                    stk[sp++] = ch.x;
-                } else {
-                    atomicOr(&counters[4], 4u);   // deeper than a subtree of leaf_pack leaves can be
-                }
-            }
-            off += cnt;
-            local_sah += (double)ha * (double)cnt;   // primitive tests
-        }
-    }
-    if (sah) atomicAdd(sah, local_sah);
-    uint4* dst = reinterpret_cast<uint4*>(nodes + w);
-    const uint4* src = reinterpret_cast<const uint4*>(&node);
-    for (int k = 0; k < 5; k++) dst[k] = src[k];
-}
-
-__global__ void k_collapse(const uint2* __restrict__ tasks_in, uint32_t* counters, uint2* tasks_out, int n,
-                           const int2* __restrict__ children, const float4* __restrict__ node_lo,
-                           const float4* __restrict__ node_hi, const uint32_t* __restrict__ leaf_count,
-                           const uint32_t* __restrict__ sorted, WideNode* nodes, uint32_t node_base,
-                           uint32_t prim_base, uint32_t* prim_order, double* sah, float root_half_area,
-                           uint32_t leaf_max, uint32_t leaf_pack, const uint32_t* __restrict__ wide_split) {
-    uint32_t ti = blockIdx.x * BLK + threadIdx.x;
-    if (ti >= counters[0]) return;
-    collapse_task(tasks_in[ti], counters, tasks_out, n, children, node_lo, node_hi, leaf_count, sorted, nodes,
-                  node_base, prim_base, prim_order, sah, root_half_area, leaf_max, leaf_pack, wide_split);
+    *child = lane < count ? y : -1;
+    return count;
 }
 
 // ---- single-CTA agglomerative builder for small primitive sets -----------------
@@ -1113,44 +983,35 @@ __device__ __forceinline__ unsigned order_f(float f) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-// collapse_task for a whole warp (every lane passes the same task): the same
-// greedy choices, made with warp reductions instead of one thread's loops.
-// counters: [2] wide nodes, [3] primitive slots, [4] capacity error bits;
-// next_tasks counts the child tasks queued in tasks_out.
+// One output node by a whole warp (every lane passes the same task: binary node, wide
+// node slot).  counters: [2] wide nodes, [3] primitive slots, [4] capacity error bits;
+// next_tasks counts the child tasks queued in tasks_out.  cap: primitives of the
+// build, cap_nodes: wide nodes it may write; internal binary nodes have ids below nl.
+// inv_root > 0: returns (lane 0) the node's part of the SAH cost, its children's areas
+// times inv_root, one traversal step per internal child and one test per primitive.
 // Lane k < nc holds candidate child k while the node is opened; the 64 (child,
 // slot) pairs p = 8k + s of the slot assignment are spread two per lane; lane s
 // < 8 then builds slot s.  Ties go to the lowest child / pair index, as in the
 // sequential loops.  stage: this warp's 80-byte staging node in shared memory.
-__device__ void collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* next_tasks, uint2* tasks_out, int n,
-                                   const int2* children,
-                                   const float4* node_lo, const float4* node_hi, const uint32_t* leaf_count,
-                                   const uint32_t* sorted, WideNode* nodes, WideNode* stage, uint32_t node_base,
-                                   uint32_t prim_base, uint32_t* prim_order, uint32_t leaf_max, uint32_t leaf_pack,
-                                   const uint32_t* wide_split) {
+__device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* next_tasks, uint2* tasks_out,
+                                     uint32_t cap, uint32_t cap_nodes, int nl, const int2* children,
+                                     const float4* node_lo, const float4* node_hi, const uint32_t* leaf_count,
+                                     const uint32_t* sorted, WideNode* nodes, WideNode* stage, uint32_t node_base,
+                                     uint32_t prim_base, uint32_t* prim_order, uint32_t leaf_max, uint32_t leaf_pack,
+                                     const uint32_t* wide_split, float inv_root) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     const int b = (int)task.x;
     const uint32_t w = task.y;
-    const int nl = n - 1;   // first leaf id
     int c = -1, nc;
     if (b >= nl) {
         nc = 1;
         if (lane == 0) c = b;
     } else if (wide_split) {
-        // the least-SAH children (lane 0 expands the split table, lane k takes child k)
-        int C[8];
-        int m = 0;
-        if (lane == 0) m = wide_children(b, nl, children, wide_split, C);
-        m = __shfl_sync(FULL, m, 0);
-        if (m < 0) {
+        nc = wide_children(b, nl, children, wide_split, reinterpret_cast<int2*>(stage), &c);
+        if (nc < 0) {
             if (lane == 0) atomicOr(&counters[4], 8u);
-            return;
-        }
-        nc = m;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int v = __shfl_sync(FULL, (lane == 0 && k < m) ? C[k] : -1, 0);
-            if (lane == k) c = v;
+            return 0.0;
         }
     } else {
         const int2 ch = children[b];
@@ -1234,9 +1095,9 @@ __device__ void collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* nex
     prim_local = __shfl_sync(FULL, prim_local, 0);
     // capacity checks (never exceeded by a correct tree; a violation is recorded,
     // the node is not written and no child task is queued)
-    if (child_local + n_int > (uint32_t)n + 1u || prim_local + n_prims > (uint32_t)n || w - node_base > (uint32_t)n) {
+    if (child_local + n_int > cap_nodes || prim_local + n_prims > cap || w - node_base >= cap_nodes) {
         if (lane == 0) atomicOr(&counters[4], 1u);
-        return;
+        return 0.0;
     }
     if (lane == 0 && n_int) task_base = atomicAdd(next_tasks, n_int);
     task_base = __shfl_sync(FULL, task_base, 0);
@@ -1259,7 +1120,7 @@ __device__ void collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* nex
                 const uint32_t rank = (uint32_t)__popc(int_mask & ((1u << s) - 1u));
                 stage->meta[s] = (uint8_t)META_INTERNAL;
                 const uint32_t slot_out = task_base + rank;
-                if (slot_out < (uint32_t)n) tasks_out[slot_out] = make_uint2((uint32_t)slot_c, node_base + child_local + rank);
+                if (slot_out < cap) tasks_out[slot_out] = make_uint2((uint32_t)slot_c, node_base + child_local + rank);
                 else atomicOr(&counters[4], 2u);
             } else {
                 stage->meta[s] = (uint8_t)((cnt << 5) | off);
@@ -1287,6 +1148,13 @@ __device__ void collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* nex
     __syncwarp();
     if (lane < 5) reinterpret_cast<uint4*>(nodes + w)[lane] = reinterpret_cast<const uint4*>(stage)[lane];
     __syncwarp();
+    double sah = 0.0;
+    if (inv_root > 0.0f) {
+        if (mine) sah = (double)(half_area(node_lo[slot_c], node_hi[slot_c]) * inv_root) * (is_int ? 1.0 : (double)cnt);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sah += __shfl_xor_sync(FULL, sah, o);
+    }
+    return sah;
 }
 
 __global__ void __launch_bounds__(SMALL_THREADS, 1)
@@ -1503,8 +1371,8 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
         for (int pass = 0; pass < passes; pass++) {
             if (tid < n) S.flags[tid] = 0;
             __syncthreads();
-            treelet_climb<false>((tid & 31) * 32 + (tid >> 5), n, S.children, S.parent, S.flags, S.node_lo,
-                                 S.node_hi, S.leaf_count, S.cost, S.tl[tid >> 5], leaf_max);
+            treelet_climb<false, false>((tid & 31) * 32 + (tid >> 5), n, nl, S.children, S.parent, S.flags, S.node_lo,
+                                        S.node_hi, S.leaf_count, S.cost, S.tl[tid >> 5], leaf_max);
             __syncthreads();
         }
     }
@@ -1520,8 +1388,8 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
         if (tid < n) S.flags[tid] = 0;
         __syncthreads();
         if (tid < n)
-            wide_cost_climb<false>(tid, n, S.children, S.parent, S.flags, S.node_lo, S.node_hi, S.leaf_count,
-                                   S.dp.wide_cost, S.dp.wide_split, leaf_max, leaf_max);
+            wide_cost_climb<false, false>(tid, nl, S.children, S.parent, S.flags, S.node_lo, S.node_hi, S.leaf_count,
+                                          S.dp.wide_cost, S.dp.wide_split, leaf_max, leaf_max);
         __syncthreads();
     }
     // 6. collapse, level by level
@@ -1548,9 +1416,10 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
                 wide_box[2 * local + 1] = S.node_hi[task.x];
                 wide_depth[local] = (uint32_t)level;
             }
-            collapse_task_warp(task, S.counters, &S.counters[1], S.tasks[cc ^ 1], n, S.children, S.node_lo, S.node_hi,
-                               S.leaf_count, S.vals, nodes, &S.stage[tid >> 5], node_base, prim_base, prim_order,
-                               leaf_max, leaf_max, dp ? S.dp.wide_split : nullptr);
+            collapse_task_warp(task, S.counters, &S.counters[1], S.tasks[cc ^ 1], (uint32_t)n, (uint32_t)n + 1u, nl,
+                               S.children, S.node_lo, S.node_hi, S.leaf_count, S.vals, nodes, &S.stage[tid >> 5],
+                               node_base, prim_base, prim_order, leaf_max, leaf_max, dp ? S.dp.wide_split : nullptr,
+                               0.0f);
         }
         __syncthreads();
         if (tid == 0) { S.counters[0] = S.counters[1]; S.counters[1] = 0u; }
@@ -1572,7 +1441,7 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
     }
 }
 
-// ---- collapse without host round trips (multi-launch builds of per-frame trees) ----------
+// ---- collapse without host round trips -----------------------------------------
 // level_tasks[l] counts the tasks of wide level l (tasks of even levels in
 // tasks_a, odd levels in tasks_b); counters: [2] wide nodes, [3] primitive
 // slots, [4] capacity error bits.  A few launches of k_collapse_level take the
@@ -1582,78 +1451,122 @@ constexpr int COLLAPSE_MAX_LEVELS = 128;
 constexpr int COLLAPSE_FAST_LEVELS = 8;
 constexpr int LEVEL_WARPS = 8;
 
-__global__ void k_collapse_init(uint2* tasks_a, uint32_t* counters, uint32_t* level_tasks, uint32_t node_base) {
-    for (int l = threadIdx.x; l <= COLLAPSE_MAX_LEVELS; l += blockDim.x) level_tasks[l] = l == 0 ? 1u : 0u;
-    if (threadIdx.x == 0) {
-        tasks_a[0] = make_uint2(0u, node_base);
-        counters[2] = 1u;
-        counters[3] = 0u;
-        counters[4] = 0u;
+// what the collapse reads and writes
+struct CollapseArgs {
+    BuildTrees B;
+    uint2 *tasks_a, *tasks_b;
+    uint32_t *level_tasks, *counters;
+    const int2* children;
+    const float4 *node_lo, *node_hi;
+    const uint32_t *leaf_count, *sorted, *wide_split;
+    WideNode* nodes;
+    uint32_t node_base, prim_base;
+    uint32_t* prim_order;
+    uint32_t leaf_max, leaf_pack;
+    uint32_t* wide_depth;   // may be null
+    double* sah;            // sum over the trees of primitives x SAH cost below the root; may be null
+};
+
+// the root of every tree: wide nodes node_base + t
+__global__ void k_collapse_init(CollapseArgs A) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t <= (uint32_t)COLLAPSE_MAX_LEVELS) A.level_tasks[t] = t == 0u ? A.B.count : 0u;
+    if (t < A.B.count) {
+        const uint32_t first = tree_begin(A.B, t);
+        const bool single = tree_end(A.B, t) - first == 1u;
+        A.tasks_a[t] = make_uint2(single ? A.B.total + first : first, A.node_base + t);
+    }
+    if (t == 0u) {
+        A.counters[2] = A.B.count;
+        A.counters[3] = 0u;
+        A.counters[4] = 0u;
+        if (A.sah) *A.sah = 0.0;
     }
 }
 
-// the depth of the wide node a task writes (for a later refit), by lane 0 of its warp
-__device__ __forceinline__ void note_depth(uint32_t* wide_depth, uint2 task, uint32_t node_base, int n, int level) {
-    const uint32_t local = task.y - node_base;
-    if (wide_depth && (threadIdx.x & 31) == 0 && local <= (uint32_t)n) wide_depth[local] = (uint32_t)level;
-}
-
-__global__ void __launch_bounds__(32 * LEVEL_WARPS) k_collapse_level(
-    int level, uint2* tasks_a, uint2* tasks_b, uint32_t* level_tasks, uint32_t* counters, int n, const int2* children,
-    const float4* node_lo, const float4* node_hi, const uint32_t* leaf_count, const uint32_t* sorted, WideNode* nodes,
-    uint32_t node_base, uint32_t prim_base, uint32_t* prim_order, uint32_t leaf_max, uint32_t leaf_pack,
-    uint32_t* wide_depth, const uint32_t* wide_split) {
-    __shared__ WideNode stage[LEVEL_WARPS];
-    const uint32_t nin = min(level_tasks[level], (uint32_t)n);   // the task arrays hold n entries
-    if (nin == 0 || counters[4] != 0u) return;
-    const uint2* tin = (level & 1) ? tasks_b : tasks_a;
-    uint2* tout = (level & 1) ? tasks_a : tasks_b;
-    const uint32_t w = threadIdx.x >> 5;
-    for (uint32_t t = blockIdx.x * LEVEL_WARPS + w; t < nin; t += gridDim.x * LEVEL_WARPS) {
+// One level's tasks t0, t0 + step, ... of this warp; returns their part of the SAH sum.
+__device__ __forceinline__ double collapse_level(const CollapseArgs& A, int level, uint32_t t0, uint32_t step,
+                                                 WideNode* stage) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t n = A.B.total;
+    if (A.counters[4] != 0u) return 0.0;                 // (a capacity error: nothing more is written)
+    const uint32_t nin = min(A.level_tasks[level], n);   // the task arrays hold n entries
+    const uint2* tin = (level & 1) ? A.tasks_b : A.tasks_a;
+    uint2* tout = (level & 1) ? A.tasks_a : A.tasks_b;
+    double sum = 0.0;
+    for (uint32_t t = t0; t < nin; t += step) {
         const uint2 task = tin[t];
-        note_depth(wide_depth, task, node_base, n, level);
-        collapse_task_warp(task, counters, &level_tasks[level + 1], tout, n, children, node_lo, node_hi, leaf_count,
-                           sorted, nodes, &stage[w], node_base, prim_base, prim_order, leaf_max, leaf_pack,
-                           wide_split);
+        const uint32_t local = task.y - A.node_base;
+        if (A.wide_depth && lane == 0 && local <= n) A.wide_depth[local] = (uint32_t)level;   // (for a later refit)
+        float inv_root = 0.0f;
+        uint32_t prims = 0;
+        if (A.sah) {
+            const uint32_t tree = tree_of(A.B, task.x >= n ? task.x - n : task.x);
+            const uint32_t first = tree_begin(A.B, tree);
+            prims = tree_end(A.B, tree) - first;
+            const uint32_t root = prims == 1u ? n + first : first;
+            const float area = half_area(A.node_lo[root], A.node_hi[root]);
+            inv_root = area > 0.0f ? 1.0f / area : 1.0f;
+        }
+        const double s = collapse_task_warp(task, A.counters, &A.level_tasks[level + 1], tout, n, n + A.B.count, (int)n,
+                                            A.children, A.node_lo, A.node_hi, A.leaf_count, A.sorted, A.nodes, stage,
+                                            A.node_base, A.prim_base, A.prim_order, A.leaf_max, A.leaf_pack,
+                                            A.wide_split, inv_root);
+        sum += s * (double)prims;
+    }
+    return sum;
+}
+
+// adds the warps' sums (lane 0) to *out, one atomic per block; all threads call this
+__device__ __forceinline__ void block_add(double sum, double* warp_sums, double* out) {
+    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if ((threadIdx.x & 31) == 0) warp_sums[w] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int k = 0; k < nw; k++) s += warp_sums[k];
+        if (s != 0.0) atomicAdd(out, s);
     }
 }
 
-__global__ void __launch_bounds__(1024) k_collapse_finish(
-    int first_level, uint2* tasks_a, uint2* tasks_b, uint32_t* level_tasks, uint32_t* counters, int n,
-    const int2* children, const float4* node_lo, const float4* node_hi, const uint32_t* leaf_count,
-    const uint32_t* sorted, WideNode* nodes, uint32_t node_base, uint32_t prim_base, uint32_t* prim_order,
-    uint32_t leaf_max, uint32_t leaf_pack, unsigned* err_word, uint32_t* wide_depth, SmallBuildOut* out,
-    const uint32_t* wide_split) {
+__global__ void __launch_bounds__(32 * LEVEL_WARPS) k_collapse_level(CollapseArgs A, int level) {
+    __shared__ WideNode stage[LEVEL_WARPS];
+    __shared__ double warp_sums[LEVEL_WARPS];
+    const uint32_t w = threadIdx.x >> 5;
+    if (blockIdx.x * LEVEL_WARPS >= A.level_tasks[level]) return;   // (this level's count is final)
+    const double sum = collapse_level(A, level, blockIdx.x * LEVEL_WARPS + w, gridDim.x * LEVEL_WARPS, &stage[w]);
+    if (A.sah) block_add(sum, warp_sums, A.sah);
+}
+
+__global__ void __launch_bounds__(1024) k_collapse_finish(CollapseArgs A, int first_level, unsigned* err_word,
+                                                          SmallBuildOut* out) {
     __shared__ WideNode stage[32];
+    __shared__ double warp_sums[32];
+    __shared__ int stop;
     const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     int level = first_level;
+    double sum = 0.0;
     for (; level < COLLAPSE_MAX_LEVELS; level++) {
-        const uint32_t nin = min(level_tasks[level], (uint32_t)n);
-        if (nin == 0 || counters[4] != 0u) break;
-        const uint2* tin = (level & 1) ? tasks_b : tasks_a;
-        uint2* tout = (level & 1) ? tasks_a : tasks_b;
-        for (uint32_t t = w; t < nin; t += nw) {
-            const uint2 task = tin[t];
-            note_depth(wide_depth, task, node_base, n, level);
-            collapse_task_warp(task, counters, &level_tasks[level + 1], tout, n, children, node_lo, node_hi,
-                               leaf_count, sorted, nodes, &stage[w], node_base, prim_base, prim_order, leaf_max,
-                               leaf_pack, wide_split);
-        }
+        if (threadIdx.x == 0) stop = A.level_tasks[level] == 0u || A.counters[4] != 0u;
+        __syncthreads();
+        if (stop) break;
+        sum += collapse_level(A, level, w, nw, &stage[w]);
         __syncthreads();   // this level's child tasks and their count are complete
     }
+    if (A.sah) block_add(sum, warp_sums, A.sah);
     if (threadIdx.x == 0) {
-        const bool unfinished = level >= COLLAPSE_MAX_LEVELS && level_tasks[COLLAPSE_MAX_LEVELS] != 0u;
-        const bool bad = counters[4] != 0u || unfinished || counters[3] != (uint32_t)n;
+        const bool unfinished = level >= COLLAPSE_MAX_LEVELS && A.level_tasks[COLLAPSE_MAX_LEVELS] != 0u;
+        const bool bad = A.counters[4] != 0u || unfinished || A.counters[3] != A.B.total;
         if (bad && err_word) atomicOr(err_word, 8u);
-        if (out) {   // the record a refit reads: node count and deepest level
+        if (out) {   // what a refit and the host read: node count, deepest level, SAH sum
             uint32_t deepest = 0;
             for (int l = 0; l < COLLAPSE_MAX_LEVELS; l++)
-                if (level_tasks[l] != 0u) deepest = (uint32_t)l;
-            out->num_nodes = counters[2];
-            out->prims = counters[3];
+                if (A.level_tasks[l] != 0u) deepest = (uint32_t)l;
+            out->num_nodes = A.counters[2];
+            out->prims = A.counters[3];
             out->error = bad ? 8u : 0u;
             out->max_depth = deepest;
-            out->sah = 0.0;
+            out->sah = A.sah ? atomicAdd(A.sah, 0.0) : 0.0;
         }
     }
 }
@@ -1721,13 +1634,18 @@ k_refit_small(WideNode* nodes, uint32_t node_base, uint32_t prim_base, const Sma
     }
 }
 
-__global__ void k_triangle_boxes(const float* __restrict__ pos, const uint32_t* __restrict__ idx, uint32_t vo,
-                                 uint32_t io, uint32_t nt, float4* lo, float4* hi) {
-    uint32_t t = blockIdx.x * BLK + threadIdx.x;
-    if (t >= nt) return;
+// primitive i of the concatenated meshes (BuildTrees over the meshes that have
+// triangles, tree_mesh[t] their indices): padded box of its triangle
+__global__ void k_triangle_boxes(const float* __restrict__ pos, const uint32_t* __restrict__ idx, BuildTrees B,
+                                 const uint32_t* __restrict__ tree_mesh, const MeshInfo* __restrict__ meshes, float4* lo,
+                                 float4* hi) {
+    const uint32_t i = blockIdx.x * BLK + threadIdx.x;
+    if (i >= B.total) return;
+    const uint32_t tree = tree_of(B, i), t = i - tree_begin(B, tree);
+    const MeshInfo& M = meshes[__ldg(tree_mesh + tree)];
     float l[3] = {3.4e38f, 3.4e38f, 3.4e38f}, h[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
     for (int k = 0; k < 3; k++) {
-        const float* p = pos + 3ull * (vo + idx[io + 3ull * t + k]);
+        const float* p = pos + 3ull * (M.vertex_offset + idx[M.index_offset + 3ull * t + k]);
         for (int a = 0; a < 3; a++) { l[a] = fminf(l[a], p[a]); h[a] = fmaxf(h[a], p[a]); }
     }
     float ext = fmaxf(fmaxf(h[0] - l[0], h[1] - l[1]), h[2] - l[2]);
@@ -1736,23 +1654,34 @@ __global__ void k_triangle_boxes(const float* __restrict__ pos, const uint32_t* 
         l[a] -= pad;
         h[a] += pad;
     }
-    lo[t] = make_float4(l[0], l[1], l[2], 0.0f);
-    hi[t] = make_float4(h[0], h[1], h[2], 0.0f);
+    lo[i] = make_float4(l[0], l[1], l[2], 0.0f);
+    hi[i] = make_float4(h[0], h[1], h[2], 0.0f);
 }
 
-__global__ void k_fill_triangles(const uint32_t* __restrict__ order, uint32_t n, const float* __restrict__ pos,
-                                 const uint32_t* __restrict__ idx, uint32_t vo, uint32_t io, TriRecord* out) {
-    uint32_t i = blockIdx.x * BLK + threadIdx.x;
-    if (i >= n) return;
-    uint32_t t = order[i];
+// triangle records in the build's primitive order, and every mesh's root node and
+// bounds (its tree's root box)
+__global__ void k_fill_triangles(const uint32_t* __restrict__ order, BuildTrees B, const uint32_t* __restrict__ tree_mesh,
+                                 uint32_t node_base, MeshInfo* meshes, const float* __restrict__ pos, const uint32_t* __restrict__ idx,
+                                 const float4* __restrict__ node_lo, const float4* __restrict__ node_hi, TriRecord* out) {
+    const uint32_t i = blockIdx.x * BLK + threadIdx.x;
+    if (i >= B.total) return;
+    const uint32_t prim = order[i], tree = tree_of(B, prim), first = tree_begin(B, tree), t = prim - first;
+    MeshInfo& M = meshes[__ldg(tree_mesh + tree)];
     TriRecord r;
     float* v[3] = {r.v0, r.v1, r.v2};
     for (int k = 0; k < 3; k++) {
-        const float* p = pos + 3ull * (vo + idx[io + 3ull * t + k]);
+        const float* p = pos + 3ull * (M.vertex_offset + idx[M.index_offset + 3ull * t + k]);
         v[k][0] = p[0]; v[k][1] = p[1]; v[k][2] = p[2]; v[k][3] = 0.0f;
     }
     r.v0[3] = __uint_as_float(t);
     out[i] = r;
+    if (t == 0u) {
+        const uint32_t root = tree_end(B, tree) - first == 1u ? B.total + first : first;
+        const float4 a = node_lo[root], z = node_hi[root];
+        M.blas_root = node_base + tree;
+        M.lo[0] = a.x; M.lo[1] = a.y; M.lo[2] = a.z;
+        M.hi[0] = z.x; M.hi[1] = z.y; M.hi[2] = z.z;
+    }
 }
 
 __global__ void k_instance_boxes(const uint32_t* __restrict__ list, uint32_t n, const InstShade* __restrict__ inst,
@@ -1789,48 +1718,56 @@ inline unsigned grid_for(uint32_t n) { return (n + BLK - 1) / BLK; }
 }  // namespace
 
 namespace {
-// sorts (sc.keys, sc.vals) by key, stably (sc.keys_alt / sc.vals_alt: scratch)
-Status sort_pairs(BuildScratch& sc, uint32_t n, cudaStream_t st) {
-    if (n <= SORT_BITONIC_MAX) {
+// Morton codes of the build's primitives, sorted by (tree, code) stably; *keys / *sorted:
+// the codes and primitives in order (either buffer pair)
+Status sort_prims(BuildScratch& sc, const BuildTrees& B, const float4* prim_lo, const float4* prim_hi, cudaStream_t st,
+                  const unsigned long long** keys, const uint32_t** sorted) {
+    const uint32_t n = B.total, g = grid_for(n);
+    *keys = sc.keys.p;
+    *sorted = sc.vals.p;
+    if (B.count == 1 && n <= SORT_BITONIC_MAX) {
+        k_morton<<<g, BLK, 0, st>>>(prim_lo, prim_hi, B, sc.cbounds.p, sc.keys.p, sc.vals.p, nullptr, 0u);
         uint32_t N = 2;
         while (N < n) N <<= 1;
-        const int bytes = (int)(N * (sizeof(unsigned long long) + sizeof(uint32_t)));
-        SNK_TRY_CUDA(cudaFuncSetAttribute(k_sort_bitonic, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        k_sort_bitonic<<<1, SORT_THREADS, bytes, st>>>(sc.keys.p, sc.vals.p, n);
+        k_sort_bitonic<<<1, SORT_THREADS, N * (sizeof(unsigned long long) + sizeof(uint32_t)), st>>>(sc.keys.p,
+                                                                                                  sc.vals.p, n);
         SNK_TRY_CUDA(cudaGetLastError());
         return Status::Ok();
     }
-    if (n <= SORT_SMALL_MAX) {
-        k_sort_small<<<1, SORT_THREADS, 0, st>>>(sc.keys.p, sc.vals.p, sc.keys_alt.p, sc.vals_alt.p, n);
-        SNK_TRY_CUDA(cudaGetLastError());
-        return Status::Ok();
-    }
-    const uint32_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
-    SNK_TRY_CUDA(sc.sort_hist.reserve((size_t)SORT_RADIX * tiles));
+    int passes = SORT_CODE_PASSES;
+    for (uint32_t t = B.count - 1u; t; t >>= 8) passes++;
+    uint32_t shift = 10;   // tiles of 1024 (one element per thread), or more when that would make over SORT_TILES
+    while (((uint64_t)n + (1ull << shift) - 1) >> shift > SORT_TILES) shift++;
+    const uint32_t tiles = (uint32_t)(((uint64_t)n + (1ull << shift) - 1) >> shift);
+    const size_t rows = (size_t)SORT_RADIX * tiles;
+    SNK_TRY_CUDA(sc.sort_hist.reserve(rows * passes));
+    SNK_TRY_CUDA(cudaMemsetAsync(sc.sort_hist.p, 0, rows * passes * sizeof(uint32_t), st));
+    k_morton<<<g, BLK, 0, st>>>(prim_lo, prim_hi, B, sc.cbounds.p, sc.keys.p, sc.vals.p, sc.sort_hist.p, shift);
     unsigned long long *sk = sc.keys.p, *dk = sc.keys_alt.p;
     uint32_t *sv = sc.vals.p, *dv = sc.vals_alt.p;
-    for (int pass = 0; pass < SORT_PASSES; pass++) {   // an even number: the result ends in sc.keys / sc.vals
-        const int shift = 8 * pass;
-        k_sort_hist<<<tiles, SORT_THREADS, 0, st>>>(sk, n, shift, sc.sort_hist.p, tiles);
-        k_sort_scan<<<1, SORT_THREADS, 0, st>>>(sc.sort_hist.p, (uint32_t)SORT_RADIX * tiles);
-        k_sort_scatter<<<tiles, SORT_THREADS, 0, st>>>(sk, sv, n, shift, sc.sort_hist.p, tiles, dk, dv);
-        SNK_TRY_CUDA(cudaGetLastError());
+    for (int pass = 0; pass < passes; pass++) {
+        k_sort_pass<<<tiles, SORT_THREADS, 0, st>>>(sk, sv, B, pass, shift, sc.sort_hist.p + rows * pass,
+                                                    pass + 1 < passes ? sc.sort_hist.p + rows * (pass + 1) : nullptr, dk,
+                                                    dv);
         std::swap(sk, dk);
         std::swap(sv, dv);
     }
-    static_assert(SORT_PASSES % 2 == 0, "the multi-CTA sort ends in the first buffer pair");
+    SNK_TRY_CUDA(cudaGetLastError());
+    *keys = sk;
+    *sorted = sv;
     return Status::Ok();
 }
+}  // namespace
 
-// the binary tree of build_wide_bvh and build_wide_bvh_device (Morton codes, radix
-// sort, Karras hierarchy, bottom-up boxes, treelet passes); *sorted_out receives
-// the primitive of each sorted position
-Status build_binary_tree(BuildScratch& sc, const float4* prim_lo, const float4* prim_hi, uint32_t n, cudaStream_t st,
-                         int treelet_passes, uint32_t leaf_max, uint32_t leaf_pack, const uint32_t** sorted_out) {
+Status build_wide_bvhs(BuildScratch& sc, const float4* prim_lo, const float4* prim_hi, const BuildTrees& B,
+                       uint32_t max_n, WideNode* nodes, uint32_t node_base, uint32_t prim_base, uint32_t* prim_order,
+                       unsigned* err_word, cudaStream_t st, int treelet_passes, uint32_t leaf_max, uint32_t leaf_pack,
+                       SmallBuildOut* out, uint32_t* wide_depth, bool sah_collapse, bool sah_cost) {
+    const uint32_t n = B.total;
     if (leaf_max < 1 || leaf_max > LEAF_MAX_LIMIT || leaf_pack < leaf_max || leaf_pack > LEAF_MAX_LIMIT)
-        return Status::Err(1, "build_wide_bvh: leaf size out of range");
-    if (n == 0) return Status::Err(1, "build_wide_bvh: no primitives");
-    if (n > (1u << 30)) return Status::Err(1, "build_wide_bvh: too many primitives");
+        return Status::Err(1, "build_wide_bvhs: leaf size out of range");
+    if (n == 0 || B.count == 0) return Status::Err(1, "build_wide_bvhs: no primitives");
+    if (n > (1u << 30)) return Status::Err(1, "build_wide_bvhs: too many primitives");
     SNK_TRY_CUDA(sc.keys.reserve(n));
     SNK_TRY_CUDA(sc.keys_alt.reserve(n));
     SNK_TRY_CUDA(sc.vals.reserve(n));
@@ -1845,138 +1782,70 @@ Status build_binary_tree(BuildScratch& sc, const float4* prim_lo, const float4* 
     SNK_TRY_CUDA(sc.tasks_a.reserve(n));
     SNK_TRY_CUDA(sc.tasks_b.reserve(n));
     SNK_TRY_CUDA(sc.counters.reserve(5));
-    SNK_TRY_CUDA(sc.cbounds.reserve(6));
+    SNK_TRY_CUDA(sc.cbounds.reserve(6 * (size_t)B.count));
     SNK_TRY_CUDA(sc.sah.reserve(1));
-
-    k_init_bounds<<<1, 32, 0, st>>>(sc.cbounds.p);
-    unsigned g = grid_for(n);
-    k_centroid_bounds<<<g < 1024u ? g : 1024u, BLK, 0, st>>>(prim_lo, prim_hi, n, sc.cbounds.p);
-    k_morton<<<g, BLK, 0, st>>>(prim_lo, prim_hi, n, sc.cbounds.p, sc.keys.p, sc.vals.p);
-    SNK_TRY_CUDA(cudaGetLastError());
-
-    SNK_TRY(sort_pairs(sc, n, st));
-    const unsigned long long* keys = sc.keys.p;
-    const uint32_t* sorted = sc.vals.p;
-    *sorted_out = sorted;
-
-    SNK_TRY_CUDA(cudaMemsetAsync(sc.flags.p, 0, sizeof(int) * n, st));
-    int minus1 = -1;
-    SNK_TRY_CUDA(cudaMemcpyAsync(sc.parent.p, &minus1, sizeof(int), cudaMemcpyHostToDevice, st));
-    if (n > 1) k_karras<<<grid_for(n - 1), BLK, 0, st>>>(keys, (int)n, sc.children.p, sc.parent.p);
-    k_bottom_up<<<g, BLK, 0, st>>>(sorted, prim_lo, prim_hi, (int)n, sc.children.p, sc.parent.p, sc.flags.p,
-                                   sc.node_lo.p, sc.node_hi.p, sc.leaf_count.p);
-    SNK_TRY_CUDA(cudaGetLastError());
-    if (n >= (uint32_t)TL_LEAVES + 1) {
-        for (int pass = 0; pass < treelet_passes; pass++) {
-            SNK_TRY_CUDA(cudaMemsetAsync(sc.flags.p, 0, sizeof(int) * n, st));
-            k_treelet_pass<<<g, BLK, 0, st>>>((int)n, sc.children.p, sc.parent.p, sc.flags.p, sc.node_lo.p,
-                                              sc.node_hi.p, sc.leaf_count.p, sc.cost.p, leaf_max);
-            SNK_TRY_CUDA(cudaGetLastError());
-        }
-    }
-    return Status::Ok();
-}
-}  // namespace
-
-Status build_wide_bvh(BuildScratch& sc, const float4* prim_lo, const float4* prim_hi, uint32_t n, WideNode* nodes,
-                      uint32_t node_base, uint32_t prim_base, uint32_t* prim_order, cudaStream_t st,
-                      BuildResult* out, int treelet_passes, uint32_t leaf_max, uint32_t leaf_pack,
-                      bool sah_collapse) {
-    const uint32_t* sorted = nullptr;
-    SNK_TRY(build_binary_tree(sc, prim_lo, prim_hi, n, st, treelet_passes, leaf_max, leaf_pack, &sorted));
-    // SAH-optimal choice of each wide node's children (bottom-up over the final binary tree)
-    const uint32_t* wide_split = nullptr;
-    if (n > 1 && sah_collapse) {
-        SNK_TRY_CUDA(sc.wide_cost.reserve(8 * (size_t)(n - 1)));
-        SNK_TRY_CUDA(sc.wide_split.reserve(n - 1));
-        SNK_TRY_CUDA(cudaMemsetAsync(sc.flags.p, 0, sizeof(int) * n, st));
-        k_collapse_cost<<<grid_for(n), BLK, 0, st>>>((int)n, sc.children.p, sc.parent.p, sc.flags.p, sc.node_lo.p,
-                                                     sc.node_hi.p, sc.leaf_count.p, sc.wide_cost.p, sc.wide_split.p,
-                                                     leaf_max, leaf_pack);
-        SNK_TRY_CUDA(cudaGetLastError());
-        wide_split = sc.wide_split.p;
-    }
-    float4 rlo, rhi;
-    SNK_TRY_CUDA(cudaMemcpyAsync(&rlo, sc.node_lo.p, sizeof(float4), cudaMemcpyDeviceToHost, st));
-    SNK_TRY_CUDA(cudaMemcpyAsync(&rhi, sc.node_hi.p, sizeof(float4), cudaMemcpyDeviceToHost, st));
-    uint2 root_task = make_uint2(0u, node_base);
-    uint32_t init_ctr[5] = {1u, 0u, 1u, 0u, 0u};
-    SNK_TRY_CUDA(cudaMemcpyAsync(sc.tasks_a.p, &root_task, sizeof(uint2), cudaMemcpyHostToDevice, st));
-    SNK_TRY_CUDA(cudaMemcpyAsync(sc.counters.p, init_ctr, sizeof(init_ctr), cudaMemcpyHostToDevice, st));
-    SNK_TRY_CUDA(cudaMemsetAsync(sc.sah.p, 0, sizeof(double), st));
-    SNK_TRY_CUDA(cudaStreamSynchronize(st));
-    float rha = (rhi.x - rlo.x) * (rhi.y - rlo.y) + (rhi.y - rlo.y) * (rhi.z - rlo.z) + (rhi.z - rlo.z) * (rhi.x - rlo.x);
-    if (!(rha > 0.0f)) rha = 1.0f;
-
-    uint32_t ntasks = 1;
-    uint2* tin = sc.tasks_a.p;
-    uint2* tout = sc.tasks_b.p;
-    for (int level = 0; ntasks > 0; level++) {
-        if (level > 4096) return Status::Err(5, "build_wide_bvh: collapse did not terminate");
-        k_collapse<<<grid_for(ntasks), BLK, 0, st>>>(tin, sc.counters.p, tout, (int)n, sc.children.p, sc.node_lo.p,
-                                                     sc.node_hi.p, sc.leaf_count.p, sorted, nodes, node_base,
-                                                     prim_base, prim_order, sc.sah.p, rha, leaf_max, leaf_pack,
-                                                     wide_split);
-        SNK_TRY_CUDA(cudaGetLastError());
-        uint32_t ctr[5];
-        SNK_TRY_CUDA(cudaMemcpyAsync(ctr, sc.counters.p, sizeof(ctr), cudaMemcpyDeviceToHost, st));
-        SNK_TRY_CUDA(cudaStreamSynchronize(st));
-        if (ctr[4]) return Status::Err(5, "build_wide_bvh: collapse exceeded its capacity");
-        ntasks = ctr[1];
-        uint32_t next[2] = {ntasks, 0u};
-        SNK_TRY_CUDA(cudaMemcpyAsync(sc.counters.p, next, sizeof(next), cudaMemcpyHostToDevice, st));
-        std::swap(tin, tout);
-        if (ntasks == 0) {
-            if (ctr[3] != n) return Status::Err(2, "build_wide_bvh: primitive count mismatch");
-            out->num_nodes = ctr[2];
-        }
-    }
-    double sah = 0.0;
-    SNK_TRY_CUDA(cudaMemcpyAsync(&sah, sc.sah.p, sizeof(double), cudaMemcpyDeviceToHost, st));
-    SNK_TRY_CUDA(cudaStreamSynchronize(st));
-    out->sah = 1.0 + sah;
-    out->lo[0] = rlo.x; out->lo[1] = rlo.y; out->lo[2] = rlo.z;
-    out->hi[0] = rhi.x; out->hi[1] = rhi.y; out->hi[2] = rhi.z;
-    return Status::Ok();
-}
-
-Status build_wide_bvh_device(BuildScratch& sc, const float4* prim_lo, const float4* prim_hi, uint32_t n,
-                             WideNode* nodes, uint32_t node_base, uint32_t prim_base, uint32_t* prim_order,
-                             unsigned* err_word, cudaStream_t st, int treelet_passes, uint32_t leaf_max,
-                             uint32_t leaf_pack, SmallBuildOut* out, uint32_t* wide_depth, bool sah_collapse) {
-    const uint32_t* sorted = nullptr;
-    SNK_TRY(build_binary_tree(sc, prim_lo, prim_hi, n, st, treelet_passes, leaf_max, leaf_pack, &sorted));
-    const uint32_t* wide_split = nullptr;
-    if (n > 1 && sah_collapse) {
-        SNK_TRY_CUDA(sc.wide_cost.reserve(8 * (size_t)(n - 1)));
-        SNK_TRY_CUDA(sc.wide_split.reserve(n - 1));
-        SNK_TRY_CUDA(cudaMemsetAsync(sc.flags.p, 0, sizeof(int) * n, st));
-        k_collapse_cost<<<grid_for(n), BLK, 0, st>>>((int)n, sc.children.p, sc.parent.p, sc.flags.p, sc.node_lo.p,
-                                                     sc.node_hi.p, sc.leaf_count.p, sc.wide_cost.p, sc.wide_split.p,
-                                                     leaf_max, leaf_pack);
-        SNK_TRY_CUDA(cudaGetLastError());
-        wide_split = sc.wide_split.p;
-    }
     SNK_TRY_CUDA(sc.level_tasks.reserve(COLLAPSE_MAX_LEVELS + 1));
-    k_collapse_init<<<1, 128, 0, st>>>(sc.tasks_a.p, sc.counters.p, sc.level_tasks.p, node_base);
+
+    const unsigned g = grid_for(n);
+    SNK_TRY_CUDA(cudaMemsetAsync(sc.cbounds.p, 0, 6 * (size_t)B.count * sizeof(unsigned), st));
+    SNK_TRY_CUDA(cudaMemsetAsync(sc.flags.p, 0, sizeof(int) * n, st));
+    k_centroid_bounds<<<g, BLK, 0, st>>>(prim_lo, prim_hi, B, sc.cbounds.p);
+    const unsigned long long* keys = nullptr;
+    const uint32_t* sorted = nullptr;
+    SNK_TRY(sort_prims(sc, B, prim_lo, prim_hi, st, &keys, &sorted));
+    k_karras<<<g, BLK, 0, st>>>(keys, B, sc.children.p, sc.parent.p);
+    bool boxes = false;   // the tree's boxes and counts are in place
+    if (max_n >= (uint32_t)TL_LEAVES + 1) {
+        for (int pass = 0; pass < treelet_passes; pass++) {
+            if (boxes)
+                k_treelet_pass<false><<<g, BLK, 0, st>>>((int)n, sorted, prim_lo, prim_hi, sc.children.p, sc.parent.p,
+                                                         sc.flags.p, sc.node_lo.p, sc.node_hi.p, sc.leaf_count.p,
+                                                         sc.cost.p, leaf_max);
+            else
+                k_treelet_pass<true><<<g, BLK, 0, st>>>((int)n, sorted, prim_lo, prim_hi, sc.children.p, sc.parent.p,
+                                                        sc.flags.p, sc.node_lo.p, sc.node_hi.p, sc.leaf_count.p,
+                                                        sc.cost.p, leaf_max);
+            boxes = true;
+        }
+    }
+    const uint32_t* wide_split = nullptr;
+    if (sah_collapse) {   // SAH-optimal choice of each wide node's children over the final binary trees
+        SNK_TRY_CUDA(sc.wide_cost.reserve(8 * (size_t)n));
+        SNK_TRY_CUDA(sc.wide_split.reserve(n));
+        if (boxes)
+            k_collapse_cost<false><<<g, BLK, 0, st>>>((int)n, sorted, prim_lo, prim_hi, sc.children.p, sc.parent.p,
+                                                      sc.flags.p, sc.node_lo.p, sc.node_hi.p, sc.leaf_count.p,
+                                                      sc.wide_cost.p, sc.wide_split.p, leaf_max, leaf_pack);
+        else
+            k_collapse_cost<true><<<g, BLK, 0, st>>>((int)n, sorted, prim_lo, prim_hi, sc.children.p, sc.parent.p,
+                                                     sc.flags.p, sc.node_lo.p, sc.node_hi.p, sc.leaf_count.p,
+                                                     sc.wide_cost.p, sc.wide_split.p, leaf_max, leaf_pack);
+        wide_split = sc.wide_split.p;
+    } else if (!boxes) {
+        k_bottom_up<<<g, BLK, 0, st>>>(sorted, prim_lo, prim_hi, (int)n, sc.children.p, sc.parent.p, sc.flags.p,
+                                       sc.node_lo.p, sc.node_hi.p, sc.leaf_count.p);
+    }
+    SNK_TRY_CUDA(cudaGetLastError());
+    CollapseArgs A;
+    A.B = B;
+    A.tasks_a = sc.tasks_a.p; A.tasks_b = sc.tasks_b.p;
+    A.level_tasks = sc.level_tasks.p; A.counters = sc.counters.p;
+    A.children = sc.children.p; A.node_lo = sc.node_lo.p; A.node_hi = sc.node_hi.p;
+    A.leaf_count = sc.leaf_count.p; A.sorted = sorted; A.wide_split = wide_split;
+    A.nodes = nodes; A.node_base = node_base; A.prim_base = prim_base; A.prim_order = prim_order;
+    A.leaf_max = leaf_max; A.leaf_pack = leaf_pack; A.wide_depth = wide_depth;
+    A.sah = sah_cost ? sc.sah.p : nullptr;
+    k_collapse_init<<<(std::max(B.count, (uint32_t)COLLAPSE_MAX_LEVELS + 1u) + 255u) / 256u, 256, 0, st>>>(A);
     // enough warps for the widest level of a typical tree, at most 1024 blocks
     uint32_t grid = (n + 8u * LEVEL_WARPS - 1u) / (8u * LEVEL_WARPS);
     grid = grid < 1u ? 1u : (grid > 1024u ? 1024u : grid);
     // multi-block launches for about the depth of a balanced 8-wide tree; deeper
     // levels (unbalanced trees) go to the single-block finish
     int fast = 1;
-    for (uint64_t cap = 8; cap < n && fast < COLLAPSE_FAST_LEVELS; cap *= 8) fast++;
+    for (uint64_t cap = 8; cap < max_n && fast < COLLAPSE_FAST_LEVELS; cap *= 8) fast++;
     fast = fast + 1 < COLLAPSE_FAST_LEVELS ? fast + 1 : COLLAPSE_FAST_LEVELS;
-    for (int level = 0; level < fast; level++)
-        k_collapse_level<<<grid, 32 * LEVEL_WARPS, 0, st>>>(level, sc.tasks_a.p, sc.tasks_b.p, sc.level_tasks.p,
-                                                            sc.counters.p, (int)n, sc.children.p, sc.node_lo.p,
-                                                            sc.node_hi.p, sc.leaf_count.p, sorted, nodes, node_base,
-                                                            prim_base, prim_order, leaf_max, leaf_pack, wide_depth,
-                                                            wide_split);
-    k_collapse_finish<<<1, 1024, 0, st>>>(fast, sc.tasks_a.p, sc.tasks_b.p, sc.level_tasks.p,
-                                          sc.counters.p, (int)n, sc.children.p, sc.node_lo.p, sc.node_hi.p,
-                                          sc.leaf_count.p, sorted, nodes, node_base, prim_base, prim_order, leaf_max,
-                                          leaf_pack, err_word, wide_depth, out, wide_split);
+    for (int level = 0; level < fast; level++) k_collapse_level<<<grid, 32 * LEVEL_WARPS, 0, st>>>(A, level);
+    k_collapse_finish<<<1, 1024, 0, st>>>(A, fast, err_word, out);
     SNK_TRY_CUDA(cudaGetLastError());
     return Status::Ok();
 }
@@ -2006,16 +1875,19 @@ Status refit_wide_bvh(const float4* prim_lo, const float4* prim_hi, uint32_t n, 
     return Status::Ok();
 }
 
-Status launch_triangle_boxes(const float* positions, const uint32_t* indices, uint32_t vo, uint32_t io,
-                             uint32_t nt, float4* lo, float4* hi, cudaStream_t s) {
-    if (nt) k_triangle_boxes<<<grid_for(nt), BLK, 0, s>>>(positions, indices, vo, io, nt, lo, hi);
+Status launch_triangle_boxes(const float* positions, const uint32_t* indices, const BuildTrees& B,
+                             const uint32_t* tree_mesh, const MeshInfo* meshes, float4* lo, float4* hi, cudaStream_t s) {
+    if (B.total) k_triangle_boxes<<<grid_for(B.total), BLK, 0, s>>>(positions, indices, B, tree_mesh, meshes, lo, hi);
     SNK_TRY_CUDA(cudaGetLastError());
     return Status::Ok();
 }
 
-Status launch_fill_triangles(const uint32_t* order, uint32_t n, const float* positions, const uint32_t* indices,
-                             uint32_t vo, uint32_t io, TriRecord* out, cudaStream_t s) {
-    if (n) k_fill_triangles<<<grid_for(n), BLK, 0, s>>>(order, n, positions, indices, vo, io, out);
+Status launch_fill_triangles(const BuildScratch& sc, const uint32_t* order, const BuildTrees& B,
+                             const uint32_t* tree_mesh, uint32_t node_base, MeshInfo* meshes, const float* positions,
+                             const uint32_t* indices, TriRecord* out, cudaStream_t s) {
+    if (B.total)
+        k_fill_triangles<<<grid_for(B.total), BLK, 0, s>>>(order, B, tree_mesh, node_base, meshes, positions, indices,
+                                                           sc.node_lo.p, sc.node_hi.p, out);
     SNK_TRY_CUDA(cudaGetLastError());
     return Status::Ok();
 }

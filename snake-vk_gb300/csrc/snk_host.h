@@ -73,51 +73,48 @@ struct BuildScratch {
     DBuf<uint32_t> leaf_count;
     DBuf<float> cost;             // binary-tree SAH cost per node (treelet restructuring)
     DBuf<uint2> tasks_a, tasks_b;
-    DBuf<uint32_t> counters;      // [0] tasks in, [1] tasks out, [2] wide nodes, [3] prims
-    DBuf<unsigned> cbounds;       // centroid bounds, order-preserving encoded
-    DBuf<uint32_t> sort_hist;     // per-tile digit counts of the multi-CTA radix sort
+    DBuf<uint32_t> counters;      // [2] wide nodes, [3] prims, [4] error bits
+    DBuf<unsigned> cbounds;       // centroid bounds per tree, order-preserving encoded
+    DBuf<uint32_t> sort_hist;     // per-tile digit counts of the radix sort, every digit
     DBuf<double> sah;             // SAH accumulator
-    DBuf<uint32_t> level_tasks;   // task count per wide level (device-driven collapse)
+    DBuf<uint32_t> level_tasks;   // task count per wide level
     DBuf<float> wide_cost;        // 8 per binary internal node: SAH cost of its subtree in 1..8 wide children
     DBuf<uint32_t> wide_split;    // per binary internal node: the split of those children (4-bit fields)
-    size_t cap = 0;
 };
 
-struct BuildResult {
-    uint32_t num_nodes = 0;
-    float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-    double sah = 0.0;   // SAH cost of the wide BVH (internal 1, primitive 1, area relative to the root)
+// The trees of one build: tree t's primitives are [first[t], first[t + 1]) of the
+// concatenated boxes (device array of count + 1, each tree at least one primitive;
+// not read for a single tree)
+struct BuildTrees {
+    const uint32_t* first;
+    uint32_t count, total;
 };
-
-// Builds an 8-wide compressed BVH over n primitive boxes (prim_lo/prim_hi, xyz used).
-// Nodes are written at nodes[node_base + k] (root at node_base) with absolute child
-// indices; primitive slots are [prim_base, prim_base + n) and prim_order[k] receives
-// the primitive id stored in slot prim_base + k.
-Status build_wide_bvh(BuildScratch& sc, const float4* prim_lo, const float4* prim_hi, uint32_t n, WideNode* nodes,
-                      uint32_t node_base, uint32_t prim_base, uint32_t* prim_order, cudaStream_t stream,
-                      BuildResult* out, int treelet_passes, uint32_t leaf_max, uint32_t leaf_pack,
-                      bool sah_collapse = true);
 
 struct SmallBuildOut;
-// The same tree without host round trips (for per-frame rebuilds): the collapse
-// runs level by level on the device, nothing is read back, and a build error
-// (never seen for a correct tree) sets bit 8 of *err_word.  At most n + 1 nodes
-// are written.  With out and wide_depth (n + 1 entries) given, the device keeps
-// the node count, the deepest level and every node's depth for a later refit.
-Status build_wide_bvh_device(BuildScratch& sc, const float4* prim_lo, const float4* prim_hi, uint32_t n,
-                             WideNode* nodes, uint32_t node_base, uint32_t prim_base, uint32_t* prim_order,
-                             unsigned* err_word, cudaStream_t stream, int treelet_passes, uint32_t leaf_max,
-                             uint32_t leaf_pack, SmallBuildOut* out = nullptr, uint32_t* wide_depth = nullptr,
-                             bool sah_collapse = true);
+// Builds the 8-wide compressed BVHs of B's trees over their primitive boxes
+// (prim_lo/prim_hi, xyz used) without host round trips.  Tree t's root is
+// nodes[node_base + t], the other nodes follow with absolute child indices, at most
+// total + count nodes in all; primitive slots are [prim_base, prim_base + total) and
+// prim_order[k] receives the primitive (index of its box) stored in slot prim_base + k.
+// max_n: the largest tree's primitives.  A build error (never seen for a correct tree)
+// sets bit 8 of *err_word (when given) and out->error.  out (may be null) receives the
+// node count, the deepest level and, with sah_cost, the sum over the trees of
+// primitives x SAH cost below the root (internal 1, primitive 1, area relative to the
+// root); wide_depth (total + 1 entries, may be null) every node's depth: with it a
+// single tree can be refitted.
+Status build_wide_bvhs(BuildScratch& sc, const float4* prim_lo, const float4* prim_hi, const BuildTrees& B,
+                       uint32_t max_n, WideNode* nodes, uint32_t node_base, uint32_t prim_base, uint32_t* prim_order,
+                       unsigned* err_word, cudaStream_t stream, int treelet_passes, uint32_t leaf_max,
+                       uint32_t leaf_pack, SmallBuildOut* out, uint32_t* wide_depth, bool sah_collapse, bool sah_cost);
 
 // Single-launch build for n <= SMALL_BUILD_MAX primitives (one CTA, shared
-// memory, no host synchronisation); same algorithm and output layout as
-// build_wide_bvh.  The result record stays on the device.  A build error (never
+// memory, no host synchronisation); same collapse and output layout as
+// build_wide_bvhs.  The result record stays on the device.  A build error (never
 // seen for a correct tree) sets out->error and bit 8 of *err_word.
 constexpr int SMALL_BUILD_MAX = 1024;
 struct SmallBuildOut {
     uint32_t num_nodes, prims, error, max_depth;
-    double sah;   // not computed by the single-launch build (0)
+    double sah;   // not computed by the per-frame builds (0)
     float lo[4], hi[4];
 };
 // wide_box (2 x (n + 1) float4: exact lo, hi per wide node) and wide_depth
@@ -126,7 +123,7 @@ Status build_wide_bvh_small(const float4* prim_lo, const float4* prim_hi, uint32
                             uint32_t node_base, uint32_t prim_base, uint32_t* prim_order, int treelet_passes,
                             SmallBuildOut* out, unsigned* err_word, float4* wide_box, uint32_t* wide_depth,
                             cudaStream_t stream, uint32_t leaf_max, bool sah_collapse = true);
-// Refit of a tree made by build_wide_bvh_small or build_wide_bvh_device (with its
+// Refit of a tree made by build_wide_bvh_small or build_wide_bvhs (one tree, with its
 // record and depths) for the same n primitives in new boxes (prim_order as that
 // build wrote it; wide_box: 2 x (n + 1) float4 of scratch that receives every
 // node's exact box; everything stays on the device).
@@ -134,12 +131,14 @@ Status refit_wide_bvh(const float4* prim_lo, const float4* prim_hi, uint32_t n, 
                       uint32_t prim_base, const uint32_t* prim_order, const SmallBuildOut* info, float4* wide_box,
                       const uint32_t* wide_depth, unsigned* err_word, cudaStream_t stream);
 
-// Per-triangle padded boxes of one mesh (object space).
-Status launch_triangle_boxes(const float* positions, const uint32_t* indices, uint32_t vertex_offset,
-                             uint32_t index_offset, uint32_t num_tris, float4* lo, float4* hi, cudaStream_t s);
-// Triangle records of one mesh from the build's primitive order.
-Status launch_fill_triangles(const uint32_t* prim_order, uint32_t n, const float* positions, const uint32_t* indices,
-                             uint32_t vertex_offset, uint32_t index_offset, TriRecord* out, cudaStream_t s);
+// Padded object-space boxes of the triangles of B's meshes (tree t is mesh tree_mesh[t]).
+Status launch_triangle_boxes(const float* positions, const uint32_t* indices, const BuildTrees& B,
+                             const uint32_t* tree_mesh, const MeshInfo* meshes, float4* lo, float4* hi, cudaStream_t s);
+// Triangle records from the build's primitive order, and the meshes' root nodes
+// (node_base + t) and bounds (after the build that left its trees in sc).
+Status launch_fill_triangles(const BuildScratch& sc, const uint32_t* prim_order, const BuildTrees& B,
+                             const uint32_t* tree_mesh, uint32_t node_base, MeshInfo* meshes, const float* positions,
+                             const uint32_t* indices, TriRecord* out, cudaStream_t s);
 // World boxes of the listed instances (transform of the mesh bounds) for the instance BVH.
 Status launch_instance_boxes(const uint32_t* inst_list, uint32_t n, const InstShade* inst, const MeshInfo* meshes,
                              float4* lo, float4* hi, cudaStream_t s);

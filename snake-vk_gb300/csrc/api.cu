@@ -634,12 +634,17 @@ int shade_grid(snk_pt_ctx* ctx) { return grid_of(ctx, ctx->tune.shade_blocks_per
 int any_grid(snk_pt_ctx* ctx) {
     return ctx->tune.shadow_blocks_per_sm ? grid_of(ctx, (int)ctx->tune.shadow_blocks_per_sm) : trace_grid(ctx);
 }
+// warps of a traversal kernel's register variant that the GPU holds at once (4 per block)
+uint32_t resident_warps(snk_pt_ctx* ctx, uint32_t variant) {
+    return (uint32_t)ctx->num_sms * 4u * (variant == 1 ? 8u : (variant == 2 ? 4u : 6u));
+}
 TraceTuning trace_tuning(snk_pt_ctx* ctx) {
     TraceTuning t;
     t.chunk = ctx->tune.ray_chunk;
     t.refill_idle = ctx->tune.refill_idle;
     t.prim_bias = ctx->tune.prim_bias;
     t.variant = ctx->tune.trace_variant;
+    t.warps = resident_warps(ctx, t.variant);
     return t;
 }
 // knobs of the any-hit kernels: each falls back to the closest-hit knob when 0
@@ -650,6 +655,7 @@ TraceTuning any_tuning(snk_pt_ctx* ctx) {
     if (k.shadow_refill_idle) t.refill_idle = k.shadow_refill_idle;
     if (k.shadow_prim_bias) t.prim_bias = k.shadow_prim_bias;
     if (k.shadow_variant) t.variant = k.shadow_variant - 1u;
+    t.warps = resident_warps(ctx, t.variant);
     return t;
 }
 

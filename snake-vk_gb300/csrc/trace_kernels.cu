@@ -2,8 +2,8 @@
 //
 // One lane traces one ray.  Warps are persistent (the grid is a fixed multiple
 // of the SM count and the number of rays is read on the device, which keeps the
-// frame capturable in a CUDA graph).  Each warp takes chunks of CHUNK rays from
-// a global counter and, between traversal steps, hands a new ray to every lane
+// frame capturable in a CUDA graph).  Each warp takes chunks of rays from
+// a global counter (Knobs) and, between traversal steps, hands a new ray to every lane
 // whose ray has finished, so lanes do not idle until the warp's longest ray ends
 // (Aila & Laine, HPG 2009, persistent threads with ray replacement).  The short
 // traversal stack of every lane lives in shared memory (STACK_SH entries) with a
@@ -17,13 +17,34 @@ namespace {
 
 constexpr int TBLK = 128;
 
+// Launch knobs of a queue of n rays.  At each fetch a warp takes a quarter
+// of its share of the rays that are left: the knob's 64 while the queue is long (few
+// atomics, neighbouring rays in one warp), less towards its end, so that the warps finish
+// together; but at least four times its share of the whole queue up to a warp's 32
+// rays (a small queue fills warps with neighbours), and one ray per warp when there
+// are fewer rays than that.  With always 64 the queue's end, and any queue of
+// fewer rays than 64 per resident warp (233,472), left most warps without work: 64
+// rays traced by one warp took 0.54 ms, one warp each 0.08 ms; a 65,536-path room frame
+// 0.407 and 0.312 ms, the small 8-view terrain batch 2.37 and 1.60 ms, 1080p 2.19
+// and 2.12 ms.  (Caps on the lanes that take rays, and asking for the next chunk
+// ahead, gained nothing.)
+constexpr uint32_t CHUNK_MAX = 64, CHUNK_MIN = 32;
+
 struct Knobs {
-    uint32_t chunk;
+    uint32_t chunk, chunk_min;
+    float share;      // chunk per ray left
     int refill_idle;
     uint32_t prim_bias;
-    __device__ __forceinline__ explicit Knobs(const TraceTuning& t)
-        : chunk(t.chunk ? t.chunk : 64u), refill_idle(t.refill_idle ? (int)t.refill_idle : 4),
-          prim_bias(t.prim_bias ? t.prim_bias : 4u) {}
+    __device__ __forceinline__ Knobs(const TraceTuning& t, uint32_t n)
+        : chunk(t.chunk ? t.chunk : CHUNK_MAX), share(0.25f / (float)t.warps),
+          refill_idle(t.refill_idle ? (int)t.refill_idle : 4), prim_bias(t.prim_bias ? t.prim_bias : 4u) {
+        const uint32_t c = (uint32_t)((float)n * (16.0f * share));
+        chunk_min = min(max(c, 1u), min(CHUNK_MIN, chunk));
+    }
+    // the chunk to take when at most `left` rays are left
+    __device__ __forceinline__ uint32_t next_chunk(uint32_t left) const {
+        return min(max((uint32_t)((float)left * share), chunk_min), chunk);
+    }
 };
 
 // One warp-voted traversal step: every active lane first pops until it has work
@@ -66,9 +87,10 @@ struct RayFeed {
     // Assigns new indices to the idle lanes (mask `idle`); returns this lane's index
     // or INVALID.  Must be called by the whole warp.
     __device__ __forceinline__ uint32_t refill(unsigned idle, uint32_t lane, uint32_t* work, uint32_t n,
-                                               uint32_t chunk) {
+                                               const Knobs& kn) {
         if (next >= end && !exhausted) {
             uint32_t b = 0;
+            const uint32_t chunk = kn.next_chunk(n - end);
             if (lane == 0) b = atomicAdd(work, chunk);
             b = __shfl_sync(0xFFFFFFFFu, b, 0);
             if (b >= n) {
@@ -92,9 +114,9 @@ struct RayFeed {
 // closest hit of the rays queued for segment d
 template <bool COUNT, int MINB, bool SINGLE>
 __global__ void __launch_bounds__(TBLK, MINB) k_trace_closest(FrameParams F, uint32_t d) {
-    const Knobs kn(F.tune);
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     const uint32_t n = F.counters[CNT_QUEUE + d];
+    const Knobs kn(F.tune, n);
     const float4* rays = F.rays[d & 1u];
     uint32_t* work = &F.counters[CNT_WORK_TRACE + d];
     const uint32_t lane = threadIdx.x & 31u;
@@ -108,7 +130,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_closest(FrameParams F, uin
     for (;;) {
         unsigned act = __ballot_sync(0xFFFFFFFFu, active);
         if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t i = feed.refill(~act, lane, work, n, kn.chunk);
+            uint32_t i = feed.refill(~act, lane, work, n, kn);
             if (i != INVALID) {
                 float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
                 tv.init(F.S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
@@ -177,9 +199,9 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_packet(FrameParams F, uint
 // (the same order as the CPU oracle, so sums are bit-identical).
 template <bool COUNT, int MINB, bool SINGLE>
 __global__ void __launch_bounds__(TBLK, MINB) k_trace_shadow(FrameParams F, uint32_t d) {
-    const Knobs kn(F.tune_any);
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     const uint32_t n0 = F.counters[CNT_SHADOW_Q + 2 * d], n = n0 + F.counters[CNT_SHADOW_Q + 2 * d + 1];
+    const Knobs kn(F.tune_any, n);
     uint32_t* work = &F.counters[CNT_WORK_SHADOW + d];
     const uint32_t lane = threadIdx.x & 31u;
     TraceCounters ctr{0ull, 0ull};
@@ -192,7 +214,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_shadow(FrameParams F, uint
     for (;;) {
         unsigned act = __ballot_sync(0xFFFFFFFFu, active);
         if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t j = feed.refill(~act, lane, work, n, kn.chunk);
+            uint32_t j = feed.refill(~act, lane, work, n, kn);
             if (j != INVALID) {
                 const size_t e = j < n0 ? (size_t)j : (size_t)F.n_paths + (j - n0);
                 const float4* sr = F.shadow_rays + 2 * e;
@@ -271,11 +293,11 @@ struct FilteredFeed {
     RayFeed raw;
     uint32_t head, cnt;   // the ring's pending entries (warp-uniform)
     __device__ __forceinline__ void init() { raw.init(); head = 0; cnt = 0; }
-    __device__ __forceinline__ uint32_t refill(unsigned idle, uint32_t lane, uint32_t* work, uint32_t n, uint32_t chunk,
+    __device__ __forceinline__ uint32_t refill(unsigned idle, uint32_t lane, uint32_t* work, uint32_t n, const Knobs& kn,
                                                const float4* rays, uint32_t* ring) {
         const uint32_t nidle = (uint32_t)__popc(idle), lt = (1u << lane) - 1u;
         while (cnt < nidle && !raw.done()) {   // (cnt < 32 here, so the ring of 64 never overflows)
-            const uint32_t e = raw.refill(0xFFFFFFFFu, lane, work, n, chunk);
+            const uint32_t e = raw.refill(0xFFFFFFFFu, lane, work, n, kn);
             const bool real = e != INVALID && __ldg(reinterpret_cast<const float*>(rays + 2ull * e + 1) + 3) >= 0.0f;
             const unsigned rm = __ballot_sync(0xFFFFFFFFu, real);
             if (real) ring[(head + cnt + (uint32_t)__popc(rm & lt)) & 63u] = e;
@@ -302,7 +324,7 @@ template <int MINB, bool SINGLE>
 __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(SceneDev S, const float4* __restrict__ rays,
                                                                  uint32_t n, uint8_t* vis, uint32_t* work,
                                                                  TraceTuning tune) {
-    const Knobs kn(tune);
+    const Knobs kn(tune, n);
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     __shared__ uint32_t ring[TBLK / 32][64];
     const uint32_t lane = threadIdx.x & 31u;
@@ -315,7 +337,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(SceneDev S, con
     for (;;) {
         unsigned act = __ballot_sync(0xFFFFFFFFu, active);
         if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t i = feed.refill(~act, lane, work, n, kn.chunk, rays, ring[threadIdx.x >> 5]);
+            uint32_t i = feed.refill(~act, lane, work, n, kn, rays, ring[threadIdx.x >> 5]);
             if (i != INVALID) {
                 const float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
                 tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
@@ -340,7 +362,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(SceneDev S, con
 template <bool ANY, bool SINGLE>
 __global__ void __launch_bounds__(TBLK, 6) k_trace_rays(SceneDev S, const float4* __restrict__ rays, uint32_t n,
                                                      HitDev* hits, uint32_t* work, TraceTuning tune) {
-    const Knobs kn(tune);
+    const Knobs kn(tune, n);
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     const uint32_t lane = threadIdx.x & 31u;
     Traverser<ANY, false, SINGLE> tv;
@@ -352,7 +374,7 @@ __global__ void __launch_bounds__(TBLK, 6) k_trace_rays(SceneDev S, const float4
     for (;;) {
         unsigned act = __ballot_sync(0xFFFFFFFFu, active);
         if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t i = feed.refill(~act, lane, work, n, kn.chunk);
+            uint32_t i = feed.refill(~act, lane, work, n, kn);
             if (i != INVALID) {
                 float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
                 tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);

@@ -1313,13 +1313,12 @@ int render_impl(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, cons
                 return fail(ctx, SNK_ERR_CUDA, "restir queue reset");
             const RestirQueue q1{ctx->rq_rays.p, ctx->rq_vis_a.p, K1, (uint32_t)np},
                 q2{ctx->rq_rays.p, ctx->rq_vis_b.p, K2, (uint32_t)np}, q3{ctx->rq_rays.p, ctx->rq_vis_a.p, K3, (uint32_t)np};
-            const int tg = trace_grid(ctx);
             const SceneDev SD = scene_dev(ctx);
             const TraceTuning tt = any_tuning(ctx);
             const int ta = any_grid(ctx);
             auto pass = [&](int stage, int phase, const RestirQueue& qa, const RestirQueue& qb) {
                 return staged(ctx, profile, SNK_STAGE_RESTIR_GBUFFER + stage,
-                              [&] { return launch_restir_stage(stage, phase, F, v, RV, s, qa, qb, tg, st); });
+                              [&] { return launch_restir_stage(stage, phase, F, v, RV, s, qa, qb, st); });
             };
             auto visibility = [&](uint32_t K, uint8_t* vis, int slot) {
                 return staged(ctx, profile, SNK_STAGE_TRACE_SHADOW, [&] {

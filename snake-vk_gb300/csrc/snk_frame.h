@@ -173,7 +173,7 @@ constexpr uint32_t RESTIR_SHADE_SLOTS = 2;
 //          writes the spatial reservoirs and records qs's (final shading) rays;
 //          phase 2 replays the sun ray of q and qs, writes the frame's outputs
 cudaError_t launch_restir_stage(int stage, int phase, const FrameParams& F, uint32_t view_index, const RestirView& R,
-                                const RestirSettings& rs, const RestirQueue& q, const RestirQueue& qs, int grid,
+                                const RestirSettings& rs, const RestirQueue& q, const RestirQueue& qs,
                                 cudaStream_t s);
 
 // Read-only view of a context (defined in api.cu) for entry points that live in

@@ -743,26 +743,36 @@ __device__ __forceinline__ uint32_t ceil_exp_biased(float x) {
 
 // 8-bit child-box quantisation of a wide node: a power-of-two scale per axis
 // (the smallest with 255 steps covering the parent box, rounded up) and child
-// planes rounded outwards, so the decoded boxes always contain the exact ones.
+// planes rounded outwards by at least QUANT_PAD of a step, which covers the rounding of
+// the traversal's plane offsets (box_hits); the decoded boxes contain the exact ones.
+// The grid starts 1/16 of a step (of the unpadded grid) below the box, rounded down,
+// so that the lowest planes have their pad too: where the subtraction is exact the
+// step is at most doubled by it, where it is not the origin moves by an ulp u of the
+// box's corner, and the step, at most 2 (255 x 16 u + u) / 254.75, stays below 64 u.
+constexpr float QUANT_PAD = 1.0f / 64.0f;
+constexpr uint32_t QUANT_EXP_BIAS = 15;   // the stored exponents carry the traversal's 2^15
 struct QuantFrame {
     float p[3], inv_scale[3];
-    uint32_t eb[3];
+    uint32_t eb[3];   // stored exponent bytes
 };
 __device__ __forceinline__ QuantFrame quant_frame(float4 plo, float4 phi) {
     QuantFrame F;
-    const float ex_[3] = {__fsub_ru(phi.x, plo.x), __fsub_ru(phi.y, plo.y), __fsub_ru(phi.z, plo.z)};
-    F.p[0] = plo.x; F.p[1] = plo.y; F.p[2] = plo.z;
+    const float lo[3] = {plo.x, plo.y, plo.z}, hi[3] = {phi.x, phi.y, phi.z};
     for (int a = 0; a < 3; a++) {
-        F.eb[a] = ceil_exp_biased(__fdiv_ru(ex_[a], 255.0f));
-        F.inv_scale[a] = __uint_as_float((254u - F.eb[a]) << 23);   // 2^(127 - (eb - 127))
+        const uint32_t e0 = ceil_exp_biased(__fdiv_ru(__fsub_ru(hi[a], lo[a]), 255.0f));
+        F.p[a] = __fsub_rd(lo[a], __uint_as_float(e0 << 23) * 0.0625f);
+        const uint32_t e1 = ceil_exp_biased(__fdiv_ru(__fsub_ru(hi[a], F.p[a]), 254.75f));
+        const uint32_t e = min(max(e0, e1), 254u - QUANT_EXP_BIAS);
+        F.eb[a] = e + QUANT_EXP_BIAS;
+        F.inv_scale[a] = __uint_as_float((254u - e) << 23);   // 2^(127 - e)
     }
     return F;
 }
 __device__ __forceinline__ void quant_child(const QuantFrame& F, float4 a4, float4 z4, WideNode& node, int s) {
     const float clo[3] = {a4.x, a4.y, a4.z}, chi[3] = {z4.x, z4.y, z4.z};
     for (int a = 0; a < 3; a++) {
-        const float ql = floorf(__fmul_rd(__fsub_rd(clo[a], F.p[a]), F.inv_scale[a]));
-        const float qh = ceilf(__fmul_ru(__fsub_ru(chi[a], F.p[a]), F.inv_scale[a]));
+        const float ql = floorf(__fadd_rd(__fmul_rd(__fsub_rd(clo[a], F.p[a]), F.inv_scale[a]), -QUANT_PAD));
+        const float qh = ceilf(__fadd_ru(__fmul_ru(__fsub_ru(chi[a], F.p[a]), F.inv_scale[a]), QUANT_PAD));
         node.qlo[a][s] = (uint8_t)fminf(fmaxf(ql, 0.0f), 255.0f);
         node.qhi[a][s] = (uint8_t)fminf(fmaxf(qh, 0.0f), 255.0f);
     }
@@ -1103,7 +1113,7 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
     task_base = __shfl_sync(FULL, task_base, 0);
     const QuantFrame F = quant_frame(plo, phi);
     if (lane == 0) {
-        stage->px = plo.x; stage->py = plo.y; stage->pz = plo.z;
+        stage->px = F.p[0]; stage->py = F.p[1]; stage->pz = F.p[2];
         stage->ex = (uint8_t)F.eb[0]; stage->ey = (uint8_t)F.eb[1]; stage->ez = (uint8_t)F.eb[2];
         stage->imask = (uint8_t)(int_mask & 0xFFu);
         stage->child_base = node_base + child_local;
@@ -1619,7 +1629,7 @@ k_refit_small(WideNode* nodes, uint32_t node_base, uint32_t prim_base, const Sma
             }
             if (bad) { atomicOr(err_word, 8u); continue; }
             const QuantFrame F = quant_frame(lo, hi);
-            node.px = lo.x; node.py = lo.y; node.pz = lo.z;
+            node.px = F.p[0]; node.py = F.p[1]; node.pz = F.p[2];
             node.ex = (uint8_t)F.eb[0]; node.ey = (uint8_t)F.eb[1]; node.ez = (uint8_t)F.eb[2];
             for (int s = 0; s < 8; s++) {
                 if (node.meta[s] == 0u) continue;

@@ -214,7 +214,7 @@ SNK_HD V3 f0_of(V3 albedo, float metallic) {
 // --------------------------------------------------------------------------
 // 8-wide compressed BVH node (80 bytes = 5 x 16 B), the compressed wide node of
 // Ylitie, Karras, Laine (HPG 2017): child boxes quantised to 8 bits per plane
-// relative to origin p with per-axis power-of-two scales 2^(e-127).
+// relative to origin p with per-axis power-of-two scales 2^(e-15-127).
 //   w0: p.x p.y p.z | e.x e.y e.z imask (bytes)
 //   w1: child_base  | prim_base | meta[0..3] | meta[4..7]
 //   w2: qlo_x[8] qlo_y[8]   w3: qlo_z[8] qhi_x[8]   w4: qhi_y[8] qhi_z[8]

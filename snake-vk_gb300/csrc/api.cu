@@ -629,7 +629,7 @@ void** dev_slots(ViewDev& v) { return reinterpret_cast<void**>(&v.radiance); }
 
 int grid_of(snk_pt_ctx* ctx, int per_sm) { return ctx->num_sms * per_sm; }
 int trace_grid(snk_pt_ctx* ctx) { return grid_of(ctx, ctx->tune.trace_blocks_per_sm ? (int)ctx->tune.trace_blocks_per_sm : 16); }
-int shade_grid(snk_pt_ctx* ctx) { return grid_of(ctx, ctx->tune.shade_blocks_per_sm ? (int)ctx->tune.shade_blocks_per_sm : 8); }
+int shade_grid(snk_pt_ctx* ctx) { return grid_of(ctx, ctx->tune.shade_blocks_per_sm ? (int)ctx->tune.shade_blocks_per_sm : 4); }
 // any-hit traversal grid (shadow and visibility rays): its own knob, else the closest-hit one
 int any_grid(snk_pt_ctx* ctx) {
     return ctx->tune.shadow_blocks_per_sm ? grid_of(ctx, (int)ctx->tune.shadow_blocks_per_sm) : trace_grid(ctx);
@@ -1466,10 +1466,10 @@ int snk_pt_autotune(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, 
     };
     snk_tuning cur = ctx->tune;
     if (!cur.trace_blocks_per_sm) cur.trace_blocks_per_sm = 16;
-    if (!cur.shade_blocks_per_sm) cur.shade_blocks_per_sm = 8;
+    if (!cur.shade_blocks_per_sm) cur.shade_blocks_per_sm = 4;
     if (!cur.ray_chunk) cur.ray_chunk = 64;
     if (!cur.refill_idle) cur.refill_idle = 4;
-    if (!cur.prim_bias) cur.prim_bias = 4;
+    if (!cur.prim_bias) cur.prim_bias = 3;
     double best_ms = 0.0;
     int rc = trial(cur, &best_ms);
     if (rc) return rc;
@@ -1481,7 +1481,7 @@ int snk_pt_autotune(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, 
             {&cand.trace_variant, {0, 1, 2}},
             {&cand.refill_idle, {1, 2, 4, 8, 16}},
             {&cand.ray_chunk, {32, 64, 128, 256}},
-            {&cand.prim_bias, {2, 4, 8}},
+            {&cand.prim_bias, {2, 3, 4, 8}},
             {&cand.shade_blocks_per_sm, {4, 8, 16}},
         };
         for (Knob& k : knobs) {

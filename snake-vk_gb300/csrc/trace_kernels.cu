@@ -37,7 +37,7 @@ struct Knobs {
     uint32_t prim_bias;
     __device__ __forceinline__ Knobs(const TraceTuning& t, uint32_t n)
         : chunk(t.chunk ? t.chunk : CHUNK_MAX), share(0.25f / (float)t.warps),
-          refill_idle(t.refill_idle ? (int)t.refill_idle : 4), prim_bias(t.prim_bias ? t.prim_bias : 4u) {
+          refill_idle(t.refill_idle ? (int)t.refill_idle : 4), prim_bias(t.prim_bias ? t.prim_bias : 3u) {
         const uint32_t c = (uint32_t)((float)n * (16.0f * share));
         chunk_min = min(max(c, 1u), min(CHUNK_MIN, chunk));
     }

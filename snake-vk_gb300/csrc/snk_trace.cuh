@@ -87,6 +87,9 @@ __device__ __forceinline__ float byte_m(uint32_t w, uint32_t k) {
     return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | (k << 4)));
 }
 
+// a plane byte as byte_m decodes it
+__device__ __forceinline__ float byte_f(uint32_t q) { return __uint_as_float(0x3F800000u | (q << 8)); }
+
 // Box tests of the 8 children of a node (words w0, w2, w3, w4) against ray r on
 // [tmin, tmax]: bit s of the result is set when the box of slot s is hit.
 // Near/far planes are swapped once per node by the ray octant; each plane costs a
@@ -217,6 +220,23 @@ struct ShortStack {
     }
 };
 
+// Result of a finished ray (T: its traversal state); traversal errors are reported
+// through the scene's error word and read as a miss.
+template <class T>
+__device__ __forceinline__ bool ray_result(const T& v, const SceneDev& S, TraceResult& res) {
+    res.hit = false;
+    res.t = -1.0f; res.u = 0.0f; res.v = 0.0f; res.inst = INVALID; res.prim = INVALID;
+    if (v.err) {
+        if (S.error_word) atomicOr(S.error_word, v.err);
+        return false;
+    }
+    if (v.best_inst != INVALID) {
+        res.hit = true;
+        res.t = v.best_t; res.inst = v.best_inst; res.prim = v.best_prim; res.u = v.best_u; res.v = v.best_v;
+    }
+    return res.hit;
+}
+
 // Resumable traversal state of one ray.  The work is split into single units so
 // a warp can vote each iteration which kind of unit its lanes execute together:
 //   node_step()  intersect one internal child of the current node group
@@ -314,6 +334,31 @@ struct Traverser {
         intersect_node<ORD, SINGLE>(level ? S.blas_nodes : S.tlas_nodes, child, cr, tmin, best_t, ngroup, tgroup);
     }
 
+    // enters the instance of instance-BVH primitive pidx (what is left of the instance
+    // level is on the stack)
+    __device__ __forceinline__ void enter_instance(const SceneDev& S, uint32_t pidx) {
+        if (pidx >= S.num_tlas_prims) { fail(ERR_BAD_INDEX); return; }
+        const uint32_t inst = __ldg(&S.tlas_prims[pidx]);
+        if (inst >= S.num_instances) { fail(ERR_BAD_INDEX); return; }
+        const float4* ip = reinterpret_cast<const float4*>(S.inst_trace + inst);
+        float4 r0 = __ldg(ip), r1 = __ldg(ip + 1), r2 = __ldg(ip + 2);
+        uint32_t root = __ldg(reinterpret_cast<const uint32_t*>(ip + 3));
+        float inv[12] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w};
+        V3 o, d;
+        world_ray(o, d);
+        V3 oo = xform_point_rn(inv, o);
+        V3 od = xform_dir_rn(inv, d);
+        cr = make_node_ray(oo, od);
+        // the watertight set-up waits for the instance's first triangle test (many
+        // instances are left without one); until then its shear slots hold the direction
+        tr.k = INVALID; tr.Sx = od.x; tr.Sy = od.y; tr.Sz = od.z;
+        blas_sp = st.sp;
+        level = 1;
+        cur_inst = inst;
+        ngroup = make_uint2(root, (1u << (24 + (ORD ? cr.oct : 0u))) | 1u);
+        tgroup = make_uint2(0u, 0u);
+    }
+
     __device__ __forceinline__ void prim_step(const SceneDev& S, TraceCounters* ctr) {
         if (++steps > S.max_steps) { fail(ERR_STEP_LIMIT); return; }
         uint32_t pidx;
@@ -327,32 +372,13 @@ struct Traverser {
             pidx = tgroup.x + k;
         }
         if (level == 0) {
-            if (pidx >= S.num_tlas_prims) { fail(ERR_BAD_INDEX); return; }
-            uint32_t inst = __ldg(&S.tlas_prims[pidx]);
-            if (inst >= S.num_instances) { fail(ERR_BAD_INDEX); return; }
             if (has_prim()) {
                 if (!st.push(make_uint2(tgroup.x | PRIM_GROUP, tgroup.y))) { fail(ERR_STACK_OVERFLOW); return; }
             }
             if (has_node()) {
                 if (!st.push(ngroup)) { fail(ERR_STACK_OVERFLOW); return; }
             }
-            const float4* ip = reinterpret_cast<const float4*>(S.inst_trace + inst);
-            float4 r0 = __ldg(ip), r1 = __ldg(ip + 1), r2 = __ldg(ip + 2);
-            uint32_t root = __ldg(reinterpret_cast<const uint32_t*>(ip + 3));
-            float inv[12] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w};
-            V3 o, d;
-            world_ray(o, d);
-            V3 oo = xform_point_rn(inv, o);
-            V3 od = xform_dir_rn(inv, d);
-            cr = make_node_ray(oo, od);
-            // the watertight set-up waits for the instance's first triangle test (many
-            // instances are left without one); until then its shear slots hold the direction
-            tr.k = INVALID; tr.Sx = od.x; tr.Sy = od.y; tr.Sz = od.z;
-            blas_sp = st.sp;
-            level = 1;
-            cur_inst = inst;
-            ngroup = make_uint2(root, (1u << (24 + (ORD ? cr.oct : 0u))) | 1u);
-            tgroup = make_uint2(0u, 0u);
+            enter_instance(S, pidx);
         } else {
             if (pidx >= S.num_tris) { fail(ERR_BAD_INDEX); return; }
             if (COUNT) ctr->tris++;
@@ -373,21 +399,195 @@ struct Traverser {
         }
     }
 
-    // Result once done; traversal errors are reported through the scene's
-    // error word and read as a miss.
-    __device__ __forceinline__ bool finish(const SceneDev& S, TraceResult& res) {
-        res.hit = false;
-        res.t = -1.0f; res.u = 0.0f; res.v = 0.0f; res.inst = INVALID; res.prim = INVALID;
-        if (err) {
-            if (S.error_word) atomicOr(S.error_word, err);
-            return false;
-        }
-        if (best_inst != INVALID) {
-            res.hit = true; res.t = best_t; res.inst = best_inst; res.prim = best_prim; res.u = best_u; res.v = best_v;
-        }
-        return res.hit;
-    }
+    __device__ __forceinline__ bool finish(const SceneDev& S, TraceResult& res) { return ray_result(*this, S, res); }
 };
+
+// ---- eight lanes per ray -----------------------------------------------------------
+// The last rays of a queue, and the rays of a queue too small to fill the GPU, are bound
+// by the latency of their dependent steps, not by issue: a warp with at most
+// COOP_RAYS rays gives eight lanes to each.  A lane tests one child of a node, or the
+// triangle of one leaf slot, and the lanes vote; everything else they do alike.  Hits
+// equal the one-lane traversal's: boxes only cull, and the closest hit is the minimum
+// of the tested triangles in the same (t, instance, triangle) order.  A ray gets there
+// through a slot in shared memory (coop_save), so that the code that follows keeps no
+// registers of the one-lane loop alive.  Its stack moves into the warp's shared stack
+// rows, of which a group's eight columns hold the STACK_MAX entries (the finished rays
+// no longer need theirs); its world-ray rows stay in its owner's column.  For
+// single-primitive-leaf trees.
+constexpr int COOP_RAYS = 4;
+static_assert(STACK_SH * 8 >= STACK_MAX, "eight columns of the shared stack hold a whole stack");
+
+struct CoopSlot {   // (the result comes back in best_*, the error bits in err)
+    float tmin, tmax;
+    NodeRay cr;
+    WRay tr;
+    float best_t, best_u, best_v;
+    uint32_t best_inst, best_prim;
+    uint2 ngroup, tgroup;
+    int level, blas_sp, sp;
+    uint32_t cur_inst, steps, ri, tid;
+    unsigned err;
+};
+
+// an unfinished ray of this thread into a slot
+template <class TV>
+__device__ __forceinline__ void coop_save(CoopSlot& c, const TV& tv, uint32_t ri) {
+    c.tmin = tv.tmin; c.tmax = tv.tmax;
+    c.cr = tv.cr;
+    c.tr = tv.tr;
+    c.best_t = tv.best_t; c.best_u = tv.best_u; c.best_v = tv.best_v;
+    c.best_inst = tv.best_inst; c.best_prim = tv.best_prim;
+    c.ngroup = tv.ngroup; c.tgroup = tv.tgroup;
+    c.level = tv.level; c.blas_sp = tv.blas_sp; c.sp = tv.st.sp;
+    c.cur_inst = tv.cur_inst; c.steps = tv.steps; c.ri = ri; c.tid = threadIdx.x;
+}
+
+// Finishes the k <= COOP_RAYS rays saved in the warp's slots (all 32 lanes call this;
+// spill: the one-lane traversal's local stack entries).  A call, so that the one-lane
+// loops keep their registers (inlined, they spilled and big queues took 2 to 5 % longer).
+template <bool ANY>
+__device__ __noinline__ void coop_trace(CoopSlot* slots, uint32_t k_rays, const SceneDev& S, uint2* sh_stack,
+                                        const uint2* spill, uint32_t nthreads) {
+    using TV = Traverser<ANY, false, true>;
+    TV tv;
+    const uint32_t lane = threadIdx.x & 31u, base = threadIdx.x & ~31u, g = lane >> 3, slot = lane & 7u;
+    auto entry = [&](uint32_t group, int e) -> uint2& {   // stack entry e of a group
+        return sh_stack[(uint32_t)(e & 7) * nthreads + base + 8u * group + (uint32_t)(e >> 3)];
+    };
+    const bool valid = g < k_rays;
+    __syncwarp();   // the slots are complete
+    {   // the stacks into the groups' columns: first the entries in shared rows (entry `slot`
+        // of this lane's group), once all are read, then the owners' local ones
+        uint2 v = make_uint2(0u, 0u);
+        const bool move = valid && (int)slot < slots[g].sp;
+        if (move) v = sh_stack[slot * nthreads + slots[g].tid];
+        __syncwarp();
+        if (move) entry(g, (int)slot) = v;
+        for (uint32_t r = 0; r < k_rays; r++)
+            if (slots[r].tid == threadIdx.x)
+                for (int e = STACK_SH; e < slots[r].sp; e++) entry(r, e) = spill[e - STACK_SH];
+        __syncwarp();
+    }
+    if (valid) {
+        const CoopSlot& c = slots[g];
+        tv.tmin = c.tmin; tv.tmax = c.tmax;
+        tv.cr = c.cr;
+        tv.tr = c.tr;
+        tv.best_t = c.best_t; tv.best_u = c.best_u; tv.best_v = c.best_v;
+        tv.best_inst = c.best_inst; tv.best_prim = c.best_prim;
+        tv.ngroup = c.ngroup; tv.tgroup = c.tgroup;
+        tv.level = c.level; tv.blas_sp = c.blas_sp;
+        tv.cur_inst = c.cur_inst; tv.steps = c.steps;
+        tv.err = 0; tv.done = false;
+        tv.st.sh = sh_stack; tv.st.tid = c.tid; tv.st.nthreads = nthreads; tv.st.sp = c.sp;
+        tv.st.lim = S.stack_max < STACK_MAX ? S.stack_max : STACK_MAX;
+        const unsigned gm = 0xFFu << (8u * g);
+        auto push = [&](uint32_t x, uint32_t y) {
+            if (tv.st.sp >= tv.st.lim) { tv.fail(ERR_STACK_OVERFLOW); return; }
+            entry(g, tv.st.sp++) = make_uint2(x, y);   // (the group's lanes store the same value)
+        };
+        while (!tv.done) {
+            if (!tv.has_node() && !tv.has_prim()) {
+                if (tv.level == 1 && tv.st.sp == tv.blas_sp) { tv.level = 0; tv.restore_world(); }
+                if (tv.st.sp == 0) break;
+                const uint2 e = entry(g, --tv.st.sp);
+                if (e.x & PRIM_GROUP) tv.tgroup = make_uint2(e.x & ~PRIM_GROUP, e.y);
+                else tv.ngroup = e;
+                continue;
+            }
+            if (++tv.steps > S.max_steps) { tv.fail(ERR_STEP_LIMIT); break; }
+            if (tv.has_prim() && tv.level == 1) {
+                // the hit leaf slots' triangles, one per lane
+                const uint32_t hit = tv.tgroup.y >> 24, leaves = tv.tgroup.y & 0xFFu;
+                if (tv.tr.k == INVALID) tv.tr = wray_setup(v3(tv.tr.Sx, tv.tr.Sy, tv.tr.Sz));
+                float t = 0.0f, b1 = 0.0f, b2 = 0.0f;
+                uint32_t prim = INVALID;
+                bool found = false, bad = false;
+                if ((hit >> slot) & 1u) {
+                    const uint32_t pidx = tv.tgroup.x + (uint32_t)__popc(leaves & ((1u << slot) - 1u));
+                    bad = pidx >= S.num_tris;
+                    if (!bad) {
+                        const float4* tp = reinterpret_cast<const float4*>(S.tris + pidx);
+                        const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+                        const float va[3] = {a.x, a.y, a.z}, vb[3] = {b.x, b.y, b.z}, vc[3] = {c.x, c.y, c.z};
+                        found = intersect_tri(tv.tr, v3(tv.cr.ox, tv.cr.oy, tv.cr.oz), va, vb, vc, tv.tmin, tv.tmax, &t,
+                                              &b1, &b2);
+                        prim = __float_as_uint(a.w);
+                    }
+                }
+                tv.tgroup = make_uint2(0u, 0u);
+                if (__any_sync(gm, bad)) { tv.fail(ERR_BAD_INDEX); break; }
+                unsigned f = __ballot_sync(gm, found);
+                if (ANY) {
+                    if (f) { tv.best_inst = tv.cur_inst; break; }
+                } else {
+                    for (; f; f &= f - 1u) {   // (rarely more than one)
+                        const int l = __ffs(f) - 1;
+                        const float tl = __shfl_sync(gm, t, l), ul = __shfl_sync(gm, b1, l), vl = __shfl_sync(gm, b2, l);
+                        const uint32_t pl = __shfl_sync(gm, prim, l);
+                        if (tv.best_inst == INVALID || tl < tv.best_t ||
+                            (tl == tv.best_t && (tv.cur_inst < tv.best_inst ||
+                                                 (tv.cur_inst == tv.best_inst && pl < tv.best_prim)))) {
+                            tv.best_t = tl; tv.best_inst = tv.cur_inst; tv.best_prim = pl; tv.best_u = ul; tv.best_v = vl;
+                        }
+                    }
+                }
+                continue;
+            }
+            if (tv.has_prim()) {   // an instance
+                const uint32_t k = __ffs(tv.tgroup.y >> 24) - 1;
+                tv.tgroup.y &= ~(1u << (24 + k));
+                const uint32_t pidx = tv.tgroup.x + (uint32_t)__popc(tv.tgroup.y & ((1u << k) - 1u));
+                const uint32_t rest_x = tv.tgroup.x, rest_y = tv.tgroup.y;
+                if (tv.has_prim()) push(rest_x | PRIM_GROUP, rest_y);
+                if (!tv.done && tv.has_node()) push(tv.ngroup.x, tv.ngroup.y);
+                if (tv.done) break;
+                tv.enter_instance(S, pidx);
+                continue;
+            }
+            // a node: one child per lane
+            const uint32_t k = __ffs(tv.ngroup.y >> 24) - 1;
+            tv.ngroup.y &= ~(1u << (24 + k));
+            const uint32_t sl = TV::ORD ? k ^ tv.cr.oct : k;
+            const uint32_t child = tv.ngroup.x + (uint32_t)__popc(tv.ngroup.y & ((1u << sl) - 1u) & 0xFFu);
+            if (tv.has_node()) push(tv.ngroup.x, tv.ngroup.y);
+            if (tv.done) break;
+            if (child >= (tv.level ? S.num_blas_nodes : S.num_tlas_nodes)) { tv.fail(ERR_BAD_INDEX); break; }
+            const WideNode* N = (tv.level ? S.blas_nodes : S.tlas_nodes) + child;
+            const float4 w0 = __ldg(reinterpret_cast<const float4*>(N));
+            const uint2 w1 = __ldg(reinterpret_cast<const uint2*>(N) + 2);
+            const uint8_t* q = N->meta + slot;   // meta, then the planes: lo x y z, hi x y z, eight bytes each
+            const uint32_t meta = __ldg(q);
+            const uint32_t ox = tv.cr.oct & 1u ? 24u : 0u, oy = tv.cr.oct & 2u ? 24u : 0u, oz = tv.cr.oct & 4u ? 24u : 0u;
+            const float nx = byte_f(__ldg(q + 8 + ox)), fx = byte_f(__ldg(q + 32 - ox));
+            const float ny = byte_f(__ldg(q + 16 + oy)), fy = byte_f(__ldg(q + 40 - oy));
+            const float nz = byte_f(__ldg(q + 24 + oz)), fz = byte_f(__ldg(q + 48 - oz));
+            const uint32_t e = __float_as_uint(w0.w), imask = e >> 24;
+            const float ax = __uint_as_float((e << 23) & 0x7F800000u) * tv.cr.idx;
+            const float ay = __uint_as_float((e << 15) & 0x7F800000u) * tv.cr.idy;
+            const float az = __uint_as_float((e << 7) & 0x7F800000u) * tv.cr.idz;
+            const float bx = __fmaf_rn(w0.x - tv.cr.ox, tv.cr.idx, -ax), by = __fmaf_rn(w0.y - tv.cr.oy, tv.cr.idy, -ay),
+                        bz = __fmaf_rn(w0.z - tv.cr.oz, tv.cr.idz, -az);
+            const float tn = max3f(__fmaf_rn(nx, ax, bx), __fmaf_rn(ny, ay, by), fmaxf(__fmaf_rn(nz, az, bz), tv.tmin));
+            const float tf = min3f(__fmaf_rn(fx, ax, bx), __fmaf_rn(fy, ay, by), fminf(__fmaf_rn(fz, az, bz), tv.best_t));
+            const bool in = (int)__float_as_uint(__fmaf_rn(tf, 1.0f + BOX_SLACK, -tn)) >= 0;
+            const uint32_t hits = (__ballot_sync(gm, in) >> (8u * g)) & 0xFFu;
+            const uint32_t leaves = (__ballot_sync(gm, (meta & 0x20u) != 0u && !((imask >> slot) & 1u)) >> (8u * g)) & 0xFFu;
+            uint32_t x = hits & imask;
+            if (TV::ORD) x = visit_order(x, tv.cr.oct);
+            tv.ngroup = make_uint2(w1.x, (x << 24) | imask);
+            tv.tgroup = make_uint2(w1.y, ((hits & leaves) << 24) | leaves);
+        }
+    }
+    __syncwarp();
+    if (valid && slot == 0u) {
+        CoopSlot& c = slots[g];
+        c.best_t = tv.best_t; c.best_u = tv.best_u; c.best_v = tv.best_v;
+        c.best_inst = tv.best_inst; c.best_prim = tv.best_prim;
+        c.err = tv.err;
+    }
+    __syncwarp();
+}
 
 // ---- warp packets ------------------------------------------------------------
 // Traversal of up to 32 coherent rays (one per lane) by the whole warp together,

@@ -32,6 +32,7 @@ constexpr uint32_t CHUNK_MAX = 64, CHUNK_MIN = 32;
 
 struct Knobs {
     uint32_t chunk, chunk_min;
+    uint32_t few;     // rays per warp of a queue of at most COOP_RAYS rays per resident warp, else 0
     float share;      // chunk per ray left
     int refill_idle;
     uint32_t prim_bias;
@@ -40,7 +41,10 @@ struct Knobs {
           refill_idle(t.refill_idle ? (int)t.refill_idle : 4), prim_bias(t.prim_bias ? t.prim_bias : 3u) {
         const uint32_t c = (uint32_t)((float)n * (16.0f * share));
         chunk_min = min(max(c, 1u), min(CHUNK_MIN, chunk));
+        few = n <= (uint32_t)COOP_RAYS * t.warps ? max((n + t.warps - 1u) / t.warps, 1u) : 0u;
     }
+    // eight lanes per ray from the start: a warp takes `few` rays at a time
+    __device__ __forceinline__ void take_few() { chunk = chunk_min = few; }
     // the chunk to take when at most `left` rays are left
     __device__ __forceinline__ uint32_t next_chunk(uint32_t left) const {
         return min(max((uint32_t)((float)left * share), chunk_min), chunk);
@@ -111,49 +115,113 @@ struct RayFeed {
     __device__ __forceinline__ bool done() const { return exhausted && next >= end; }
 };
 
-// closest hit of the rays queued for segment d
-template <bool COUNT, int MINB, bool SINGLE>
-__global__ void __launch_bounds__(TBLK, MINB) k_trace_closest(FrameParams F, uint32_t d) {
-    __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
-    const uint32_t n = F.counters[CNT_QUEUE + d];
-    const Knobs kn(F.tune, n);
-    const float4* rays = F.rays[d & 1u];
-    uint32_t* work = &F.counters[CNT_WORK_TRACE + d];
-    const uint32_t lane = threadIdx.x & 31u;
-    TraceCounters ctr{0ull, 0ull};
-    Traverser<false, COUNT, SINGLE> tv;
+// Traces a queue: `refill(idle)` gives the lanes of the mask their next entries (INVALID:
+// none), `done()` tells that there are no more; start(tv, entry) sets a ray up and
+// returns the index its result goes to, emit(tv, index) writes the result of a finished
+// ray.  COOP: a warp's last COOP_RAYS rays get eight lanes each (coop_trace) once one of
+// them has taken COOP_STEPS steps: such a ray has a long way behind it and likely more to
+// go, and the queue's end waits for it (short rays, as in a closed room, finish sooner
+// where they are: a 65,536-path room frame 304 us, 328 with all last rays moved).  So do
+// all rays of a queue that gives the resident warps no more than COOP_RAYS each.  The
+// 480x270 terrain batch took 1.43 instead of 1.55 ms so, a 480x270 sphere-field frame 0.54
+// and 0.58, a 1080p frame 2.005 and 2.037, 10,000 rays 112 and 129 us, 64 rays 73 and 83 us.
+constexpr uint32_t COOP_STEPS = 48;
+
+template <bool COOP, class TV, class Refill, class Done, class Start, class Emit>
+__device__ __forceinline__ void trace_queue(const SceneDev& S, const Knobs& kn, uint2* sh_stack, TraceCounters* ctr,
+                                            Refill&& refill, Done&& done, Start&& start, Emit&& emit) {
+    __shared__ CoopSlot coop_slots[COOP ? TBLK / 32 : 1][COOP_RAYS];
     uint2 spill[STACK_MAX - STACK_SH];
-    RayFeed feed;
-    feed.init();
+    auto rank = [](unsigned mask) { return (uint32_t)__popc(mask & ((1u << (threadIdx.x & 31u)) - 1u)); };
+    auto finish_few = [&](uint32_t k) {   // the k rays in the warp's slots
+        if constexpr (COOP) {
+            CoopSlot* slots = coop_slots[threadIdx.x >> 5];
+            coop_trace<!TV::ORD>(slots, k, S, sh_stack, spill, TBLK);
+            const uint32_t lane = threadIdx.x & 31u;
+            if (lane < k) {
+                TraceResult r;
+                ray_result(slots[lane], S, r);
+                emit(r, slots[lane].ri);
+            }
+            __syncwarp();
+        }
+    };
+    TV tv;
+    if (COOP && kn.few) {
+        do {
+            const uint32_t i = refill((1u << kn.few) - 1u);
+            const unsigned act = __ballot_sync(0xFFFFFFFFu, i != INVALID);
+            if (i != INVALID) {
+                const uint32_t ri = start(tv, i, spill);
+                coop_save(coop_slots[threadIdx.x >> 5][rank(act)], tv, ri);
+            }
+            if (act) finish_few((uint32_t)__popc(act));
+        } while (!done());
+        return;
+    }
     bool active = false;
     uint32_t ri = 0;
     for (;;) {
         unsigned act = __ballot_sync(0xFFFFFFFFu, active);
-        if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t i = feed.refill(~act, lane, work, n, kn);
-            if (i != INVALID) {
-                float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
-                tv.init(F.S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
-                ri = i;
-                active = true;
+        if (__popc(~act) >= kn.refill_idle) {
+            if (!done()) {
+                const uint32_t i = refill(~act);
+                if (i != INVALID) {
+                    ri = start(tv, i, spill);
+                    active = true;
+                }
+                act = __ballot_sync(0xFFFFFFFFu, active);
+                if (act == 0) continue;
+            } else if (act == 0) {
+                break;
+            } else if (COOP && __popc(act) <= COOP_RAYS &&
+                       __any_sync(0xFFFFFFFFu, active && tv.steps >= COOP_STEPS)) {
+                if (active) coop_save(coop_slots[threadIdx.x >> 5][rank(act)], tv, ri);
+                finish_few((uint32_t)__popc(act));
+                break;
             }
-            act = __ballot_sync(0xFFFFFFFFu, active);
         }
-        if (act == 0) {
-            if (feed.done()) break;
-            continue;
-        }
-        if (warp_step(tv, active, F.S, &ctr, kn.prim_bias)) {
+        if (warp_step(tv, active, S, ctr, kn.prim_bias)) {
             TraceResult r;
-            tv.finish(F.S, r);
-            HitDev h;
-            h.t = r.t; h.inst = r.inst; h.prim = r.prim; h.u = r.u; h.v = r.v; h.flags = r.hit ? 1u : 0u;
-            uint2* dst = reinterpret_cast<uint2*>(F.hits + ri);
-            const uint2* src = reinterpret_cast<const uint2*>(&h);
-            dst[0] = src[0]; dst[1] = src[1]; dst[2] = src[2];
+            tv.finish(S, r);
+            emit(r, ri);
             active = false;
         }
     }
+}
+
+__device__ __forceinline__ void store_hit(HitDev* dst, const TraceResult& r) {
+    HitDev h;
+    h.t = r.t; h.inst = r.inst; h.prim = r.prim; h.u = r.u; h.v = r.v; h.flags = r.hit ? 1u : 0u;
+    uint2* d = reinterpret_cast<uint2*>(dst);
+    const uint2* s = reinterpret_cast<const uint2*>(&h);
+    d[0] = s[0]; d[1] = s[1]; d[2] = s[2];
+}
+
+// closest hit of the rays queued for segment d
+template <bool COUNT, int MINB, bool SINGLE>
+__global__ void __launch_bounds__(TBLK, MINB) k_trace_closest(const __grid_constant__ FrameParams F, uint32_t d) {
+    constexpr bool COOP = SINGLE && !COUNT;
+    using TV = Traverser<false, COUNT, SINGLE>;
+    __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
+    const uint32_t n = F.counters[CNT_QUEUE + d];
+    Knobs kn(F.tune, n);
+    if (COOP && kn.few) kn.take_few();
+    const float4* rays = F.rays[d & 1u];
+    uint32_t* work = &F.counters[CNT_WORK_TRACE + d];
+    const uint32_t lane = threadIdx.x & 31u;
+    TraceCounters ctr{0ull, 0ull};
+    RayFeed feed;
+    feed.init();
+    trace_queue<COOP, TV>(
+        F.S, kn, sh_stack, &ctr, [&](unsigned idle) { return feed.refill(idle, lane, work, n, kn); },
+        [&] { return feed.done(); },
+        [&](TV& tv, uint32_t i, uint2* spill) {
+            const float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
+            tv.init(F.S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
+            return i;
+        },
+        [&](const TraceResult& r, uint32_t ri) { store_hit(F.hits + ri, r); });
     flush_counts<COUNT>(ctr, F.trav_counters);
 }
 
@@ -182,13 +250,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_packet(FrameParams F, uint
         tv.run(F.S);
         TraceResult r;
         tv.finish(F.S, r);
-        if (active) {
-            HitDev h;
-            h.t = r.t; h.inst = r.inst; h.prim = r.prim; h.u = r.u; h.v = r.v; h.flags = r.hit ? 1u : 0u;
-            uint2* dst = reinterpret_cast<uint2*>(F.hits + i);
-            const uint2* src = reinterpret_cast<const uint2*>(&h);
-            dst[0] = src[0]; dst[1] = src[1]; dst[2] = src[2];
-        }
+        if (active) store_hit(F.hits + i, r);
     }
 }
 
@@ -198,44 +260,29 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_packet(FrameParams F, uint
 // component, and k_accum_shadow adds the visible contributions in entry order
 // (the same order as the CPU oracle, so sums are bit-identical).
 template <bool COUNT, int MINB, bool SINGLE>
-__global__ void __launch_bounds__(TBLK, MINB) k_trace_shadow(FrameParams F, uint32_t d) {
+__global__ void __launch_bounds__(TBLK, MINB) k_trace_shadow(const __grid_constant__ FrameParams F, uint32_t d) {
+    constexpr bool COOP = SINGLE && !COUNT;
+    using TV = Traverser<true, COUNT, SINGLE>;
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     const uint32_t n0 = F.counters[CNT_SHADOW_Q + 2 * d], n = n0 + F.counters[CNT_SHADOW_Q + 2 * d + 1];
-    const Knobs kn(F.tune_any, n);
+    Knobs kn(F.tune_any, n);
+    if (COOP && kn.few) kn.take_few();
     uint32_t* work = &F.counters[CNT_WORK_SHADOW + d];
     const uint32_t lane = threadIdx.x & 31u;
     TraceCounters ctr{0ull, 0ull};
-    Traverser<true, COUNT, SINGLE> tv;
-    uint2 spill[STACK_MAX - STACK_SH];
     RayFeed feed;
     feed.init();
-    bool active = false;
-    uint32_t ri = 0;
-    for (;;) {
-        unsigned act = __ballot_sync(0xFFFFFFFFu, active);
-        if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t j = feed.refill(~act, lane, work, n, kn);
-            if (j != INVALID) {
-                const size_t e = j < n0 ? (size_t)j : (size_t)F.n_paths + (j - n0);
-                const float4* sr = F.shadow_rays + 2 * e;
-                const float4 a = __ldg(sr), b = __ldg(sr + 1);
-                tv.init(F.S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), SHADOW_TMIN, b.w, sh_stack, spill, threadIdx.x, TBLK);
-                ri = __float_as_uint(a.w);
-                active = true;
-            }
-            act = __ballot_sync(0xFFFFFFFFu, active);
-        }
-        if (act == 0) {
-            if (feed.done()) break;
-            continue;
-        }
-        if (warp_step(tv, active, F.S, &ctr, kn.prim_bias)) {
-            TraceResult r;
-            bool occ = tv.finish(F.S, r);
-            F.shadow_contrib[ri].w = occ ? 0.0f : 1.0f;
-            active = false;
-        }
-    }
+    trace_queue<COOP, TV>(
+        F.S, kn, sh_stack, &ctr, [&](unsigned idle) { return feed.refill(idle, lane, work, n, kn); },
+        [&] { return feed.done(); },
+        [&](TV& tv, uint32_t j, uint2* spill) {
+            const size_t e = j < n0 ? (size_t)j : (size_t)F.n_paths + (j - n0);
+            const float4* sr = F.shadow_rays + 2 * e;
+            const float4 a = __ldg(sr), b = __ldg(sr + 1);
+            tv.init(F.S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), SHADOW_TMIN, b.w, sh_stack, spill, threadIdx.x, TBLK);
+            return __float_as_uint(a.w);
+        },
+        [&](const TraceResult& r, uint32_t ri) { F.shadow_contrib[ri].w = r.hit ? 0.0f : 1.0f; });
     flush_counts<COUNT>(ctr, F.trav_counters ? F.trav_counters + 2 : nullptr);
 }
 
@@ -319,88 +366,57 @@ struct FilteredFeed {
 // visibility of a queue of segments: vis[i] = 1 when nothing is hit in (tmin, tmax),
 // 0 when something is; entries with tmax < 0 are empty (skipped, vis[i] not written:
 // the passes never read the result of a slot they did not record).
-// The ReSTIR passes queue their visibility rays here instead of tracing inline.
+// The ReSTIR passes queue their visibility rays here instead of tracing inline.  (No
+// eight-lane end: these queues are long and their rays short, two 1080p ReSTIR frames
+// took 17.38 ms with it and 17.02 without.)
 template <int MINB, bool SINGLE>
-__global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(SceneDev S, const float4* __restrict__ rays,
+__global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(const __grid_constant__ SceneDev S, const float4* __restrict__ rays,
                                                                  uint32_t n, uint8_t* vis, uint32_t* work,
                                                                  TraceTuning tune) {
-    const Knobs kn(tune, n);
+    using TV = Traverser<true, false, SINGLE>;
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     __shared__ uint32_t ring[TBLK / 32][64];
+    const Knobs kn(tune, n);
     const uint32_t lane = threadIdx.x & 31u;
-    Traverser<true, false, SINGLE> tv;
-    uint2 spill[STACK_MAX - STACK_SH];
     FilteredFeed feed;
     feed.init();
-    bool active = false;
-    uint32_t ri = 0;
-    for (;;) {
-        unsigned act = __ballot_sync(0xFFFFFFFFu, active);
-        if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t i = feed.refill(~act, lane, work, n, kn, rays, ring[threadIdx.x >> 5]);
-            if (i != INVALID) {
-                const float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
-                tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
-                ri = i;
-                active = true;
-            }
-            act = __ballot_sync(0xFFFFFFFFu, active);
-        }
-        if (act == 0) {
-            if (feed.done()) break;
-            continue;
-        }
-        if (warp_step(tv, active, S, nullptr, kn.prim_bias)) {
-            TraceResult r;
-            vis[ri] = tv.finish(S, r) ? 0u : 1u;
-            active = false;
-        }
-    }
+    trace_queue<false, TV>(
+        S, kn, sh_stack, nullptr,
+        [&](unsigned idle) { return feed.refill(idle, lane, work, n, kn, rays, ring[threadIdx.x >> 5]); },
+        [&] { return feed.done(); },
+        [&](TV& tv, uint32_t i, uint2* spill) {
+            const float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
+            tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
+            return i;
+        },
+        [&](const TraceResult& r, uint32_t ri) { vis[ri] = r.hit ? 0u : 1u; });
 }
 
 // generic trace of an array of rays (the snk_pt_trace_rays test hook)
 template <bool ANY, bool SINGLE>
-__global__ void __launch_bounds__(TBLK, 6) k_trace_rays(SceneDev S, const float4* __restrict__ rays, uint32_t n,
+__global__ void __launch_bounds__(TBLK, 6) k_trace_rays(const __grid_constant__ SceneDev S, const float4* __restrict__ rays, uint32_t n,
                                                      HitDev* hits, uint32_t* work, TraceTuning tune) {
-    const Knobs kn(tune, n);
+    using TV = Traverser<ANY, false, SINGLE>;
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
+    Knobs kn(tune, n);
+    if (SINGLE && kn.few) kn.take_few();
     const uint32_t lane = threadIdx.x & 31u;
-    Traverser<ANY, false, SINGLE> tv;
-    uint2 spill[STACK_MAX - STACK_SH];
     RayFeed feed;
     feed.init();
-    bool active = false;
-    uint32_t ri = 0;
-    for (;;) {
-        unsigned act = __ballot_sync(0xFFFFFFFFu, active);
-        if (__popc(~act) >= kn.refill_idle && !feed.done()) {
-            uint32_t i = feed.refill(~act, lane, work, n, kn);
-            if (i != INVALID) {
-                float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
-                tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
-                ri = i;
-                active = true;
-            }
-            act = __ballot_sync(0xFFFFFFFFu, active);
-        }
-        if (act == 0) {
-            if (feed.done()) break;
-            continue;
-        }
-        if (warp_step(tv, active, S, nullptr, kn.prim_bias)) {
-            TraceResult r;
-            bool hit = tv.finish(S, r);
-            HitDev h;
+    trace_queue<SINGLE, TV>(
+        S, kn, sh_stack, nullptr, [&](unsigned idle) { return feed.refill(idle, lane, work, n, kn); },
+        [&] { return feed.done(); },
+        [&](TV& tv, uint32_t i, uint2* spill) {
+            const float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
+            tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
+            return i;
+        },
+        [&](TraceResult r, uint32_t ri) {
             if (ANY) {
-                h.t = hit ? 1.0f : -1.0f; h.inst = INVALID; h.prim = INVALID; h.u = 0.0f; h.v = 0.0f;
-                h.flags = hit ? 1u : 0u;
-            } else {
-                h.t = r.t; h.inst = r.inst; h.prim = r.prim; h.u = r.u; h.v = r.v; h.flags = hit ? 1u : 0u;
+                r.t = r.hit ? 1.0f : -1.0f; r.inst = INVALID; r.prim = INVALID; r.u = 0.0f; r.v = 0.0f;
             }
-            hits[ri] = h;
-            active = false;
-        }
-    }
+            store_hit(hits + ri, r);
+        });
 }
 
 }  // namespace

@@ -91,7 +91,7 @@ struct snk_pt_ctx {
     bool inst_tables_valid = false;    // instance and NEE records match the uploaded inputs
     bool lights_changed = true;        // point lights or materials changed since the NEE records
     uint32_t n_emissive = 0, n_local = 0;
-    DBuf<unsigned> d_err;
+    DBuf<unsigned> d_err;              // [0] the device error word, [1] work counter of the ray queries
     DBuf<unsigned char> q_in, q_in2, q_out, q_out2;   // staging of the particle / contact queries
     DBuf<float4> rq_rays;                              // ReSTIR visibility queue (slots x pixels x 2)
     DBuf<uint8_t> rq_vis_a, rq_vis_b;                  // its results (initial / shading, spatial)
@@ -138,9 +138,7 @@ struct snk_pt_ctx {
     uint32_t accum_w = 0, accum_h = 0;
     uint64_t accum_frames = 0;
 
-    DBuf<float4> tr_rays;
-    DBuf<HitDev> tr_hits;
-    DBuf<uint32_t> tr_work;
+    DBuf<unsigned char> tr_buf;        // rays (32 B each), then hits of a ray or contact query
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool timing_pending = false;
@@ -552,7 +550,6 @@ Status build_all(snk_pt_ctx* ctx) {
         SNK_TRY(build_instances(ctx));
         ctx->inst_dirty = false;
     }
-    SNK_TRY_CUDA(ctx->d_err.reserve(1));
     ctx->built = true;
     return Status::Ok();
 }
@@ -738,7 +735,7 @@ int snk_pt_create(const snk_pt_config* config, snk_pt_ctx** out_ctx) {
         cudaMallocHost(&ctx->h_err, sizeof(unsigned)) != cudaSuccess ||
         cudaMallocHost(&ctx->h_small, sizeof(SmallBuildOut)) != cudaSuccess ||
         cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
-        ctx->d_err.reserve(1) != cudaSuccess || cudaMemset(ctx->d_err.p, 0, sizeof(unsigned)) != cudaSuccess) {
+        ctx->d_err.reserve(2) != cudaSuccess || cudaMemset(ctx->d_err.p, 0, 2 * sizeof(unsigned)) != cudaSuccess) {
         snk_pt_destroy(ctx);
         return SNK_ERR_CUDA;
     }
@@ -1672,19 +1669,20 @@ int snk_pt_trace_rays(snk_pt_ctx* ctx, const snk_ray* rays, uint32_t n, snk_hit*
     const float4* d_rays;
     HitDev* d_hits;
     if (memory == SNK_MEM_HOST) {
-        if (ctx->tr_rays.reserve(2ull * n) || ctx->tr_hits.reserve(n)) return fail(ctx, SNK_ERR_OUT_OF_MEMORY, "trace buffers");
-        if (cudaMemcpyAsync(ctx->tr_rays.p, rays, sizeof(snk_ray) * (size_t)n, cudaMemcpyHostToDevice, st))
+        if (ctx->tr_buf.reserve((sizeof(snk_ray) + sizeof(HitDev)) * (size_t)n))
+            return fail(ctx, SNK_ERR_OUT_OF_MEMORY, "trace buffers");
+        if (cudaMemcpyAsync(ctx->tr_buf.p, rays, sizeof(snk_ray) * (size_t)n, cudaMemcpyHostToDevice, st))
             return fail(ctx, SNK_ERR_CUDA, "trace_rays: ray upload");
-        d_rays = ctx->tr_rays.p;
-        d_hits = ctx->tr_hits.p;
+        d_rays = reinterpret_cast<const float4*>(ctx->tr_buf.p);
+        d_hits = reinterpret_cast<HitDev*>(ctx->tr_buf.p + sizeof(snk_ray) * (size_t)n);
     } else {
         d_rays = reinterpret_cast<const float4*>(rays);
         d_hits = reinterpret_cast<HitDev*>(hits);
     }
-    if (ctx->tr_work.reserve(1) || cudaMemsetAsync(ctx->tr_work.p, 0, sizeof(uint32_t), st))
+    if (cudaMemsetAsync(ctx->d_err.p + 1, 0, sizeof(uint32_t), st))
         return fail(ctx, SNK_ERR_CUDA, "trace_rays: work counter");
     const bool any = (flags & SNK_TRACE_ANY_HIT) != 0;
-    cudaError_t e = launch_trace_rays(scene_dev(ctx), d_rays, n, d_hits, any, ctx->tr_work.p,
+    cudaError_t e = launch_trace_rays(scene_dev(ctx), d_rays, n, d_hits, any, ctx->d_err.p + 1,
                                       any ? any_grid(ctx) : trace_grid(ctx), any ? any_tuning(ctx) : trace_tuning(ctx), st);
     if (e != cudaSuccess) return fail(ctx, SNK_ERR_CUDA, std::string("trace_rays: ") + cudaGetErrorString(e));
     if (memory == SNK_MEM_HOST &&
@@ -1713,6 +1711,25 @@ T* stage_out(DBuf<unsigned char>& b, void* dst, size_t bytes, uint32_t memory, S
     if (b.reserve(bytes ? bytes : 1)) { *st = Status::Err(SNK_ERR_OUT_OF_MEMORY, "query staging"); return nullptr; }
     return reinterpret_cast<T*>(b.p);
 }
+// Scratch of a contact query of n items with `per` rays each; queries run in parts of at
+// most CONTACT_RAYS rays (enough to fill the GPU), which bounds it to 59 MB.
+constexpr uint32_t CONTACT_RAYS = 1u << 20;
+Status contact_scratch(snk_pt_ctx* ctx, uint32_t n, uint32_t per, bool own_rays, ContactScratch* c) {
+    const size_t rays = std::min<size_t>((size_t)n * per, CONTACT_RAYS);
+    const size_t ray_bytes = own_rays ? rays * sizeof(snk_ray) : 0;
+    SNK_TRY_CUDA(ctx->tr_buf.reserve(ray_bytes + rays * sizeof(HitDev)));
+    *c = ContactScratch{reinterpret_cast<float4*>(ctx->tr_buf.p), reinterpret_cast<HitDev*>(ctx->tr_buf.p + ray_bytes),
+                        ctx->d_err.p + 1, trace_grid(ctx), trace_tuning(ctx)};
+    return Status::Ok();
+}
+// calls part(first, count) over [0, n) in parts of at most CONTACT_RAYS / per items
+template <class Fn>
+cudaError_t in_parts(uint32_t n, uint32_t per, Fn&& part) {
+    cudaError_t e = cudaSuccess;
+    for (uint64_t b = 0; b < n && e == cudaSuccess; b += CONTACT_RAYS / per)
+        e = part((uint32_t)b, std::min(n - (uint32_t)b, CONTACT_RAYS / per));
+    return e;
+}
 Status download(snk_pt_ctx* ctx, void* dst, const void* src, size_t bytes, uint32_t memory) {
     if (memory == SNK_MEM_HOST && bytes)
         SNK_TRY_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1732,7 +1749,11 @@ int snk_pt_contact_rays(snk_pt_ctx* ctx, const snk_ray* rays, uint32_t n, float 
     const float4* d_rays = stage_in<const float4>(ctx, ctx->q_in, rays, sizeof(snk_ray) * (size_t)n, memory, &st);
     ContactOut* d_out = stage_out<ContactOut>(ctx->q_out, out, sizeof(snk_contact) * (size_t)n, memory, &st);
     if (!st.ok()) return fail(ctx, st);
-    cudaError_t e = launch_contact_rays(scene_dev(ctx), d_rays, n, timestep, d_out, grid_of(ctx, 16), ctx->stream);
+    ContactScratch sc;
+    API_TRY(contact_scratch(ctx, n, 1, false, &sc));
+    const cudaError_t e = in_parts(n, 1, [&](uint32_t b, uint32_t cnt) {
+        return launch_contact_rays(scene_dev(ctx), d_rays + 2ull * b, cnt, timestep, d_out + b, sc, ctx->stream);
+    });
     if (e != cudaSuccess) return fail(ctx, SNK_ERR_CUDA, std::string("contact_rays: ") + cudaGetErrorString(e));
     API_TRY(download(ctx, out, d_out, sizeof(snk_contact) * (size_t)n, memory));
     API_TRY(check_device_error(ctx));
@@ -1752,7 +1773,11 @@ int snk_pt_particle_probe(snk_pt_ctx* ctx, const snk_particle* particles, uint32
     ContactOut* d_c = stage_out<ContactOut>(ctx->q_out, candidate, sizeof(snk_contact) * (size_t)n, memory, &st);
     float* d_g = stage_out<float>(ctx->q_out2, gravity_dv, sizeof(float) * (size_t)n, memory, &st);
     if (!st.ok()) return fail(ctx, st);
-    cudaError_t e = launch_particle_probe(scene_dev(ctx), d_p, n, timestep, d_c, d_g, grid_of(ctx, 16), ctx->stream);
+    ContactScratch sc;
+    API_TRY(contact_scratch(ctx, n, 4, true, &sc));
+    const cudaError_t e = in_parts(n, 4, [&](uint32_t b, uint32_t cnt) {
+        return launch_particle_probe(scene_dev(ctx), d_p + b, cnt, timestep, d_c + b, d_g + b, sc, ctx->stream);
+    });
     if (e != cudaSuccess) return fail(ctx, SNK_ERR_CUDA, std::string("particle_probe: ") + cudaGetErrorString(e));
     API_TRY(download(ctx, candidate, d_c, sizeof(snk_contact) * (size_t)n, memory));
     API_TRY(download(ctx, gravity_dv, d_g, sizeof(float) * (size_t)n, memory));
@@ -1773,8 +1798,12 @@ int snk_pt_particle_constrain(snk_pt_ctx* ctx, const snk_particle* particles, co
     const float* d_off = stage_in<const float>(ctx, ctx->q_in2, offsets, 3 * sizeof(float) * (size_t)n, memory, &st);
     float* d_out = stage_out<float>(ctx->q_out, out, 3 * sizeof(float) * (size_t)n, memory, &st);
     if (!st.ok()) return fail(ctx, st);
-    cudaError_t e =
-        launch_particle_constrain(scene_dev(ctx), d_p, d_off, n, timestep, d_out, grid_of(ctx, 16), ctx->stream);
+    ContactScratch sc;
+    API_TRY(contact_scratch(ctx, n, 1, true, &sc));
+    const cudaError_t e = in_parts(n, 1, [&](uint32_t b, uint32_t cnt) {
+        return launch_particle_constrain(scene_dev(ctx), d_p + b, d_off + 3ull * b, cnt, timestep, d_out + 3ull * b, sc,
+                                         ctx->stream);
+    });
     if (e != cudaSuccess) return fail(ctx, SNK_ERR_CUDA, std::string("particle_constrain: ") + cudaGetErrorString(e));
     API_TRY(download(ctx, out, d_out, 3 * sizeof(float) * (size_t)n, memory));
     API_TRY(check_device_error(ctx));

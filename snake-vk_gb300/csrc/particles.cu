@@ -7,10 +7,14 @@
 //   CalculateGravity .......... :150-165
 //   main (scene part) ......... :151-166
 // and ParticleUpdate.rchit:41-67 (contact normal / position / velocity).
-// Every query is a closest-hit trace (the shader asks for the first hit found);
-// one thread per particle or ray, each traces with the shared traversal core.
+// Every query is a closest-hit trace (the shader asks for the first hit found).  A
+// query runs as three launches: its rays are set up (a particle's four side by side in
+// the queue's four parts, so that a warp's rays are of one kind), traced by the
+// persistent closest-hit kernel of the ray queries, and turned into contacts.  A thread
+// per particle that traced its rays one after the other, without ray replacement, left
+// lanes waiting for the longest of 32 particles: 100,000 particles took 250 us, now 169
+// (set-up 6, trace 108, contacts 14, the rest the call).
 #include "snk_frame.h"
-#include "snk_trace.cuh"
 #include "snk_shade.cuh"
 #include "snk_particles.h"
 
@@ -35,14 +39,17 @@ __device__ __forceinline__ void store(ContactOut* out, const Contact& c) {
     *out = o;
 }
 
-// traceRayEXT + ParticleUpdate.rchit
-__device__ __noinline__ Contact contact_ray(const SceneDev& S, V3 o, V3 d, float tmin, float tmax, float timestep,
-                                            uint2* sh) {
+__device__ __forceinline__ Contact no_contact() {
     Contact c;
     c.n = v3(0.0f, 0.0f, 0.0f); c.p = c.n; c.v = c.n;
     c.dist = -1.0f;
-    TraceResult r;
-    if (!trace_scene<false, false>(S, o, d, tmin, tmax, r, sh, threadIdx.x, PBLK, nullptr)) return c;
+    return c;
+}
+
+// ParticleUpdate.rchit of a ray's closest hit
+__device__ __forceinline__ Contact contact_of(const SceneDev& S, const HitDev& r, V3 o, V3 d, float timestep) {
+    if (!r.flags) return no_contact();
+    Contact c;
     const InstShade& I = S.inst_shade[r.inst];
     const MeshInfo& M = S.meshes[I.mesh_id];
     const uint32_t* ix = S.indices + M.index_offset + 3ull * r.prim;
@@ -64,95 +71,147 @@ __device__ __noinline__ Contact contact_ray(const SceneDev& S, V3 o, V3 d, float
     c.dist = r.t;
     return c;
 }
-
-__global__ void __launch_bounds__(PBLK) k_contact_rays(SceneDev S, const float4* __restrict__ rays, uint32_t n,
-                                                       float timestep, ContactOut* out) {
-    __shared__ uint2 sh[TRACE_SH_ROWS * PBLK];
-    for (uint32_t i = blockIdx.x * PBLK + threadIdx.x; i < n; i += gridDim.x * PBLK) {
-        const float4 a = rays[2ull * i], b = rays[2ull * i + 1];
-        store(out + i, contact_ray(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, timestep, sh));
-    }
+// the same for queue entry e
+__device__ __forceinline__ Contact contact_at(const SceneDev& S, const HitDev* hits, const float4* rays, size_t e,
+                                              float timestep) {
+    const HitDev r = hits[e];
+    if (!r.flags) return no_contact();
+    const float4 a = rays[2 * e], b = rays[2 * e + 1];
+    return contact_of(S, r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), timestep);
 }
 
-__global__ void __launch_bounds__(PBLK) k_particle_probe(SceneDev S, const ParticleDev* __restrict__ P, uint32_t n,
-                                                         float timestep, ContactOut* cand_out, float* gravity) {
-    __shared__ uint2 sh[TRACE_SH_ROWS * PBLK];
-    for (uint32_t i = blockIdx.x * PBLK + threadIdx.x; i < n; i += gridDim.x * PBLK) {
-        const ParticleDev q = P[i];
-        const V3 pos = v3(q.pr.x, q.pr.y, q.pr.z), vel = v3(q.vel.x, q.vel.y, q.vel.z);
-        const float rad = q.pr.w;
-        const bool asleep = q.vel.w < 0.5f;   // IsParticleAsleep
-        Contact cand;
-        cand.n = v3(0.0f, 0.0f, 0.0f); cand.p = cand.n; cand.v = cand.n;
-        cand.dist = -1.0f;
-        float best = 0.0f;
-        const float speed = length(vel);
-        if (!asleep && speed > 0.0f && speed <= 3.0e38f) {
-            const V3 vdir = v3(vel.x / speed, vel.y / speed, vel.z / speed);
-            const V3 right = fabsf(dot(vdir, v3(0.0f, 1.0f, 0.0f))) > 0.99f ? cross(vdir, v3(0.0f, 0.0f, 1.0f))
-                                                                          : cross(vdir, v3(0.0f, 1.0f, 0.0f));
-            const V3 up = cross(right, vdir);
-            const V3 dirs[3] = {vdir, right, up};
-            for (int k = 0; k < 3; k++) {
-                const float len = k == 0 ? speed * PARTICLE_DT + rad * 2.0f : rad * 2.0f;
-                const V3 o = sub(pos, mul(dirs[k], rad));
-                const Contact c = contact_ray(S, o, dirs[k], 0.0f, len, timestep, sh);
-                const float w = length(sub(c.v, vel));
-                if (c.dist > 0.0f && w > best) { best = w; cand = c; }
-            }
+__device__ __forceinline__ void put_ray(float4* rays, size_t e, V3 o, V3 d, float tmax) {
+    rays[2 * e] = make_float4(o.x, o.y, o.z, 0.0f);
+    rays[2 * e + 1] = make_float4(d.x, d.y, d.z, tmax);
+}
+
+__global__ void __launch_bounds__(PBLK) k_contacts(SceneDev S, const HitDev* __restrict__ hits,
+                                                   const float4* __restrict__ rays, uint32_t n, float timestep,
+                                                   ContactOut* out) {
+    const uint32_t i = blockIdx.x * PBLK + threadIdx.x;
+    if (i < n) store(out + i, contact_at(S, hits, rays, i, timestep));
+}
+
+// entries k n + i: particle i's collision rays (k = 0, 1, 2; an empty one, which hits
+// nothing, for a particle asleep or at rest) and its gravity ray (k = 3); the work counter
+// of the trace that follows starts at 0
+__global__ void __launch_bounds__(PBLK) k_particle_rays(const ParticleDev* __restrict__ P, uint32_t n, float4* rays,
+                                                        uint32_t* work) {
+    const uint32_t i = blockIdx.x * PBLK + threadIdx.x;
+    if (i == 0) *work = 0u;
+    if (i >= n) return;
+    const ParticleDev q = P[i];
+    const V3 pos = v3(q.pr.x, q.pr.y, q.pr.z), vel = v3(q.vel.x, q.vel.y, q.vel.z);
+    const float rad = q.pr.w;
+    const bool asleep = q.vel.w < 0.5f;   // IsParticleAsleep
+    const float speed = length(vel);
+    const V3 down = v3(0.0f, -1.0f, 0.0f);
+    if (!asleep && speed > 0.0f && speed <= 3.0e38f) {
+        const V3 vdir = v3(vel.x / speed, vel.y / speed, vel.z / speed);
+        const V3 right = fabsf(dot(vdir, v3(0.0f, 1.0f, 0.0f))) > 0.99f ? cross(vdir, v3(0.0f, 0.0f, 1.0f))
+                                                                      : cross(vdir, v3(0.0f, 1.0f, 0.0f));
+        const V3 up = cross(right, vdir);
+        const V3 dirs[3] = {vdir, right, up};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float len = k == 0 ? speed * PARTICLE_DT + rad * 2.0f : rad * 2.0f;
+            put_ray(rays, (size_t)k * n + i, sub(pos, mul(dirs[k], rad)), dirs[k], len);
         }
-        store(cand_out + i, cand);
-        const Contact g = contact_ray(S, pos, v3(0.0f, -1.0f, 0.0f), 0.0f, rad + 0.001f, timestep, sh);
-        gravity[i] = g.dist < 0.0f ? -9.8f * PARTICLE_DT : 0.0f;
+    } else {
+        for (int k = 0; k < 3; k++) put_ray(rays, (size_t)k * n + i, pos, down, -1.0f);
     }
+    put_ray(rays, 3 * (size_t)n + i, pos, down, rad + 0.001f);
 }
 
-__global__ void __launch_bounds__(PBLK) k_particle_constrain(SceneDev S, const ParticleDev* __restrict__ P,
-                                                             const float* __restrict__ off, uint32_t n, float timestep,
-                                                             float* out) {
-    __shared__ uint2 sh[TRACE_SH_ROWS * PBLK];
-    for (uint32_t i = blockIdx.x * PBLK + threadIdx.x; i < n; i += gridDim.x * PBLK) {
-        const ParticleDev q = P[i];
-        const V3 o = v3(off[3ull * i], off[3ull * i + 1], off[3ull * i + 2]);
-        const float len = length(o);
-        V3 res = v3(0.0f, 0.0f, 0.0f);
-        if (!(len < 0.00001f)) {
-            const V3 dir = v3(o.x / len, o.y / len, o.z / len);
-            const float rad = q.pr.w;
-            const Contact c = contact_ray(S, v3(q.pr.x, q.pr.y, q.pr.z), dir, 0.0f, len + rad, timestep, sh);
-            if (c.dist > 0.0f) {
-                const float m = fmaxf(c.dist - rad * 0.9f, 0.0f), s = rad * 0.05f;
-                res = add(mul(dir, m), mul(c.n, s));
-            } else {
-                res = o;
-            }
+__global__ void __launch_bounds__(PBLK) k_particle_contacts(SceneDev S, const ParticleDev* __restrict__ P,
+                                                            const HitDev* __restrict__ hits,
+                                                            const float4* __restrict__ rays, uint32_t n, float timestep,
+                                                            ContactOut* cand_out, float* gravity) {
+    const uint32_t i = blockIdx.x * PBLK + threadIdx.x;
+    if (i >= n) return;
+    const float4 v4 = P[i].vel;
+    const V3 vel = v3(v4.x, v4.y, v4.z);
+    Contact cand = no_contact();
+    float best = 0.0f;
+    for (int k = 0; k < 3; k++) {
+        const Contact c = contact_at(S, hits, rays, (size_t)k * n + i, timestep);
+        const float w = length(sub(c.v, vel));
+        if (c.dist > 0.0f && w > best) { best = w; cand = c; }
+    }
+    store(cand_out + i, cand);
+    const HitDev& g = hits[3 * (size_t)n + i];
+    gravity[i] = g.flags && g.t >= 0.0f ? 0.0f : -9.8f * PARTICLE_DT;
+}
+
+// the ray of offset i (an empty one for an offset of no length)
+__global__ void __launch_bounds__(PBLK) k_constrain_rays(const ParticleDev* __restrict__ P, const float* __restrict__ off,
+                                                         uint32_t n, float4* rays, uint32_t* work) {
+    const uint32_t i = blockIdx.x * PBLK + threadIdx.x;
+    if (i == 0) *work = 0u;
+    if (i >= n) return;
+    const float4 pr = P[i].pr;
+    const V3 o = v3(off[3ull * i], off[3ull * i + 1], off[3ull * i + 2]), pos = v3(pr.x, pr.y, pr.z);
+    const float len = length(o);
+    if (!(len < 0.00001f)) put_ray(rays, i, pos, v3(o.x / len, o.y / len, o.z / len), len + pr.w);
+    else put_ray(rays, i, pos, v3(0.0f, -1.0f, 0.0f), -1.0f);
+}
+
+__global__ void __launch_bounds__(PBLK) k_constrain(SceneDev S, const ParticleDev* __restrict__ P,
+                                                    const float* __restrict__ off, const HitDev* __restrict__ hits,
+                                                    const float4* __restrict__ rays, uint32_t n, float timestep,
+                                                    float* out) {
+    const uint32_t i = blockIdx.x * PBLK + threadIdx.x;
+    if (i >= n) return;
+    const V3 o = v3(off[3ull * i], off[3ull * i + 1], off[3ull * i + 2]);
+    V3 res = v3(0.0f, 0.0f, 0.0f);
+    if (!(length(o) < 0.00001f)) {
+        const float rad = P[i].pr.w;
+        const Contact c = contact_at(S, hits, rays, i, timestep);
+        if (c.dist > 0.0f) {
+            const float4 b = rays[2ull * i + 1];
+            const float m = fmaxf(c.dist - rad * 0.9f, 0.0f), s = rad * 0.05f;
+            res = add(mul(v3(b.x, b.y, b.z), m), mul(c.n, s));
+        } else {
+            res = o;
         }
-        out[3ull * i] = res.x; out[3ull * i + 1] = res.y; out[3ull * i + 2] = res.z;
     }
+    out[3ull * i] = res.x; out[3ull * i + 1] = res.y; out[3ull * i + 2] = res.z;
 }
 
-inline int pgrid(uint32_t n, int max_blocks) {
-    const uint32_t g = (n + PBLK - 1) / PBLK;
-    return (int)(g < (uint32_t)max_blocks ? (g ? g : 1u) : (uint32_t)max_blocks);
+inline unsigned pgrid(uint32_t n) { return (n + PBLK - 1) / PBLK; }
+
+cudaError_t trace(const SceneDev& S, const ContactScratch& c, const float4* rays, uint32_t n, cudaStream_t s) {
+    return launch_trace_rays(S, rays, n, c.hits, false, c.work, c.grid, c.tune, s);
 }
 
 }  // namespace
 
 cudaError_t launch_contact_rays(const SceneDev& S, const float4* rays, uint32_t n, float timestep, ContactOut* out,
-                                int max_blocks, cudaStream_t s) {
-    k_contact_rays<<<pgrid(n, max_blocks), PBLK, 0, s>>>(S, rays, n, timestep, out);
+                                const ContactScratch& c, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(c.work, 0, sizeof(uint32_t), s);
+    if (e == cudaSuccess) e = trace(S, c, rays, n, s);
+    if (e != cudaSuccess) return e;
+    k_contacts<<<pgrid(n), PBLK, 0, s>>>(S, c.hits, rays, n, timestep, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_particle_probe(const SceneDev& S, const ParticleDev* p, uint32_t n, float timestep,
-                                  ContactOut* cand, float* gravity, int max_blocks, cudaStream_t s) {
-    k_particle_probe<<<pgrid(n, max_blocks), PBLK, 0, s>>>(S, p, n, timestep, cand, gravity);
+                                  ContactOut* cand, float* gravity, const ContactScratch& c, cudaStream_t s) {
+    k_particle_rays<<<pgrid(n), PBLK, 0, s>>>(p, n, c.rays, c.work);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = trace(S, c, c.rays, 4u * n, s);
+    if (e != cudaSuccess) return e;
+    k_particle_contacts<<<pgrid(n), PBLK, 0, s>>>(S, p, c.hits, c.rays, n, timestep, cand, gravity);
     return cudaGetLastError();
 }
 
 cudaError_t launch_particle_constrain(const SceneDev& S, const ParticleDev* p, const float* off, uint32_t n,
-                                      float timestep, float* out, int max_blocks, cudaStream_t s) {
-    k_particle_constrain<<<pgrid(n, max_blocks), PBLK, 0, s>>>(S, p, off, n, timestep, out);
+                                      float timestep, float* out, const ContactScratch& c, cudaStream_t s) {
+    k_constrain_rays<<<pgrid(n), PBLK, 0, s>>>(p, off, n, c.rays, c.work);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = trace(S, c, c.rays, n, s);
+    if (e != cudaSuccess) return e;
+    k_constrain<<<pgrid(n), PBLK, 0, s>>>(S, p, off, c.hits, c.rays, n, timestep, out);
     return cudaGetLastError();
 }
 

@@ -809,21 +809,4 @@ struct PacketTraverser {
     }
 };
 
-// Traces one ray to completion by itself (for kernels that trace inline, e.g.
-// the ReSTIR passes): primitives first, then nodes.
-template <bool ANY, bool COUNT>
-__device__ __forceinline__ bool trace_scene(const SceneDev& S, V3 o, V3 d, float tmin, float tmax, TraceResult& res,
-                                            uint2* sh_stack, uint32_t tid, uint32_t nthreads, TraceCounters* ctr) {
-    Traverser<ANY, COUNT> tv;
-    uint2 spill[STACK_MAX - STACK_SH];
-    tv.init(S, o, d, tmin, tmax, sh_stack, spill, tid, nthreads);
-    for (;;) {
-        tv.settle();
-        if (tv.done) break;
-        if (tv.has_prim()) tv.prim_step(S, ctr);
-        else tv.node_step(S, ctr);
-    }
-    return tv.finish(S, res);
-}
-
 }  // namespace snk

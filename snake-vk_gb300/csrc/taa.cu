@@ -20,9 +20,9 @@
 // Kernel: 32x8 pixels per block, the 34x10 halo tile of the current frame staged
 // in shared memory (coalesced float4 loads, issued first and held in registers
 // until the motion-dependent gathers are in flight), history and previous
-// velocity fetched through L1 (neighbouring pixels share texels).  HBM bound: 88 B per
+// velocity fetched through L1 (neighbouring pixels share texels).  88 B per
 // pixel (16 current + 8 motion + 16 history + 8 previous motion in; 16 out, 16
-// next history, 8 next previous motion).
+// next history, 8 next previous motion).  The first frame reads itself as its history.
 #include <cstring>
 #include <string>
 
@@ -33,6 +33,11 @@ namespace snk {
 namespace {
 
 constexpr int TX = 32, TY = 8;
+constexpr int HALO = 2 * (TX + 2) + 2 * TY;
+static_assert(HALO <= TX * TY, "one halo texel per thread");
+// blocks between a block and the one whose texels it prefetches into L2: about twice
+// as many as run at once
+constexpr int PREFETCH_BLOCKS = 912;
 
 struct TaaImages {
     const float4* cur;
@@ -43,13 +48,35 @@ struct TaaImages {
     float4* hist_next;
     float2* pmot_next;
     int w, h;
+    int ahead;          // rows of blocks from a block down to the one it prefetches for
 };
 
+// repeat addressing of a texel index in [-n, 2n): the coordinate is clamped to [0, 1], so
+// the filter's texels are at most one image away
 __device__ __forceinline__ int wrap_repeat(int i, int n) {
-    int r = i % n;
-    return r < 0 ? r + n : r;
+    if (i < 0) i += n;
+    return i >= n ? i - n : i;
 }
 
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float min3f(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// two channels per addition, each rounded by itself (packed products feeding packed
+// additions came back fused, so the products stay single)
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)),
+        "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
 // texture() with a linear filter and repeat addressing, in FP32: the four texels
 // are fetched first (so that their loads are in flight together with the
 // frame's tile), the weights are applied later
@@ -64,79 +91,30 @@ struct Bilinear {
         const int i0 = wrap_repeat((int)fu, w), i1 = wrap_repeat((int)fu + 1, w);
         const int j0 = wrap_repeat((int)fv, h), j1 = wrap_repeat((int)fv + 1, h);
         w00 = (1.0f - a) * (1.0f - b); w10 = a * (1.0f - b); w01 = (1.0f - a) * b; w11 = a * b;
-        t00 = img[(size_t)j0 * w + i0];
-        t10 = img[(size_t)j0 * w + i1];
-        t01 = img[(size_t)j1 * w + i0];
-        t11 = img[(size_t)j1 * w + i1];
+        const uint32_t r0 = (uint32_t)(j0 * w), r1 = (uint32_t)(j1 * w);   // (an image has at most 2^30 texels)
+        t00 = img[r0 + i0];
+        t10 = img[r0 + i1];
+        t01 = img[r1 + i0];
+        t11 = img[r1 + i1];
     }
-    template <int C>
-    __device__ __forceinline__ void apply(float* o) const {
+    // component k of the filtered value
+    __device__ __forceinline__ float at(int k) const {
         const float* a = reinterpret_cast<const float*>(&t00);
         const float* b = reinterpret_cast<const float*>(&t10);
         const float* c = reinterpret_cast<const float*>(&t01);
         const float* d = reinterpret_cast<const float*>(&t11);
-        for (int k = 0; k < C; k++) o[k] = ((w00 * a[k] + w10 * b[k]) + w01 * c[k]) + w11 * d[k];
+        return ((w00 * a[k] + w10 * b[k]) + w01 * c[k]) + w11 * d[k];
     }
 };
 
-__global__ void __launch_bounds__(TX * TY) k_taa_resolve(TaaImages I) {
-    __shared__ float4 tile[TY + 2][TX + 2];
-    const int bx = blockIdx.x * TX, by = blockIdx.y * TY;
-    const int t = threadIdx.y * TX + threadIdx.x;
-    const int x = bx + threadIdx.x, y = by + threadIdx.y;
-    const bool inside = x < I.w && y < I.h;
-    const size_t pix = inside ? (size_t)y * I.w + x : 0;
-    // the tile's texels first (independent loads, into registers), then this
-    // pixel's motion and its reprojected history and previous-velocity texels
-    constexpr int TN = ((TX + 2) * (TY + 2) + TX * TY - 1) / (TX * TY);
-    float4 tv[TN];
-#pragma unroll
-    for (int q = 0; q < TN; q++) {
-        const int k = t + q * TX * TY;
-        if (k < (TX + 2) * (TY + 2)) {
-            const int ly = k / (TX + 2), lx = k % (TX + 2);
-            const int gx = min(max(bx + lx - 1, 0), I.w - 1), gy = min(max(by + ly - 1, 0), I.h - 1);
-            tv[q] = I.cur[(size_t)gy * I.w + gx];
-        }
-    }
-    float2 vel = make_float2(0.0f, 0.0f);
-    Bilinear<float4> hb;
-    Bilinear<float2> pb;
-    if (inside) {
-        vel = I.motion[pix];
-        float hx = ((float)x + 0.5f) / (float)I.w + vel.x;
-        float hy = ((float)y + 0.5f) / (float)I.h + vel.y;
-        hx = fminf(fmaxf(hx, 0.0f), 1.0f);
-        hy = fminf(fmaxf(hy, 0.0f), 1.0f);
-        hb.fetch(I.hist, I.w, I.h, hx, hy);
-        pb.fetch(I.pmot, I.w, I.h, hx, hy);
-    }
-#pragma unroll
-    for (int q = 0; q < TN; q++) {
-        const int k = t + q * TX * TY;
-        if (k < (TX + 2) * (TY + 2)) tile[k / (TX + 2)][k % (TX + 2)] = tv[q];
-    }
-    __syncthreads();
-    if (!inside) return;
-    const float4 cur4 = tile[threadIdx.y + 1][threadIdx.x + 1];
+// The resolve of one pixel from its neighbourhood's sums and bounds.
+__device__ __forceinline__ float4 resolve_pixel(const float4 cur4, const float* mn, const float* mx, const float* m,
+                                                const float* m2, const Bilinear<float4>& hb, const Bilinear<float2>& pb,
+                                                float2 vel) {
     const float cur[3] = {cur4.x, cur4.y, cur4.z};
-    float mn[3] = {9999.0f, 9999.0f, 9999.0f}, mx[3] = {-9999.0f, -9999.0f, -9999.0f};
-    float m[3] = {0.0f, 0.0f, 0.0f}, m2[3] = {0.0f, 0.0f, 0.0f};
-    for (int ox = -1; ox <= 1; ox++) {
-        for (int oy = -1; oy <= 1; oy++) {
-            // the tile's halo already holds the clamped neighbours
-            const float4 c4 = tile[threadIdx.y + 1 + oy][threadIdx.x + 1 + ox];
-            const float col[3] = {fmaxf(c4.x, 0.0f), fmaxf(c4.y, 0.0f), fmaxf(c4.z, 0.0f)};
-            for (int c = 0; c < 3; c++) {
-                mn[c] = fminf(mn[c], col[c]);
-                mx[c] = fmaxf(mx[c], col[c]);
-                m[c] = m[c] + col[c];
-                m2[c] = m2[c] + col[c] * col[c];
-            }
-        }
-    }
     const float inv9 = 1.0f / 9.0f, gamma = 0.55f, eps = 0.00000001f;
     float mu[3], minc[3], maxc[3], p[3];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
         mu[c] = m[c] * inv9;
         const float sigma = sqrtf(fabsf(m2[c] * inv9 - mu[c] * mu[c]));
@@ -144,11 +122,11 @@ __global__ void __launch_bounds__(TX * TY) k_taa_resolve(TaaImages I) {
         maxc[c] = mu[c] + gamma * sigma;
         p[c] = fminf(fmaxf(mu[c], mn[c]), mx[c]);
     }
-    float hist[3];
-    hb.apply<3>(hist);
     // clip_aabb(minc, maxc, vec4(p, 1), vec4(hist, 1)); r.w stays 0
     float r[3];
-    for (int c = 0; c < 3; c++) r[c] = fmaxf(hist[c], 0.0f) - p[c];
+#pragma unroll
+    for (int c = 0; c < 3; c++) r[c] = fmaxf(hb.at(c), 0.0f) - p[c];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
         const float rmax = maxc[c] - p[c];
         if (r[c] > rmax + eps) {
@@ -156,6 +134,7 @@ __global__ void __launch_bounds__(TX * TY) k_taa_resolve(TaaImages I) {
             for (int k = 0; k < 3; k++) r[k] = r[k] * s;
         }
     }
+#pragma unroll
     for (int c = 0; c < 3; c++) {
         const float rmin = minc[c] - p[c];
         if (r[c] < rmin - eps) {
@@ -163,18 +142,100 @@ __global__ void __launch_bounds__(TX * TY) k_taa_resolve(TaaImages I) {
             for (int k = 0; k < 3; k++) r[k] = r[k] * s;
         }
     }
-    float pv[2];
-    pb.apply<2>(pv);
-    const float vx = pv[0] + vel.x, vy = pv[1] + vel.y;
+    const float vx = pb.at(0) + vel.x, vy = pb.at(1) + vel.y;
     const float vlen = sqrtf(vx * vx + vy * vy);
     const float dis = fminf(fmaxf((vlen - 0.001f) * 10.0f, 0.0f), 1.0f);
     float fin[3];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
         const float hc = p[c] + r[c];
         const float f = cur[c] * (1.0f - 0.9f) + hc * 0.9f;
         fin[c] = f * (1.0f - dis) + mu[c] * dis;
     }
-    const float4 o = make_float4(fin[0], fin[1], fin[2], 1.0f);
+    return make_float4(fin[0], fin[1], fin[2], 1.0f);
+}
+
+// Bound by latency and issue: a thread waits for its motion, then for the texels that
+// it points to, with 24 warps per SM to cover both, and runs some 570 instructions (the
+// exact divisions and square roots among them).  So a block asks L2 for the texels of
+// one that runs later, neither index needs a division, and the bounds take three
+// operands at a time: a 1080p resolve 43 us, 50 before (49 without the prefetch), 88 B per
+// pixel at 4.2 TB/s.  (Two pixels per thread need 126 registers and were slower, as were
+// 512-thread blocks; 64 registers changed nothing.)
+__global__ void __launch_bounds__(TX * TY) k_taa_resolve(TaaImages I) {
+    __shared__ float4 tile[TY + 2][TX + 2];   // clamped to >= 0, as the neighbourhood takes it
+    const int bx = blockIdx.x * TX, by = blockIdx.y * TY;
+    const int t = threadIdx.y * TX + threadIdx.x;
+    const int x = bx + threadIdx.x, y = by + threadIdx.y;
+    const bool inside = x < I.w && y < I.h;
+    const uint32_t pix = inside ? (uint32_t)(y * I.w + x) : 0u;
+    auto texel = [&](int lx, int ly) {   // tile entry (lx, ly): the frame's texel, its edges repeated
+        const int gx = min(max(bx + lx - 1, 0), I.w - 1), gy = min(max(by + ly - 1, 0), I.h - 1);
+        return I.cur[(uint32_t)(gy * I.w + gx)];
+    };
+    auto positive = [](float4 c) { return make_float4(fmaxf(c.x, 0.0f), fmaxf(c.y, 0.0f), fmaxf(c.z, 0.0f), 0.0f); };
+    // the loads that wait for nothing: this thread's texel and motion, one halo texel
+    const float2 vel = inside ? I.motion[pix] : make_float2(0.0f, 0.0f);
+    const float4 own = texel(threadIdx.x + 1, threadIdx.y + 1);
+    float4 halo;
+    int hx = 0, hy = 0;
+    if (t < HALO) {
+        if (t < 2 * (TX + 2)) {
+            hx = t < TX + 2 ? t : t - (TX + 2);
+            hy = t < TX + 2 ? 0 : TY + 1;
+        } else {
+            hx = (t & 1) * (TX + 1);
+            hy = 1 + ((t - 2 * (TX + 2)) >> 1);
+        }
+        halo = texel(hx, hy);
+    }
+    {   // the later block's rows of the four images, one 128-byte line per thread: 4 lines
+        // of the frame and of the history, 2 of each motion
+        const int py = by + I.ahead * TY + (t & (TY - 1)), line = t / TY;
+        const int px = line < 8 ? bx + 8 * (line & 3) : bx + 16 * (line & 1);
+        if (line < 12 && py < I.h && px < I.w) {
+            const uint32_t at = (uint32_t)(py * I.w + px);
+            const void* p = line < 4 ? (const void*)(I.cur + at) : line < 8 ? (const void*)(I.hist + at)
+                          : line < 10 ? (const void*)(I.motion + at) : (const void*)(I.pmot + at);
+            asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
+        }
+    }
+    // then the reprojected history and previous velocity
+    Bilinear<float4> hb;
+    Bilinear<float2> pb;
+    if (inside) {
+        float u = ((float)x + 0.5f) / (float)I.w + vel.x;
+        float v = ((float)y + 0.5f) / (float)I.h + vel.y;
+        u = fminf(fmaxf(u, 0.0f), 1.0f);
+        v = fminf(fmaxf(v, 0.0f), 1.0f);
+        hb.fetch(I.hist, I.w, I.h, u, v);
+        pb.fetch(I.pmot, I.w, I.h, u, v);
+    }
+    tile[threadIdx.y + 1][threadIdx.x + 1] = positive(own);
+    if (t < HALO) tile[hy][hx] = positive(halo);
+    __syncthreads();
+    if (!inside) return;
+    // neighbourhood sums in the shader's order (columns, then rows) and bounds
+    float2 sxy = make_float2(0.0f, 0.0f), qxy = sxy;
+    float sz = 0.0f, qz = 0.0f;
+    float mn[3] = {9999.0f, 9999.0f, 9999.0f}, mx[3] = {-9999.0f, -9999.0f, -9999.0f};
+#pragma unroll
+    for (int ox = 0; ox < 3; ox++) {
+        float4 col[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float4 c = col[k] = tile[threadIdx.y + k][threadIdx.x + ox];
+            sxy = add2(sxy, make_float2(c.x, c.y));
+            qxy = add2(qxy, make_float2(c.x * c.x, c.y * c.y));
+            sz = sz + c.z;
+            qz = qz + c.z * c.z;
+        }
+        mn[0] = fminf(min3f(mn[0], col[0].x, col[1].x), col[2].x); mx[0] = fmaxf(max3f(mx[0], col[0].x, col[1].x), col[2].x);
+        mn[1] = fminf(min3f(mn[1], col[0].y, col[1].y), col[2].y); mx[1] = fmaxf(max3f(mx[1], col[0].y, col[1].y), col[2].y);
+        mn[2] = fminf(min3f(mn[2], col[0].z, col[1].z), col[2].z); mx[2] = fmaxf(max3f(mx[2], col[0].z, col[1].z), col[2].z);
+    }
+    const float m[3] = {sxy.x, sxy.y, sz}, m2[3] = {qxy.x, qxy.y, qz};
+    const float4 o = resolve_pixel(own, mn, mx, m, m2, hb, pb, vel);
     if (I.out) I.out[pix] = o;
     I.hist_next[pix] = o;
     I.pmot_next[pix] = vel;
@@ -270,17 +331,12 @@ int snk_taa_resolve(snk_taa* t, const float* radiance, const float* motion, floa
                                                 "and 8-byte (motion) aligned");
     }
     const int nxt = t->cur ^ 1;
-    if (!t->valid) {
-        // first frame: the history is the current frame, the previous motion this frame's
-        if (cudaMemcpyAsync(t->hist[t->cur].p, cur, np * sizeof(float4), cudaMemcpyDeviceToDevice, st) ||
-            cudaMemcpyAsync(t->pmot[t->cur].p, mot, np * sizeof(float2), cudaMemcpyDeviceToDevice, st))
-            return taa_fail(t, SNK_ERR_CUDA, "taa_resolve: history seed");
-    }
     TaaImages I;
     I.cur = cur;
     I.motion = mot;
-    I.hist = t->hist[t->cur].p;
-    I.pmot = t->pmot[t->cur].p;
+    // first frame: the history is the current frame, the previous motion this frame's
+    I.hist = t->valid ? t->hist[t->cur].p : cur;
+    I.pmot = t->valid ? t->pmot[t->cur].p : mot;
     // in place (or host output): write the history only, then copy it out
     const bool direct = memory == SNK_MEM_DEVICE && out != radiance;
     I.out = direct ? reinterpret_cast<float4*>(out) : nullptr;
@@ -289,6 +345,7 @@ int snk_taa_resolve(snk_taa* t, const float* radiance, const float* motion, floa
     I.w = (int)t->w;
     I.h = (int)t->h;
     dim3 grid((t->w + TX - 1) / TX, (t->h + TY - 1) / TY);
+    I.ahead = (PREFETCH_BLOCKS + (int)grid.x - 1) / (int)grid.x;
     k_taa_resolve<<<grid, dim3(TX, TY), 0, st>>>(I);
     if (cudaGetLastError() != cudaSuccess) return taa_fail(t, SNK_ERR_CUDA, "taa_resolve: launch");
     if (!direct) {

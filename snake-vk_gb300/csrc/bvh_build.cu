@@ -1656,20 +1656,78 @@ k_refit_small(WideNode* nodes, uint32_t node_base, uint32_t prim_base, const Sma
     }
 }
 
+// the 13 axes of a mesh's extents (MeshExtents): x y z, x+y x-y, x+z x-z, y+z y-z, then
+// x+y+z x+y-z x-y+z x-y-z
+__device__ __forceinline__ void extent_axes(const float* q, float* d) {
+    d[0] = q[0]; d[1] = q[1]; d[2] = q[2];
+    d[3] = q[0] + q[1]; d[4] = q[0] - q[1];
+    d[5] = q[0] + q[2]; d[6] = q[0] - q[2];
+    d[7] = q[1] + q[2]; d[8] = q[1] - q[2];
+    d[9] = d[3] + q[2]; d[10] = d[3] - q[2]; d[11] = d[4] + q[2]; d[12] = d[4] - q[2];
+}
+
 // primitive i of the concatenated meshes (BuildTrees over the meshes that have
-// triangles, tree_mesh[t] their indices): padded box of its triangle
-__global__ void k_triangle_boxes(const float* __restrict__ pos, const uint32_t* __restrict__ idx, BuildTrees B,
-                                 const uint32_t* __restrict__ tree_mesh, const MeshInfo* __restrict__ meshes, float4* lo,
-                                 float4* hi) {
+// triangles, tree_mesh[t] their indices): padded box of its triangle, and its part of
+// the mesh's extents (zero at the start)
+__global__ void __launch_bounds__(BLK) k_triangle_boxes(const float* __restrict__ pos, const uint32_t* __restrict__ idx,
+                                                        BuildTrees B, const uint32_t* __restrict__ tree_mesh,
+                                                        const MeshInfo* __restrict__ meshes, MeshExtents* extents,
+                                                        float4* lo, float4* hi) {
+    __shared__ unsigned red[BLK / 32][26];
     const uint32_t i = blockIdx.x * BLK + threadIdx.x;
-    if (i >= B.total) return;
-    const uint32_t tree = tree_of(B, i), t = i - tree_begin(B, tree);
-    const MeshInfo& M = meshes[__ldg(tree_mesh + tree)];
+    const bool valid = i < B.total;
+    const uint32_t tree = tree_of(B, valid ? i : B.total - 1u), first = tree_begin(B, tree), t = i - first;
+    const uint32_t mesh = __ldg(tree_mesh + tree);
+    const MeshInfo& M = meshes[mesh];
     float l[3] = {3.4e38f, 3.4e38f, 3.4e38f}, h[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-    for (int k = 0; k < 3; k++) {
-        const float* p = pos + 3ull * (M.vertex_offset + idx[M.index_offset + 3ull * t + k]);
-        for (int a = 0; a < 3; a++) { l[a] = fminf(l[a], p[a]); h[a] = fmaxf(h[a], p[a]); }
+    unsigned ext26[26];   // order-preserving codes: largest along each axis, complements of the smallest
+    for (int k = 0; k < 26; k++) ext26[k] = 0u;
+    if (valid) {
+        const float* c = pos + 3ull * (M.vertex_offset + idx[M.index_offset]);   // the mesh's reference point
+        for (int k = 0; k < 3; k++) {
+            const float* p = pos + 3ull * (M.vertex_offset + idx[M.index_offset + 3ull * t + k]);
+            for (int a = 0; a < 3; a++) { l[a] = fminf(l[a], p[a]); h[a] = fmaxf(h[a], p[a]); }
+            const float q[3] = {p[0] - c[0], p[1] - c[1], p[2] - c[2]};
+            float d[13];
+            extent_axes(q, d);
+#pragma unroll
+            for (int a = 0; a < 13; a++) {
+                const unsigned e = enc_f(d[a]);
+                ext26[a] = max(ext26[a], e);
+                ext26[13 + a] = max(ext26[13 + a], ~e);
+            }
+        }
+        if (t == 0u)
+            for (int a = 0; a < 3; a++) extents[mesh].ref[a] = c[a];
     }
+    {   // one atomic per axis and block (or warp, where the block holds several meshes)
+        const uint32_t b0 = blockIdx.x * BLK, w0 = i & ~31u;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const bool block_one = min(b0 + BLK, B.total) <= tree_end(B, tree_of(B, b0));
+        const bool warp_one = __all_sync(0xFFFFFFFFu, !valid || w0 >= first);
+        unsigned mine = 0u;
+#pragma unroll
+        for (int k = 0; k < 26; k++) {
+            const unsigned m = __reduce_max_sync(0xFFFFFFFFu, ext26[k]);
+            if (lane == k) mine = m;
+        }
+        unsigned* dst = extents[mesh].code;
+        if (block_one) {
+            if (lane < 26) red[warp][lane] = mine;
+            __syncthreads();
+            if (threadIdx.x < 26) {
+                unsigned m = 0u;
+                for (int w = 0; w < BLK / 32; w++) m = max(m, red[w][threadIdx.x]);
+                atomicMax(&dst[threadIdx.x], m);
+            }
+        } else if (warp_one) {
+            if (lane < 26 && w0 < B.total) atomicMax(&dst[lane], mine);
+        } else if (valid) {
+#pragma unroll
+            for (int k = 0; k < 26; k++) atomicMax(&dst[k], ext26[k]);
+        }
+    }
+    if (!valid) return;
     float ext = fmaxf(fmaxf(h[0] - l[0], h[1] - l[1]), h[2] - l[2]);
     for (int a = 0; a < 3; a++) {
         float pad = 1e-5f * (ext + fabsf(l[a]) + fabsf(h[a])) + 1e-7f;
@@ -1706,18 +1764,62 @@ __global__ void k_fill_triangles(const uint32_t* __restrict__ order, BuildTrees 
     }
 }
 
+// How far a mesh reaches from its reference point along direction n, at most: with
+// |n| sorted as p >= q >= r, n = (p - q) axis + (q - r) edge + r corner of the cube's
+// directions, and what a shape reaches along a sum of directions is at most the sum of
+// what it reaches along each.
+__device__ __forceinline__ float reach(const MeshExtents& E, const float* n) {
+    const float a[3] = {fabsf(n[0]), fabsf(n[1]), fabsf(n[2])};
+    const bool neg[3] = {n[0] < 0.0f, n[1] < 0.0f, n[2] < 0.0f};
+    auto along = [&](int axis, bool minus) {   // along +axis or -axis
+        return minus ? -dec_f(~E.code[13 + axis]) : dec_f(E.code[axis]);
+    };
+    int p = 0, r = 0;
+    if (a[1] > a[p]) p = 1;
+    if (a[2] > a[p]) p = 2;
+    if (a[1] <= a[r]) r = 1;
+    if (a[2] <= a[r]) r = 2;
+    if (p == r) { p = 0; r = 2; }   // (all alike)
+    const int q = 3 - p - r, lo = min(p, q), hi = max(p, q);
+    const int edge = (lo == 0 ? (hi == 1 ? 3 : 5) : 7) + (neg[lo] != neg[hi] ? 1 : 0);
+    const int corner = 9 + (neg[1] != neg[0] ? 2 : 0) + (neg[2] != neg[0] ? 1 : 0);
+    return (a[p] - a[q]) * along(p, neg[p]) + (a[q] - a[r]) * along(edge, neg[lo]) + a[r] * along(corner, neg[0]);
+}
+
+// World box of an instance: the box of its mesh's box corners, cut to what the mesh
+// reaches along the box's own directions (26 object-space extents: a rotated mesh that
+// does not fill its box gets a box of its own size, not of the box's corners; a
+// sphere's is 1.1 to 1.2 instead of up to 1.7 times its diameter), with 1 % of the extent
+// to spare for the roundings of the object-space ray (0.1 % to spare gave 0.3 % more on
+// the terrain, 5 % to spare took 1 % back).  A ray that enters an instance and leaves it
+// without a hit costs its transform and a walk from the mesh's root: over 4,097 turned
+// spheres, a 1920x1080 path-traced frame 1.997 -> 1.918 ms, one with reservoirs 16.98 ->
+// 16.40 ms, 2^20 device rays 370 -> 347 us; the eight-view terrain (19.2 Mpx) 2.3 % less
+// over eight seeds.  The extents cost the mesh build 12 us at 132,000 triangles
+// (k_triangle_boxes 3 -> 7 us and a memset).
 __global__ void k_instance_boxes(const uint32_t* __restrict__ list, uint32_t n, const InstShade* __restrict__ inst,
-                                 const MeshInfo* __restrict__ meshes, float4* lo, float4* hi) {
+                                 const MeshInfo* __restrict__ meshes, const MeshExtents* __restrict__ extents,
+                                 float4* lo, float4* hi) {
     uint32_t i = blockIdx.x * BLK + threadIdx.x;
     if (i >= n) return;
     const InstShade& I = inst[list[i]];
     const MeshInfo& M = meshes[I.mesh_id];
+    const MeshExtents& E = extents[I.mesh_id];
     float l[3] = {3.4e38f, 3.4e38f, 3.4e38f}, h[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
     for (int c = 0; c < 8; c++) {
         V3 p = v3((c & 1) ? M.hi[0] : M.lo[0], (c & 2) ? M.hi[1] : M.lo[1], (c & 4) ? M.hi[2] : M.lo[2]);
         V3 q = xform_point(I.m, p);
         l[0] = fminf(l[0], q.x); l[1] = fminf(l[1], q.y); l[2] = fminf(l[2], q.z);
         h[0] = fmaxf(h[0], q.x); h[1] = fmaxf(h[1], q.y); h[2] = fmaxf(h[2], q.z);
+    }
+    const V3 ref = xform_point(I.m, v3(E.ref[0], E.ref[1], E.ref[2]));
+    const float r[3] = {ref.x, ref.y, ref.z};
+    for (int a = 0; a < 3; a++) {
+        const float up[3] = {I.m[4 * a], I.m[4 * a + 1], I.m[4 * a + 2]}, down[3] = {-up[0], -up[1], -up[2]};
+        const float zl = r[a] - reach(E, down), zh = r[a] + reach(E, up);
+        const float spare = 0.01f * (zh - zl);
+        if (zl - spare > l[a]) l[a] = zl - spare;   // (false for a NaN: the corners' box stays)
+        if (zh + spare < h[a]) h[a] = zh + spare;
     }
     float ext = fmaxf(fmaxf(h[0] - l[0], h[1] - l[1]), h[2] - l[2]);
     for (int a = 0; a < 3; a++) {
@@ -1898,8 +2000,10 @@ Status refit_wide_bvh(const float4* prim_lo, const float4* prim_hi, uint32_t n, 
 }
 
 Status launch_triangle_boxes(const float* positions, const uint32_t* indices, const BuildTrees& B,
-                             const uint32_t* tree_mesh, const MeshInfo* meshes, float4* lo, float4* hi, cudaStream_t s) {
-    if (B.total) k_triangle_boxes<<<grid_for(B.total), BLK, 0, s>>>(positions, indices, B, tree_mesh, meshes, lo, hi);
+                             const uint32_t* tree_mesh, const MeshInfo* meshes, MeshExtents* extents, float4* lo,
+                             float4* hi, cudaStream_t s) {
+    if (B.total)
+        k_triangle_boxes<<<grid_for(B.total), BLK, 0, s>>>(positions, indices, B, tree_mesh, meshes, extents, lo, hi);
     SNK_TRY_CUDA(cudaGetLastError());
     return Status::Ok();
 }
@@ -1915,8 +2019,8 @@ Status launch_fill_triangles(const BuildScratch& sc, const uint32_t* order, cons
 }
 
 Status launch_instance_boxes(const uint32_t* list, uint32_t n, const InstShade* inst, const MeshInfo* meshes,
-                             float4* lo, float4* hi, cudaStream_t s) {
-    if (n) k_instance_boxes<<<grid_for(n), BLK, 0, s>>>(list, n, inst, meshes, lo, hi);
+                             const MeshExtents* extents, float4* lo, float4* hi, cudaStream_t s) {
+    if (n) k_instance_boxes<<<grid_for(n), BLK, 0, s>>>(list, n, inst, meshes, extents, lo, hi);
     SNK_TRY_CUDA(cudaGetLastError());
     return Status::Ok();
 }

@@ -82,6 +82,15 @@ struct BuildScratch {
     DBuf<uint32_t> wide_split;    // per binary internal node: the split of those children (4-bit fields)
 };
 
+// How far a mesh reaches from one of its vertices (ref) along 13 axes: order-preserving
+// codes of the largest distances, then the complements of the codes of the smallest
+// (made by atomic maxima, so zero is the start).
+struct MeshExtents {
+    unsigned code[26];
+    float ref[3];
+    unsigned pad[3];
+};
+
 // The trees of one build: tree t's primitives are [first[t], first[t + 1]) of the
 // concatenated boxes (device array of count + 1, each tree at least one primitive;
 // not read for a single tree)
@@ -131,17 +140,19 @@ Status refit_wide_bvh(const float4* prim_lo, const float4* prim_hi, uint32_t n, 
                       uint32_t prim_base, const uint32_t* prim_order, const SmallBuildOut* info, float4* wide_box,
                       const uint32_t* wide_depth, unsigned* err_word, cudaStream_t stream);
 
-// Padded object-space boxes of the triangles of B's meshes (tree t is mesh tree_mesh[t]).
+// Padded object-space boxes of the triangles of B's meshes (tree t is mesh tree_mesh[t]),
+// and the meshes' extents (zeroed by the caller).
 Status launch_triangle_boxes(const float* positions, const uint32_t* indices, const BuildTrees& B,
-                             const uint32_t* tree_mesh, const MeshInfo* meshes, float4* lo, float4* hi, cudaStream_t s);
+                             const uint32_t* tree_mesh, const MeshInfo* meshes, MeshExtents* extents, float4* lo,
+                             float4* hi, cudaStream_t s);
 // Triangle records from the build's primitive order, and the meshes' root nodes
 // (node_base + t) and bounds (after the build that left its trees in sc).
 Status launch_fill_triangles(const BuildScratch& sc, const uint32_t* prim_order, const BuildTrees& B,
                              const uint32_t* tree_mesh, uint32_t node_base, MeshInfo* meshes, const float* positions,
                              const uint32_t* indices, TriRecord* out, cudaStream_t s);
-// World boxes of the listed instances (transform of the mesh bounds) for the instance BVH.
+// World boxes of the listed instances (from the mesh bounds and extents) for the instance BVH.
 Status launch_instance_boxes(const uint32_t* inst_list, uint32_t n, const InstShade* inst, const MeshInfo* meshes,
-                             float4* lo, float4* hi, cudaStream_t s);
+                             const MeshExtents* extents, float4* lo, float4* hi, cudaStream_t s);
 // ---- per-frame scene tables (scene_tables.cu) ---------------------------------
 struct LightCdfScratch {
     DBuf<unsigned long long> acc, wmax, tile_sums, q;   // prefix sums, max weight, tile sums, quantised weights

@@ -431,17 +431,23 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 // ---- treelet restructuring -----------------------------------------------------
 // Bound by latency: a climb towards the root is a chain of treelets, each of which
 // waits for the one below it (about 20 on the way up a 131,072-triangle tree).  So a
-// warp works one treelet out with all its lanes and as few dependent loads as there
-// are levels in it: lane k holds treelet leaf k (box, cost, count, children), an
-// opened leaf's two children are fetched by two lanes at once, the subsets of each
-// size are costed one per lane (four lanes share a subset of six leaves), and the
-// six rewritten nodes are stored by six lanes.  Subtrees below seven primitives only
-// need their cost, which each lane works out for its own node.  Loading 50 small meshes
-// (150 passes then) took 58.1 ms with one lane growing and rewriting every treelet and
-// small subtrees costed one after another, 29.3 ms so; a 131,072-triangle terrain and a
-// sphere 5.77 and 3.66 ms; the trees are the same bit for bit.  With 64 registers (four
-// blocks per SM) all of a large mesh's warps run at once: terrain and sphere 2.43 and
-// 2.18 ms.
+// warp works one treelet out with all its lanes and as few dependent loads as it can:
+// the four levels below the root are fetched a level at a time, before it is known which
+// of their nodes will be opened (30 lanes, a node each; seven rounds of loads when every
+// opening waited for its own), the subsets of each size are costed one per lane (four
+// lanes share a subset of six leaves), and the six rewritten nodes are stored by six
+// lanes.  A treelet whose present form costs no more than the best one stays as it is
+// without the rewriting, the stores and the wait for them: 21 %, 63 % and 82 % of the
+// treelets of the three passes.  Subtrees below seven primitives only need their cost,
+// which each lane works out for its own node.  A node's parent, children and count are
+// loaded before the arrival at it, not after.
+// Loading 50 small meshes (150 passes then) took 58.1 ms with one lane growing and
+// rewriting every treelet and small subtrees costed one after another, 29.3 ms with lane
+// k opening and storing leaf and node k; a 131,072-triangle terrain and a sphere 5.77 and
+// 3.66 ms.  With 64 registers (four blocks per SM) all of a large mesh's warps run at
+// once: terrain and sphere 2.43 and 2.18 ms.  Four levels at a time, kept forms and the
+// early loads: 1.885 and 1.658 ms (three passes about 250 and 170 us each), 50 small
+// meshes, now built together, 1.452 and 1.279 ms; the trees' SAH costs agree to 1e-5.
 constexpr int TL_LEAVES = 7;
 constexpr int TL_SUBSETS = 1 << TL_LEAVES;
 constexpr int TL_WARPS = BLK / 32;
@@ -522,20 +528,20 @@ __device__ __forceinline__ void treelet_min(float& best, uint32_t& bp, int lanes
     }
 }
 
-// Optimises the treelet rooted at `root`, a subtree of at least TL_LEAVES primitives
-// (all 32 lanes of the warp call this).  Internal nodes have ids below nl.
+// Optimises the treelet rooted at `root` (children rc), a subtree of at least TL_LEAVES
+// primitives (all 32 lanes of the warp call this).  Internal nodes have ids below nl.
 template <bool G>
-__device__ void treelet_optimise(int root, int nl, int2* children, int* parent, float4* node_lo, float4* node_hi,
-                                 uint32_t* leaf_count, float* cost, TreeletSmem& T, const TreeletLane& mine,
-                                 uint32_t leaf_max) {
+__device__ void treelet_optimise(int root, int2 rc, int nl, int2* children, int* parent, float4* node_lo,
+                                 float4* node_hi, uint32_t* leaf_count, float* cost, TreeletSmem& T,
+                                 const TreeletLane& mine, uint32_t leaf_max) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
-    // grow: open the largest treelet leaf until there are seven.  A leaf's children are
-    // fetched with its box, so each step waits for one round of loads.
-    int id = 0, inner = root;   // lane k: treelet leaf k / internal node k
+    // the four levels below the root, a round of loads for each: lanes 0 and 1 the root's
+    // children, lanes 2 h + 2 and 2 h + 3 those of lane h
+    int id = lane == 0 ? rc.x : rc.y, inner = root;   // lane k: a node / internal node k of the treelet
     float area = 0.0f;
     int2 ch = make_int2(0, 0);
-    float4 lo, hi;
+    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
     auto fetch = [&](int c) {
         id = c;
         lo = ldx<G>(&node_lo[c]);
@@ -547,23 +553,45 @@ __device__ void treelet_optimise(int root, int nl, int2* children, int* parent, 
         lo.w = k;
         hi.w = __uint_as_float(n);
     };
-    const int2 rc = ldx<G>(&children[root]);
-    if (lane < 2) fetch(lane == 0 ? rc.x : rc.y);
+    bool have = lane < 2;
+    if (have) fetch(id);
+#pragma unroll
+    for (int first = 2; first < 30; first = 2 * first + 2) {   // 2, 6, 14
+        const int from = (lane >> 1) - 1;   // (lane - 2) / 2
+        const int bx = __shfl_sync(FULL, ch.x, from), by = __shfl_sync(FULL, ch.y, from);
+        const bool opens = __shfl_sync(FULL, have && id < nl, from);
+        if (lane >= first && lane < 2 * first + 2 && opens) {
+            have = true;
+            fetch((lane & 1) ? by : bx);
+        }
+    }
+    // grow: open the largest treelet leaf until there are seven; the children of a node of
+    // the fourth level are fetched, into its lane and lane 30 or 31
+    // (a subtree of >= 7 primitives always has an internal node to open; areas are >= 0)
+    unsigned leaves = 3u;
+    const float unchanged = __shfl_sync(FULL, lo.w, 0) + __shfl_sync(FULL, lo.w, 1);
+    int spare = 30;
 #pragma unroll
     for (int nleaf = 2; nleaf < TL_LEAVES; nleaf++) {
-        // (a subtree of >= 7 primitives always has an internal node to open; areas are >= 0)
-        const unsigned key = (lane < nleaf && id < nl) ? __float_as_uint(area) + 1u : 0u;
+        const unsigned key = (((leaves >> lane) & 1u) && id < nl) ? __float_as_uint(area) + 1u : 0u;
         const unsigned mx = __reduce_max_sync(FULL, key);
         const int best = __ffs(__ballot_sync(FULL, key == mx)) - 1;
-        const int bx = __shfl_sync(FULL, ch.x, best), by = __shfl_sync(FULL, ch.y, best);
         const int opened = __shfl_sync(FULL, id, best);
         if (lane == nleaf - 1) inner = opened;
-        if (lane == best || lane == nleaf) fetch(lane == best ? bx : by);
+        if (best < 14) {
+            leaves = (leaves & ~(1u << best)) | (3u << (2 * best + 2));
+        } else {
+            const int bx = __shfl_sync(FULL, ch.x, best), by = __shfl_sync(FULL, ch.y, best);
+            if (lane == best || lane == spare) fetch(lane == best ? bx : by);
+            leaves |= 1u << spare;
+            spare++;
+        }
     }
-    if (lane < TL_LEAVES) {
-        T.lo[lane] = lo;
-        T.hi[lane] = hi;
-        T.leaf[lane] = id;
+    if ((leaves >> lane) & 1u) {
+        const int k = __popc(leaves & ((1u << lane) - 1u));
+        T.lo[k] = lo;
+        T.hi[k] = hi;
+        T.leaf[k] = id;
     }
     __syncwarp();
     // areas and primitive counts of the subsets lane + 32 h: the union of the leaves
@@ -637,34 +665,39 @@ __device__ void treelet_optimise(int root, int nl, int2* children, int* parent, 
             if (c < best) { best = c; bp = P; }
         }
         treelet_min(best, bp, 32);
+        // (the costs of the nodes inside were stored when each was the root)
+        const float area_root = T.area[full];
+        const uint32_t n_root = T.count[full];
+        if (!(best < unchanged)) {
+            if (lane == 0) cost[root] = node_cost(area_root, n_root, unchanged, leaf_max);
+            __syncwarp();
+            return;
+        }
         if (lane == 0) {
-            T.cost[full] = node_cost(T.area[full], T.count[full], best, leaf_max);
+            T.cost[full] = node_cost(area_root, n_root, best, leaf_max);
             T.part[full] = (uint8_t)bp;
         }
     }
     __syncwarp();
-    // rewrite the treelet's six internal nodes: every lane follows the partitions,
-    // lane k keeps and stores node k
-    uint32_t sub = lane == 0 ? TL_SUBSETS - 1 : 0u;
-    int2 kids = make_int2(0, 0);
-    int next = 1;
+    // rewrite the treelet's six internal nodes: every lane follows the partitions (the
+    // nodes' subsets in order, a byte each), lane k keeps and stores node k
+    unsigned long long queue = TL_SUBSETS - 1;
+    uint32_t sub = 0u, part = 0u;
+    int at0 = 0, at1 = 0, next = 1;
 #pragma unroll
     for (int k = 0; k < TL_LEAVES - 1; k++) {
-        const uint32_t s = __shfl_sync(FULL, sub, k);
-        const uint32_t half[2] = {T.part[s], s ^ T.part[s]};
-        int c[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            if (__popc(half[h]) == 1) {
-                c[h] = T.leaf[__ffs(half[h]) - 1];
-            } else {
-                if (lane == next) sub = half[h];
-                c[h] = __shfl_sync(FULL, inner, next);
-                next++;
-            }
-        }
-        if (lane == k) kids = make_int2(c[0], c[1]);
+        const uint32_t u = (uint32_t)(queue >> (8 * k)) & 0xFFu, a = T.part[u], b = u ^ a;
+        const int i0 = next;
+        if (__popc(a) > 1) queue |= (unsigned long long)a << (8 * next++);
+        const int i1 = next;
+        if (__popc(b) > 1) queue |= (unsigned long long)b << (8 * next++);
+        if (lane == k) { sub = u; part = a; at0 = i0; at1 = i1; }
     }
+    int2 kids;
+    kids.x = __shfl_sync(FULL, inner, at0);
+    kids.y = __shfl_sync(FULL, inner, at1);
+    if (__popc(part) == 1) kids.x = T.leaf[__ffs(part) - 1];
+    if (__popc(sub ^ part) == 1) kids.y = T.leaf[__ffs(sub ^ part) - 1];
     if (lane < TL_LEAVES - 1) {
         children[inner] = kids;
         parent[kids.x] = inner;
@@ -704,17 +737,20 @@ __device__ void treelet_climb(int j, int n, int nl, int2* children, int* parent,
     }
     while (true) {
         bool ready = false, big = false;
+        int2 ch = make_int2(0, 0);
         if (active) {
-            active = ready = arrive_second<G>(&flags[p]);
-        }
-        if (ready) {
+            // (nothing below p changes these, and what is above comes later)
             up = ldx<G>(&parent[p]);
-            const int2 ch = ldx<G>(&children[p]);
-            const uint32_t total = FIRST ? join_children<G>(p, ch, node_lo, node_hi, leaf_count) : ldx<G>(&leaf_count[p]);
-            big = total >= (uint32_t)TL_LEAVES;
-            if (!big) {
-                const float c = ldx<G>(&cost[ch.x]) + ldx<G>(&cost[ch.y]);
-                cost[p] = node_cost(half_area(ldx<G>(&node_lo[p]), ldx<G>(&node_hi[p])), total, c, leaf_max);
+            ch = ldx<G>(&children[p]);
+            uint32_t total = FIRST ? 0u : ldx<G>(&leaf_count[p]);
+            active = ready = arrive_second<G>(&flags[p]);
+            if (ready) {
+                if (FIRST) total = join_children<G>(p, ch, node_lo, node_hi, leaf_count);
+                big = total >= (uint32_t)TL_LEAVES;
+                if (!big) {
+                    const float c = ldx<G>(&cost[ch.x]) + ldx<G>(&cost[ch.y]);
+                    cost[p] = node_cost(half_area(ldx<G>(&node_lo[p]), ldx<G>(&node_hi[p])), total, c, leaf_max);
+                }
             }
         }
         __syncwarp();
@@ -723,7 +759,8 @@ __device__ void treelet_climb(int j, int n, int nl, int2* children, int* parent,
             const int l = __ffs(m) - 1;
             m &= m - 1;
             const int root = __shfl_sync(0xFFFFFFFFu, p, l);
-            treelet_optimise<G>(root, nl, children, parent, node_lo, node_hi, leaf_count, cost, T, mine, leaf_max);
+            const int2 rc = make_int2(__shfl_sync(0xFFFFFFFFu, ch.x, l), __shfl_sync(0xFFFFFFFFu, ch.y, l));
+            treelet_optimise<G>(root, rc, nl, children, parent, node_lo, node_hi, leaf_count, cost, T, mine, leaf_max);
         }
         if (ready) {
             p = up;

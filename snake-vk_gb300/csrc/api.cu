@@ -75,6 +75,7 @@ struct snk_pt_ctx {
     DBuf<uint32_t> d_tlas_prims;
     uint32_t tlas_root = INVALID;
     uint64_t blas_nodes = 0, tlas_nodes = 0, total_tris = 0, tlas_prim_count = 0;
+    uint64_t instance_tris = 0;   // triangles of all instances
     double blas_sah = 0.0;
     bool blas_leaf_single = true;      // the mesh BVHs were built with one primitive per leaf
     bool tlas_leaf_single = true;      // the instance BVH was built with one instance per leaf
@@ -374,6 +375,7 @@ Status build_instances(snk_pt_ctx* ctx) {
     std::vector<uint32_t> list, emissive, em_first;
     list.reserve(ni);
     uint64_t n_em_tris = 0;
+    ctx->instance_tris = 0;
     for (size_t i = 0; i < ni; i++) {
         const snk_instance& in = ctx->instances[i];
         if (in.mesh_id >= ctx->meshes.size()) return Status::Err(SNK_ERR_INVALID_ARG, "instance mesh_id out of range");
@@ -382,6 +384,7 @@ Status build_instances(snk_pt_ctx* ctx) {
         const MeshInfo& M = ctx->h_meshes[in.mesh_id];
         if (M.blas_root == INVALID) continue;
         list.push_back((uint32_t)i);
+        ctx->instance_tris += M.num_triangles;
         if (ctx->materials[in.material_id].flags & SNK_MAT_EMISSIVE) {
             emissive.push_back((uint32_t)i);
             em_first.push_back((uint32_t)n_em_tris);
@@ -1083,13 +1086,16 @@ int render_impl(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, cons
     F.seed = restir_pt ? rs.seed + 0x9E3779B9u * rs.frame_index : rs.seed;
     F.n_paths = n_paths;
     F.n_pixels = (uint32_t)n_pixels;
-    // camera packets: every view large, single-primitive leaves, the default
+    // camera packets: every view large for its scene, single-primitive leaves, the default
     // traversal bounds (their limits are per ray) and no counting of traversal work
     F.packet_primary = F.S.single_leaf && !(rs.flags & SNK_RENDER_COUNT_NODES) &&
                        F.S.max_steps == MAX_TRAVERSAL_STEPS && F.S.stack_max >= STACK_MAX;
     for (uint32_t v = 0; v < num_views; v++) {
         const uint32_t w = views[v].width, h = views[v].height;
-        if (w % PACKET_TILE_W || h % PACKET_TILE_H || (uint64_t)w * h < PACKET_MIN_PIXELS) F.packet_primary = 0u;
+        const double rays = (double)((uint64_t)w * h * spp);
+        if (w % PACKET_TILE_W || h % PACKET_TILE_H || rays < (double)PACKET_MIN_RAYS ||
+            rays * rays < PACKET_RAYS2 * (double)ctx->instance_tris)
+            F.packet_primary = 0u;
     }
     F.tune = trace_tuning(ctx);
     F.tune_any = any_tuning(ctx);

@@ -9,10 +9,25 @@ namespace snk {
 constexpr uint32_t MAX_DEPTH = 16;
 constexpr uint32_t MAX_VIEWS = 64;
 
-// counters (uint32) of one frame, zeroed at frame start
-constexpr uint64_t PACKET_MIN_PIXELS = 1280ull * 720ull;   // smallest view traced in warp packets
+// A view's camera rays suit warp packets when there are at least PACKET_MIN_RAYS of them
+// and sqrt(PACKET_RAYS2) times the square root of the scene's triangles (of all
+// instances): the fewer rays for the triangles, the more often neighbouring rays end in
+// different parts of the scene, so that a packet visits every ray's nodes and the longest
+// packets end late; and a few packets leave SMs idle.  Frames of two segments, packets
+// and ray by ray: a room of 2,120 triangles (line at 55,000 rays) with 128x72 pixels
+// 157 and 141 us, 320x180 173 and 179, 640x360 244 and 265, 3840x2160 4273 and 4469;
+// spheres and a terrain tile of 387,000 (747,000 rays) 960x540 739 and 649 us, 720p 927
+// and 916, 1080p 1558 and 1654; 64 tiles of 8.6 million (3.5 million rays) 720p 2104 and
+// 1809 us, 1080p 3591 and 3491, 1440p 5715 and 5789, 3840x2160 11516 and 12266.  With
+// a line at 1280x720 for all scenes a 256x256 room frame of depth 4 took 303 us (296 now),
+// a 1080p terrain frame with the radiance cache 3.91 ms (3.67).  (Packets that hand their
+// tile over to the ray-by-ray kernel after 64 to 512 steps, or when few rays share
+// their nodes, lost to both: the second kernel's tail costs more than it saves.)
+constexpr uint64_t PACKET_MIN_RAYS = 1ull << 15;
+constexpr double PACKET_RAYS2 = 1200.0 * 1200.0;
 // camera-ray tile of one warp packet (16 x 2 and 4 x 8 tiles were slower at 1080p)
 constexpr uint32_t PACKET_TILE_W = 8, PACKET_TILE_H = 4;
+// counters (uint32) of one frame, zeroed at frame start
 constexpr uint32_t CNT_QUEUE = 0;         // [d]: rays queued for segment d
 constexpr uint32_t CNT_WORK_TRACE = 16;   // [d]: work fetch of the closest-hit pass of segment d
 constexpr uint32_t CNT_WORK_SHADOW = 32;  // [d]: work fetch of the shadow pass of segment d
@@ -78,9 +93,8 @@ struct FrameParams {
     // k_shade marks the queue entries whose path ends (bit 31 of the path id) and
     // k_accum_shadow writes those pixels' outputs; no resolve pass follows
     uint32_t early_resolve;
-    // every view's sides are multiples of the tile's and it has at least
-    // PACKET_MIN_PIXELS pixels (neighbouring pixels of smaller images are too far
-    // apart in the scene for a packet's rays to share their nodes), both trees have
+    // every view's sides are multiples of the tile's and its rays suit packets
+    // (PACKET_MIN_RAYS), both trees have
     // single-primitive leaves, the traversal bounds are the defaults (their limits
     // are per ray) and the frame does not count traversal work: the camera rays are
     // queued in PACKET_TILE_W x PACKET_TILE_H pixel tiles and traced in warp packets

@@ -157,43 +157,51 @@ SNK_HD V3 fresnel_schlick(float cos_theta, V3 f0) {
     float p = ((c * c) * (c * c)) * c;
     return v3(f0.x + (1.0f - f0.x) * p, f0.y + (1.0f - f0.y) * p, f0.z + (1.0f - f0.z) * p);
 }
-SNK_HD float distribution_ggx(V3 h, V3 n, float roughness) {
-    float a = roughness * roughness;
-    float a2 = a * a;
+SNK_HD float distribution_ggx(V3 h, V3 n, float a2) {
     float ndh = fmax_(dot(n, h), 0.0f);
     float ndh2 = ndh * ndh;
     float denom = ndh2 * (a2 - 1.0f) + 1.0f;
     denom = (PI * denom) * denom;
     return a2 / denom;
 }
-SNK_HD float geometry_schlick_ggx(float ndv, float roughness) {
-    float r = roughness + 1.0f;
-    float k = (r * r) / 8.0f;
-    return ndv / (ndv * (1.0f - k) + k);
+SNK_HD float ggx_a2(float roughness) {
+    float a = roughness * roughness;
+    return a * a;
 }
-SNK_HD float geometry_smith(V3 v, V3 l, V3 n, float roughness) {
-    float ndv = fmax_(dot(n, v), 0.0f);
-    float ndl = fmax_(dot(n, l), 0.0f);
-    return geometry_schlick_ggx(ndv, roughness) * geometry_schlick_ggx(ndl, roughness);
-}
+SNK_HD float geometry_schlick_ggx(float ndv, float k) { return ndv / (ndv * (1.0f - k) + k); }
 struct Terms { V3 kd, spec; float ndl; };
+// what a surface's BRDF terms share over the light directions
+struct Facing { float k, a2, g, ndv4, om; };
+SNK_HD Facing facing_of(V3 v, V3 n, float roughness, float metallic) {
+    Facing c;
+    float r = roughness + 1.0f;
+    c.k = (r * r) / 8.0f;
+    c.a2 = ggx_a2(roughness);
+    float ndv = fmax_(dot(n, v), 0.0f);
+    c.g = geometry_schlick_ggx(ndv, c.k);
+    c.ndv4 = 4.0f * ndv;
+    c.om = 1.0f - metallic;
+    return c;
+}
 // shared body of CookTorranceBRDF and CalcDirectionalLight for a unit light direction
-SNK_HD Terms brdf_terms(V3 l, V3 v, V3 f0, V3 n, float roughness, float metallic) {
+SNK_HD Terms brdf_terms(V3 l, V3 v, V3 f0, V3 n, const Facing& c) {
     V3 vl = add(v, l);
     float vl2 = dot(vl, vl);
     V3 h = vl2 > 0.0f ? divs(vl, sqrtf(vl2)) : n;
     V3 f = fresnel_schlick(fmax_(dot(h, v), 0.0f), f0);
-    float ndf = distribution_ggx(h, n, roughness);
-    float g = geometry_smith(v, l, n, roughness);
+    float ndf = distribution_ggx(h, n, c.a2);
     float ndl = fmax_(dot(n, l), 0.0f);
+    float g = c.g * geometry_schlick_ggx(ndl, c.k);
     float ng = ndf * g;
-    float denom = ((4.0f * fmax_(dot(n, v), 0.0f)) * ndl) + 0.0001f;
+    float denom = (c.ndv4 * ndl) + 0.0001f;
     Terms t;
     t.spec = v3((ng * f.x) / denom, (ng * f.y) / denom, (ng * f.z) / denom);
-    float om = 1.0f - metallic;
-    t.kd = v3((1.0f - f.x) * om, (1.0f - f.y) * om, (1.0f - f.z) * om);
+    t.kd = v3((1.0f - f.x) * c.om, (1.0f - f.y) * c.om, (1.0f - f.z) * c.om);
     t.ndl = ndl;
     return t;
+}
+SNK_HD Terms brdf_terms(V3 l, V3 v, V3 f0, V3 n, float roughness, float metallic) {
+    return brdf_terms(l, v, f0, n, facing_of(v, n, roughness, metallic));
 }
 SNK_HD V3 cook_torrance(const Terms& t) {
     return v3((t.kd.x / PI + t.spec.x) * t.ndl, (t.kd.y / PI + t.spec.y) * t.ndl, (t.kd.z / PI + t.spec.z) * t.ndl);

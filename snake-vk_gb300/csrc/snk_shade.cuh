@@ -235,7 +235,7 @@ __device__ __forceinline__ bool sample_continuation(const Surface& s, V3 v, V3 f
     V3 vl = add(v, l);
     float vl2 = dot(vl, vl);
     V3 hh = vl2 > 0.0f ? divs(vl, sqrtf(vl2)) : s.n;
-    float D = distribution_ggx(hh, s.n, s.roughness);
+    float D = distribution_ggx(hh, s.n, ggx_a2(s.roughness));
     float pdf_spec = (D * fmax_(dot(s.n, hh), 0.0f)) / (4.0f * fmax_(dot(v, hh), 1e-6f));
     float pdf = p_spec * pdf_spec + (1.0f - p_spec) * (ndl / PI);
     if (!(pdf > 0.0f)) return false;

@@ -986,14 +986,13 @@ struct SmallSmem {
     int2 children[SMALL_BUILD_MAX];
     float4 node_lo[2 * SMALL_BUILD_MAX], node_hi[2 * SMALL_BUILD_MAX];
     uint32_t leaf_count[2 * SMALL_BUILD_MAX];
-    uint2 tasks[2][SMALL_BUILD_MAX];
+    uint32_t tasks[2 * SMALL_BUILD_MAX];       // clustering: nearest neighbours; collapse: wide node l's binary node
     int parent[2 * SMALL_BUILD_MAX];           // treelet passes
     int flags[SMALL_BUILD_MAX];
     float cost[2 * SMALL_BUILD_MAX];
     uint32_t warp_sums[32];
     uint32_t counters[8];
     unsigned cb[6];
-    double sah;
     union {
         TreeletSmem tl[SMALL_THREADS / 32];    // treelet passes
         struct {                               // then the least-SAH collapse table
@@ -1042,26 +1041,34 @@ __device__ __forceinline__ unsigned order_f(float f) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-// One output node by a whole warp (every lane passes the same task: binary node, wide
-// node slot).  counters: [2] wide nodes, [3] primitive slots, [4] capacity error bits;
-// next_tasks counts the child tasks queued in tasks_out.  cap: primitives of the
-// build, cap_nodes: wide nodes it may write; internal binary nodes have ids below nl.
-// inv_root > 0: returns (lane 0) the node's part of the SAH cost, its children's areas
-// times inv_root, one traversal step per internal child and one test per primitive.
+// Wide node `local` of the build, made of binary node b, by a whole warp (every lane
+// passes the same).  counters: [2] wide nodes, [3] primitive slots, [4] capacity error
+// bits.  Its internal children are nodes local' whose binary nodes go to tasks[local'];
+// next_level (may be null) counts them.  cap: primitives of the build, cap_nodes: wide
+// nodes it may write; internal binary nodes have ids below nl.  root_lo, root_hi (not
+// null): returns (lane 0) the node's part of the SAH cost, its children's areas over the
+// root's, one traversal step per internal child and one test per primitive.
+// A level of the collapse is as long as one node's chain of loads: counts and leaf
+// primitives are fetched with the boxes, the root's box before it is needed, the task
+// before the level's size is known, and a child's task is found by its node's number
+// (five rounds of loads and an atomic fewer in the chain: loading a 131,072-triangle
+// terrain 1.678 -> 1.662 ms).  One launch whose warps wait for their node's parent instead
+// of a launch per level was no faster (1.676 ms; 4,297 instances 264 -> 288 us).
 // Lane k < nc holds candidate child k while the node is opened; the 64 (child,
 // slot) pairs p = 8k + s of the slot assignment are spread two per lane; lane s
 // < 8 then builds slot s.  Ties go to the lowest child / pair index, as in the
 // sequential loops.  stage: this warp's 80-byte staging node in shared memory.
-__device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* next_tasks, uint2* tasks_out,
+__device__ double collapse_task_warp(int b, uint32_t local, uint32_t* counters, uint32_t* next_level, uint32_t* tasks,
                                      uint32_t cap, uint32_t cap_nodes, int nl, const int2* children,
                                      const float4* node_lo, const float4* node_hi, const uint32_t* leaf_count,
                                      const uint32_t* sorted, WideNode* nodes, WideNode* stage, uint32_t node_base,
                                      uint32_t prim_base, uint32_t* prim_order, uint32_t leaf_max, uint32_t leaf_pack,
-                                     const uint32_t* wide_split, float inv_root) {
+                                     const uint32_t* wide_split, const float4* root_lo, const float4* root_hi) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
-    const int b = (int)task.x;
-    const uint32_t w = task.y;
+    const uint32_t w = node_base + local;
+    float4 rlo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), rhi = rlo;
+    if (root_lo) { rlo = *root_lo; rhi = *root_hi; }
     int c = -1, nc;
     if (b >= nl) {
         nc = 1;
@@ -1093,7 +1100,15 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
     // parent box (min / max are exact, so the reduction order does not matter)
     float4 lo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), hi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
     float4 clo = lo, chi = hi;
-    if (lane < nc) { clo = node_lo[c]; chi = node_hi[c]; lo = clo; hi = chi; }
+    uint32_t c_count = 0, c_prim = 0;
+    if (lane < nc) {
+        clo = node_lo[c];
+        chi = node_hi[c];
+        c_count = leaf_count[c];
+        if (c >= nl) c_prim = sorted[c - nl];
+        lo = clo;
+        hi = chi;
+    }
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) {
         lo.x = fminf(lo.x, __shfl_xor_sync(FULL, lo.x, o)); lo.y = fminf(lo.y, __shfl_xor_sync(FULL, lo.y, o));
@@ -1115,7 +1130,7 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
         sc[1] = ((s_ & 1) ? x1 : -x1) + ((s_ & 2) ? y1 : -y1) + ((s_ & 4) ? z1 : -z1);
     }
     uint32_t used_c = 0, used_s = 0;
-    int slot_c = -1;   // lane s < 8: the child in slot s
+    int slot_k = -1;   // lane s < 8: the child in slot s
     for (int it = 0; it < nc; it++) {
         const bool v0 = k0 < nc && !((used_c >> k0) & 1u) && !((used_s >> s_) & 1u);
         const bool v1 = k1 < nc && !((used_c >> k1) & 1u) && !((used_s >> s_) & 1u);
@@ -1128,13 +1143,15 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
         const int bk = (int)(pm >> 3), bs = (int)(pm & 7u);
         used_c |= 1u << bk;
         used_s |= 1u << bs;
-        const int cb = __shfl_sync(FULL, c, bk);
-        if (lane == bs) slot_c = cb;
+        if (lane == bs) slot_k = bk;
     }
+    const int from = slot_k < 0 ? 0 : slot_k;
+    const int slot_c = __shfl_sync(FULL, c, from);
+    const uint32_t slot_count = __shfl_sync(FULL, c_count, from), slot_prim = __shfl_sync(FULL, c_prim, from);
     // classify and allocate
-    const bool mine = lane < 8 && slot_c >= 0;
-    const bool is_int = mine && slot_c < nl && leaf_count[slot_c] > leaf_pack;
-    const uint32_t cnt = (mine && !is_int) ? leaf_count[slot_c] : 0u;
+    const bool mine = lane < 8 && slot_k >= 0;
+    const bool is_int = mine && slot_c < nl && slot_count > leaf_pack;
+    const uint32_t cnt = (mine && !is_int) ? slot_count : 0u;
     const unsigned int_mask = __ballot_sync(FULL, is_int);
     const uint32_t n_int = (uint32_t)__popc(int_mask);
     uint32_t off = cnt;   // inclusive scan of the leaf counts over the slots, then exclusive
@@ -1145,7 +1162,7 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
     }
     const uint32_t n_prims = __shfl_sync(FULL, off, 7);
     off -= cnt;
-    uint32_t child_local = 0, prim_local = 0, task_base = 0;
+    uint32_t child_local = 0, prim_local = 0;
     if (lane == 0) {
         child_local = n_int ? atomicAdd(&counters[2], n_int) : 0u;
         prim_local = n_prims ? atomicAdd(&counters[3], n_prims) : 0u;
@@ -1153,13 +1170,12 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
     child_local = __shfl_sync(FULL, child_local, 0);
     prim_local = __shfl_sync(FULL, prim_local, 0);
     // capacity checks (never exceeded by a correct tree; a violation is recorded,
-    // the node is not written and no child task is queued)
-    if (child_local + n_int > cap_nodes || prim_local + n_prims > cap || w - node_base >= cap_nodes) {
+    // the node is not written and none of its children is made)
+    if (child_local + n_int > cap_nodes || prim_local + n_prims > cap || local >= cap_nodes) {
         if (lane == 0) atomicOr(&counters[4], 1u);
         return 0.0;
     }
-    if (lane == 0 && n_int) task_base = atomicAdd(next_tasks, n_int);
-    task_base = __shfl_sync(FULL, task_base, 0);
+    if (next_level && lane == 0 && n_int) atomicAdd(next_level, n_int);
     const QuantFrame F = quant_frame(plo, phi);
     if (lane == 0) {
         stage->px = F.p[0]; stage->py = F.p[1]; stage->pz = F.p[2];
@@ -1170,7 +1186,7 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
     }
     if (lane < 8) {
         const int s = lane;
-        if (slot_c < 0) {
+        if (!mine) {
             stage->meta[s] = 0;
             for (int a = 0; a < 3; a++) { stage->qlo[a][s] = 0; stage->qhi[a][s] = 0; }
         } else {
@@ -1178,9 +1194,10 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
             if (is_int) {
                 const uint32_t rank = (uint32_t)__popc(int_mask & ((1u << s) - 1u));
                 stage->meta[s] = (uint8_t)META_INTERNAL;
-                const uint32_t slot_out = task_base + rank;
-                if (slot_out < cap) tasks_out[slot_out] = make_uint2((uint32_t)slot_c, node_base + child_local + rank);
-                else atomicOr(&counters[4], 2u);
+                tasks[child_local + rank] = (uint32_t)slot_c;
+            } else if (slot_c >= nl) {
+                stage->meta[s] = (uint8_t)((1u << 5) | off);
+                prim_order[prim_local + off] = slot_prim;
             } else {
                 stage->meta[s] = (uint8_t)((cnt << 5) | off);
                 // the (<= leaf_pack) leaves of subtree slot_c, in order
@@ -1208,7 +1225,8 @@ __device__ double collapse_task_warp(uint2 task, uint32_t* counters, uint32_t* n
     if (lane < 5) reinterpret_cast<uint4*>(nodes + w)[lane] = reinterpret_cast<const uint4*>(stage)[lane];
     __syncwarp();
     double sah = 0.0;
-    if (inv_root > 0.0f) {
+    if (root_lo) {
+        const float area = half_area(rlo, rhi), inv_root = area > 0.0f ? 1.0f / area : 1.0f;
         if (mine) sah = (double)(half_area(node_lo[slot_c], node_hi[slot_c]) * inv_root) * (is_int ? 1.0 : (double)cnt);
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) sah += __shfl_xor_sync(FULL, sah, o);
@@ -1308,7 +1326,7 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
                 const uint32_t on = __shfl_xor_sync(0xFFFFFFFFu, nn, o);
                 if (ob < best || (ob == best && on < nn)) { best = ob; nn = on; }
             }
-            if (sub == 0 && g < (int)m) S.tasks[0][g].x = nn;   // scratch: nearest neighbour per position
+            if (sub == 0 && g < (int)m) S.tasks[g] = nn;   // scratch: nearest neighbour per position
         }
         __syncthreads();
         const int i = tid;
@@ -1318,11 +1336,11 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
             const int ci = S.clusters[cur][i];
             mylo = S.node_lo[ci];
             myhi = S.node_hi[ci];
-            nn = (int)S.tasks[0][i].x;
+            nn = (int)S.tasks[i];
         }
         bool merge = false, keep = false;
         if (i < (int)m) {
-            const bool mutual = nn >= 0 && (int)S.tasks[0][nn].x == i;
+            const bool mutual = nn >= 0 && (int)S.tasks[nn] == i;
             merge = mutual && i < nn;
             keep = !mutual || i < nn;
         }
@@ -1456,33 +1474,32 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
     float rha = half_area(rlo, rhi);
     if (!(rha > 0.0f)) rha = 1.0f;
     if (tid == 0) {
-        S.tasks[0][0] = make_uint2(0u, node_base);
-        S.counters[0] = 1u; S.counters[1] = 0u; S.counters[2] = 1u; S.counters[3] = 0u; S.counters[4] = 0u;
-        S.sah = 0.0;
+        S.tasks[0] = 0u;
+        S.counters[2] = 1u; S.counters[3] = 0u; S.counters[4] = 0u;
     }
     __syncthreads();
-    int cc = 0, level = 0;
+    // (a level's nodes are the ones that the level above has allocated: a run of numbers)
+    uint32_t begin = 0, end = 1;
+    int level = 0;
     for (; level < 4096; level++) {
-        const uint32_t nin = min(S.counters[0], (uint32_t)n);   // the task arrays hold n entries
-        if (nin == 0 || S.counters[4] != 0u) break;               // done, or a capacity error
+        if (begin == end || S.counters[4] != 0u) break;   // done, or a capacity error
         // one warp per wide node (no SAH statistic: the per-frame build skips it)
-        for (uint32_t t = (uint32_t)(tid >> 5); t < nin; t += (uint32_t)(nt >> 5)) {
-            const uint2 task = S.tasks[cc][t];
+        for (uint32_t local = begin + (uint32_t)(tid >> 5); local < end; local += (uint32_t)(nt >> 5)) {
+            const int b = (int)S.tasks[local];
             // refit data: exact box and depth of every wide node
-            const uint32_t local = task.y - node_base;
-            if ((tid & 31) == 0 && local <= (uint32_t)n) {
-                wide_box[2 * local] = S.node_lo[task.x];
-                wide_box[2 * local + 1] = S.node_hi[task.x];
+            if ((tid & 31) == 0) {
+                wide_box[2 * local] = S.node_lo[b];
+                wide_box[2 * local + 1] = S.node_hi[b];
                 wide_depth[local] = (uint32_t)level;
             }
-            collapse_task_warp(task, S.counters, &S.counters[1], S.tasks[cc ^ 1], (uint32_t)n, (uint32_t)n + 1u, nl,
-                               S.children, S.node_lo, S.node_hi, S.leaf_count, S.vals, nodes, &S.stage[tid >> 5],
-                               node_base, prim_base, prim_order, leaf_max, leaf_max, dp ? S.dp.wide_split : nullptr,
-                               0.0f);
+            collapse_task_warp(b, local, S.counters, nullptr, S.tasks, (uint32_t)n, (uint32_t)n + 1u, nl, S.children,
+                               S.node_lo, S.node_hi, S.leaf_count, S.vals, nodes, &S.stage[tid >> 5], node_base,
+                               prim_base, prim_order, leaf_max, leaf_max, dp ? S.dp.wide_split : nullptr, nullptr,
+                               nullptr);
         }
         __syncthreads();
-        if (tid == 0) { S.counters[0] = S.counters[1]; S.counters[1] = 0u; }
-        cc ^= 1;
+        begin = end;
+        end = min(S.counters[2], (uint32_t)n + 1u);
         __syncthreads();
     }
     if (tid == 0) {
@@ -1501,9 +1518,9 @@ k_build_small(const float4* __restrict__ plo, const float4* __restrict__ phi, in
 }
 
 // ---- collapse without host round trips -----------------------------------------
-// level_tasks[l] counts the tasks of wide level l (tasks of even levels in
-// tasks_a, odd levels in tasks_b); counters: [2] wide nodes, [3] primitive
-// slots, [4] capacity error bits.  A few launches of k_collapse_level take the
+// level_tasks[l] counts the wide nodes of level l, whose numbers follow those of the
+// level above; tasks[number] is the binary node one is made of.  counters: [2] wide
+// nodes, [3] primitive slots, [4] capacity error bits.  A few launches of k_collapse_level take the
 // usual depths with every SM; k_collapse_finish takes whatever is left in one
 // block, so no level count has to come back to the host.
 constexpr int COLLAPSE_MAX_LEVELS = 128;
@@ -1513,8 +1530,7 @@ constexpr int LEVEL_WARPS = 8;
 // what the collapse reads and writes
 struct CollapseArgs {
     BuildTrees B;
-    uint2 *tasks_a, *tasks_b;
-    uint32_t *level_tasks, *counters;
+    uint32_t *tasks, *level_tasks, *counters;
     const int2* children;
     const float4 *node_lo, *node_hi;
     const uint32_t *leaf_count, *sorted, *wide_split;
@@ -1533,7 +1549,7 @@ __global__ void k_collapse_init(CollapseArgs A) {
     if (t < A.B.count) {
         const uint32_t first = tree_begin(A.B, t);
         const bool single = tree_end(A.B, t) - first == 1u;
-        A.tasks_a[t] = make_uint2(single ? A.B.total + first : first, A.node_base + t);
+        A.tasks[t] = single ? A.B.total + first : first;
     }
     if (t == 0u) {
         A.counters[2] = A.B.count;
@@ -1543,34 +1559,30 @@ __global__ void k_collapse_init(CollapseArgs A) {
     }
 }
 
-// One level's tasks t0, t0 + step, ... of this warp; returns their part of the SAH sum.
-__device__ __forceinline__ double collapse_level(const CollapseArgs& A, int level, uint32_t t0, uint32_t step,
-                                                 WideNode* stage) {
+// Nodes begin + t0, begin + t0 + step, ... of the `count` of a level by this warp; returns
+// their part of the SAH sum.  first_task: tasks[begin + t0], when that is in the array.
+__device__ __forceinline__ double collapse_level(const CollapseArgs& A, int level, uint32_t begin, uint32_t count,
+                                                 uint32_t t0, uint32_t step, uint32_t first_task, WideNode* stage) {
     const int lane = threadIdx.x & 31;
-    const uint32_t n = A.B.total;
-    if (A.counters[4] != 0u) return 0.0;                 // (a capacity error: nothing more is written)
-    const uint32_t nin = min(A.level_tasks[level], n);   // the task arrays hold n entries
-    const uint2* tin = (level & 1) ? A.tasks_b : A.tasks_a;
-    uint2* tout = (level & 1) ? A.tasks_a : A.tasks_b;
+    const uint32_t n = A.B.total, cap_nodes = n + A.B.count;
     double sum = 0.0;
-    for (uint32_t t = t0; t < nin; t += step) {
-        const uint2 task = tin[t];
-        const uint32_t local = task.y - A.node_base;
-        if (A.wide_depth && lane == 0 && local <= n) A.wide_depth[local] = (uint32_t)level;   // (for a later refit)
-        float inv_root = 0.0f;
-        uint32_t prims = 0;
+    for (uint32_t t = t0; t < count; t += step) {
+        const uint32_t local = begin + t;
+        if (local >= cap_nodes) break;   // (the task array holds cap_nodes entries)
+        const uint32_t b = t == t0 ? first_task : A.tasks[local];
+        if (A.wide_depth && lane == 0) A.wide_depth[local] = (uint32_t)level;   // (for a later refit)
+        uint32_t prims = 0, root = 0;
         if (A.sah) {
-            const uint32_t tree = tree_of(A.B, task.x >= n ? task.x - n : task.x);
+            const uint32_t tree = tree_of(A.B, b >= n ? b - n : b);
             const uint32_t first = tree_begin(A.B, tree);
             prims = tree_end(A.B, tree) - first;
-            const uint32_t root = prims == 1u ? n + first : first;
-            const float area = half_area(A.node_lo[root], A.node_hi[root]);
-            inv_root = area > 0.0f ? 1.0f / area : 1.0f;
+            root = prims == 1u ? n + first : first;
         }
-        const double s = collapse_task_warp(task, A.counters, &A.level_tasks[level + 1], tout, n, n + A.B.count, (int)n,
-                                            A.children, A.node_lo, A.node_hi, A.leaf_count, A.sorted, A.nodes, stage,
-                                            A.node_base, A.prim_base, A.prim_order, A.leaf_max, A.leaf_pack,
-                                            A.wide_split, inv_root);
+        const double s = collapse_task_warp((int)b, local, A.counters, &A.level_tasks[level + 1], A.tasks, n, cap_nodes,
+                                            (int)n, A.children, A.node_lo, A.node_hi, A.leaf_count, A.sorted, A.nodes,
+                                            stage, A.node_base, A.prim_base, A.prim_order, A.leaf_max, A.leaf_pack,
+                                            A.wide_split, A.sah ? A.node_lo + root : nullptr,
+                                            A.sah ? A.node_hi + root : nullptr);
         sum += s * (double)prims;
     }
     return sum;
@@ -1591,9 +1603,16 @@ __device__ __forceinline__ void block_add(double sum, double* warp_sums, double*
 __global__ void __launch_bounds__(32 * LEVEL_WARPS) k_collapse_level(CollapseArgs A, int level) {
     __shared__ WideNode stage[LEVEL_WARPS];
     __shared__ double warp_sums[LEVEL_WARPS];
-    const uint32_t w = threadIdx.x >> 5;
-    if (blockIdx.x * LEVEL_WARPS >= A.level_tasks[level]) return;   // (this level's count is final)
-    const double sum = collapse_level(A, level, blockIdx.x * LEVEL_WARPS + w, gridDim.x * LEVEL_WARPS, &stage[w]);
+    const uint32_t w = threadIdx.x >> 5, t0 = blockIdx.x * LEVEL_WARPS + w;
+    uint32_t begin = 0;
+#pragma unroll
+    for (int l = 0; l < COLLAPSE_FAST_LEVELS; l++) begin += l < level ? A.level_tasks[l] : 0u;
+    uint32_t count = A.level_tasks[level];   // (final)
+    const uint32_t bad = A.counters[4];
+    if (blockIdx.x * LEVEL_WARPS >= count) return;
+    if (bad != 0u) count = 0;                // (a capacity error: nothing more is written)
+    const uint32_t task = begin + t0 < A.B.total + A.B.count ? A.tasks[begin + t0] : 0u;
+    const double sum = collapse_level(A, level, begin, count, t0, gridDim.x * LEVEL_WARPS, task, &stage[w]);
     if (A.sah) block_add(sum, warp_sums, A.sah);
 }
 
@@ -1601,15 +1620,20 @@ __global__ void __launch_bounds__(1024) k_collapse_finish(CollapseArgs A, int fi
                                                           SmallBuildOut* out) {
     __shared__ WideNode stage[32];
     __shared__ double warp_sums[32];
-    __shared__ int stop;
+    __shared__ uint32_t size;
     const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    uint32_t begin = 0;
+    for (int l = 0; l < first_level; l++) begin += A.level_tasks[l];
     int level = first_level;
     double sum = 0.0;
     for (; level < COLLAPSE_MAX_LEVELS; level++) {
-        if (threadIdx.x == 0) stop = A.level_tasks[level] == 0u || A.counters[4] != 0u;
+        if (threadIdx.x == 0) size = A.counters[4] != 0u ? 0u : A.level_tasks[level];
         __syncthreads();
-        if (stop) break;
-        sum += collapse_level(A, level, w, nw, &stage[w]);
+        const uint32_t count = size;
+        if (count == 0u) break;
+        const uint32_t task = begin + w < A.B.total + A.B.count ? A.tasks[begin + w] : 0u;
+        sum += collapse_level(A, level, begin, count, w, nw, task, &stage[w]);
+        begin += count;
         __syncthreads();   // this level's child tasks and their count are complete
     }
     if (A.sah) block_add(sum, warp_sums, A.sah);
@@ -1940,8 +1964,7 @@ Status build_wide_bvhs(BuildScratch& sc, const float4* prim_lo, const float4* pr
     SNK_TRY_CUDA(sc.node_hi.reserve(2 * (size_t)n));
     SNK_TRY_CUDA(sc.leaf_count.reserve(2 * (size_t)n));
     SNK_TRY_CUDA(sc.cost.reserve(2 * (size_t)n));
-    SNK_TRY_CUDA(sc.tasks_a.reserve(n));
-    SNK_TRY_CUDA(sc.tasks_b.reserve(n));
+    SNK_TRY_CUDA(sc.tasks.reserve((size_t)n + B.count));
     SNK_TRY_CUDA(sc.counters.reserve(5));
     SNK_TRY_CUDA(sc.cbounds.reserve(6 * (size_t)B.count));
     SNK_TRY_CUDA(sc.sah.reserve(1));
@@ -1989,7 +2012,7 @@ Status build_wide_bvhs(BuildScratch& sc, const float4* prim_lo, const float4* pr
     SNK_TRY_CUDA(cudaGetLastError());
     CollapseArgs A;
     A.B = B;
-    A.tasks_a = sc.tasks_a.p; A.tasks_b = sc.tasks_b.p;
+    A.tasks = sc.tasks.p;
     A.level_tasks = sc.level_tasks.p; A.counters = sc.counters.p;
     A.children = sc.children.p; A.node_lo = sc.node_lo.p; A.node_hi = sc.node_hi.p;
     A.leaf_count = sc.leaf_count.p; A.sorted = sorted; A.wide_split = wide_split;

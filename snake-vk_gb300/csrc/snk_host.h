@@ -72,7 +72,7 @@ struct BuildScratch {
     DBuf<float4> node_lo, node_hi;
     DBuf<uint32_t> leaf_count;
     DBuf<float> cost;             // binary-tree SAH cost per node (treelet restructuring)
-    DBuf<uint2> tasks_a, tasks_b;
+    DBuf<uint32_t> tasks;         // per wide node: the binary node it is made of
     DBuf<uint32_t> counters;      // [2] wide nodes, [3] prims, [4] error bits
     DBuf<unsigned> cbounds;       // centroid bounds per tree, order-preserving encoded
     DBuf<uint32_t> sort_hist;     // per-tile digit counts of the radix sort, every digit

@@ -80,9 +80,8 @@ __global__ void __launch_bounds__(BLK) k_generate(FrameParams F) {
         F.rays[0][2ull * q] = make_float4(V.v.pos[0], V.v.pos[1], V.v.pos[2], 0.0f);
         F.rays[0][2ull * q + 1] = make_float4(d.x, d.y, d.z, T_FAR);
         F.path_ids[0][q] = p;
-        F.beta[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-        F.L[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (F.cache) F.spread[p] = make_float2(0.0f, 0.0f);
+        // (throughput and radiance start at 1 and 0 in segment 0's shading and shadow pass)
+        if (F.indirect) F.L[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
 
@@ -166,7 +165,7 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
             head = (head + take) & 63u;
             cnt -= take;
             __syncwarp();
-            bool cont = false, sv0 = false, sv1 = false, query = false;
+            bool cont = false, sv0 = false, sv1 = false, query = false, emits = false;
             uint32_t p = 0;
             float4 nr0 = make_float4(0, 0, 0, 0), nr1 = make_float4(0, 0, 0, 0);
             // shadow rays: their origin and the local-light ray's direction + tmax (the
@@ -198,14 +197,14 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
                     float u_sel = pcg_float(rng), u1 = pcg_float(rng), u2 = pcg_float(rng);
                     float u_rr = pcg_float(rng), u_d1 = pcg_float(rng), u_d2 = pcg_float(rng);
                     float u_lobe = pcg_float(rng);
-                    float4 b4 = F.beta[p];
+                    const float4 b4 = FIRST ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : F.beta[p];
                     V3 beta = v3(b4.x, b4.y, b4.z);
                     bool to_cache = false;
                     if (CACHE) {
                         // path spread (Mueller et al. 2021): a0 = t^2 / (4 pi cos) at the primary
                         // vertex; later vertices add sqrt(t^2 / (pdf cos)); the path is handed
                         // to the cache once spread^2 > c a0
-                        float2 sp = F.spread[p];
+                        float2 sp = FIRST ? make_float2(0.0f, 0.0f) : F.spread[p];
                         const float cosv = fmax_(fabsf(dot(sf.n, rd)), 1e-6f);
                         if (FIRST) sp = make_float2((h.t * h.t) / ((4.0f * PI) * cosv), 0.0f);
                         else sp.y = sp.y + sqrtf((h.t * h.t) / (fmax_(b4.w, 1e-6f) * cosv));
@@ -229,10 +228,10 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
                         qb = make_float4(beta.x, beta.y, beta.z, 0.0f);
                         query = true;
                     } else if (sf.flags & MAT_EMISSIVE) {
-                        if (FIRST && direct) {
-                            float4 l4 = F.L[p];
-                            V3 Lp = add(v3(l4.x, l4.y, l4.z), cmul(beta, sf.albedo));
-                            F.L[p] = make_float4(Lp.x, Lp.y, Lp.z, 0.0f);
+                        if (FIRST && direct && !train) {   // as a visible contribution (a training path's is not used)
+                            const V3 c = cmul(beta, sf.albedo);
+                            F.shadow_contrib[shadow_entry(F, i, 0)] = make_float4(c.x, c.y, c.z, 1.0f);
+                            emits = true;
                         }
                     } else {
                         V3 v = neg(rd);
@@ -279,7 +278,7 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
             }
             if (have) {   // zero contribution: no shadow ray of that kind
                 const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (!sv0) F.shadow_contrib[shadow_entry(F, i, 0)] = z;
+                if (!sv0 && !emits) F.shadow_contrib[shadow_entry(F, i, 0)] = z;
                 if (!sv1) F.shadow_contrib[shadow_entry(F, i, 1)] = z;
             }
             // warp-ballot compaction of the continuing paths into the next queue and of

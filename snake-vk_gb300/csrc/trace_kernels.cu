@@ -286,7 +286,11 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_shadow(const __grid_consta
     flush_counts<COUNT>(ctr, F.trav_counters ? F.trav_counters + 2 : nullptr);
 }
 
-// adds the visible shadow-ray contributions of segment d to the path radiance
+// adds the visible shadow-ray contributions of segment d to the path radiance, which
+// segment 0's (of every path) start; an emitter met by a camera ray is such a contribution.
+// (The generation wrote a throughput of 1 and a radiance of 0 for every path and the
+// first shading and shadow passes read them back, 64 bytes a path: a 1080p frame of
+// the sphere field 1.921 ms, 1.899 so.)
 __global__ void __launch_bounds__(256) k_accum_shadow(FrameParams F, uint32_t d) {
     const uint32_t n = F.counters[CNT_QUEUE + d];
     const uint32_t* pids = F.path_ids[d & 1u];
@@ -300,11 +304,11 @@ __global__ void __launch_bounds__(256) k_accum_shadow(FrameParams F, uint32_t d)
             p = raw & 0x7FFFFFFFu;
             fin = (raw >> 31) != 0u;
         } else {
-            if (!add) continue;
+            if (!add && d) continue;
             p = pids[i];
         }
-        if (!add && !fin) continue;
-        float4 l = F.L[p];
+        if (!add && !fin && d) continue;
+        float4 l = d ? F.L[p] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (c0.w != 0.0f) l = make_float4(l.x + c0.x, l.y + c0.y, l.z + c0.z, 0.0f);
         if (c1.w != 0.0f) l = make_float4(l.x + c1.x, l.y + c1.y, l.z + c1.z, 0.0f);
         if (fin) {   // the pixel's outputs, as the resolve pass writes them for one sample

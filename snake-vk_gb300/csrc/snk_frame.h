@@ -33,7 +33,7 @@ constexpr uint32_t CNT_WORK_TRACE = 16;   // [d]: work fetch of the closest-hit 
 constexpr uint32_t CNT_WORK_SHADOW = 32;  // [d]: work fetch of the shadow pass of segment d
 constexpr uint32_t CNT_SHADOW_RAYS = 48;  // valid shadow rays
 constexpr uint32_t CNT_CACHE_QUERIES = 49; // paths terminated into the radiance cache
-constexpr uint32_t CNT_SHADOW_REUSED = 50;  // ReSTIR visibility tests answered by an identical earlier test
+constexpr uint32_t CNT_SHADOW_REUSED = 50;  // ReSTIR visibility tests not traced (answered by an identical earlier one, or of no effect)
 constexpr uint32_t CNT_SHADOW_Q = 64;     // [2d + k]: shadow rays of light kind k queued by segment d
 constexpr uint32_t CNT_TOTAL = 96;
 constexpr uint32_t TRAIN_V = 4;           // recorded vertices per cache training path

@@ -154,14 +154,18 @@ __device__ __forceinline__ float memo_answer(Ctx& c, uint32_t code) {
 }
 
 // shadow test toward point light idx at its full distance (minus == false) or at
-// distance - 0.001, reusing an identical earlier test of this pixel
+// distance - 0.001, reusing an identical earlier test of this pixel.  The shorter
+// segment is part of the longer one: it is free when that is known to be, and the longer
+// one is blocked when the shorter one is known to be (1.0 M of 12.3 M rays of a 1080p
+// frame; two frames 15.64 -> 15.14 ms).  Known are the results of earlier
+// launches, the same in a recording and in its replay.
 __device__ __forceinline__ float shadow_test_pl(Ctx& c, uint32_t idx, bool minus, V3 o, V3 d, float tmax) {
     Memo* m = c.m;
     if (m) {
         if (!minus && m->pla_idx == idx) return memo_answer(c, m->pla_code);
-        if (minus)
-            for (uint32_t j = 0; j < m->n_pl; j++)
-                if (m->pl_idx[j] == idx) return memo_answer(c, m->pl_code[j]);
+        for (uint32_t j = 0; j < m->n_pl; j++)
+            if (m->pl_idx[j] == idx && (minus || m->pl_code[j] == MEMO_KNOWN)) return memo_answer(c, m->pl_code[j]);
+        if (minus && m->pla_idx == idx && m->pla_code == (MEMO_KNOWN | 1u)) return memo_answer(c, m->pla_code);
     }
     const uint32_t k = c.k;
     const float r = shadow_test(c, o, d, tmax);
@@ -383,7 +387,8 @@ struct ComboSlots {
     bool fill, use;
 };
 
-// FIXED: nb is the same in the recording and in the replaying run.  A sample whose weight
+// FIXED: nb is the same in the recording and in the replaying run; else it is the pass's
+// own sample, whose light this pass has tested at its full distance.  A sample whose weight
 // is 0 with the light visible (its reservoir's weight is 0: it was found occluded, or its
 // radiance here is) has weight 0 without it too and is never taken: no test is made
 // (two 1080p frames, the first without history, 16.33 -> 15.66 ms).
@@ -403,6 +408,9 @@ __device__ __forceinline__ void combine(Ctx& c, Reservoir& cur, const Reservoir&
         float vis = 0.0f;
         if (FIXED && (len * (float)nb.pl_m) * nb.w_pl == 0.0f) {
             skip_test(c);
+        } else if (!FIXED && len * (float)nb.pl_m <= 3.0e38f) {
+            // nb's weight is 0 unless its light is free at the full distance, as it then is at the shorter one
+            vis = shadow_test_pl(c, nb.pl_idx, false, none, none, 0.0f);
         } else if (use) {
             vis = shadow_test_pl(c, nb.pl_idx, true, none, none, 0.0f);
         } else {

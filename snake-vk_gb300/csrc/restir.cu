@@ -86,6 +86,7 @@ __device__ __forceinline__ void res_store(void* base, uint32_t i, const Reservoi
 // queue being recorded.
 constexpr uint32_t MEMO_KNOWN = 0x100;  // answer code: MEMO_KNOWN | visibility, else a slot of the current queue
 constexpr uint32_t MEMO_NONE = 0xFFFF;  // plan code of a test that was not made
+constexpr float PL_SHORTER = 0.001f;    // a combine tests a point light at its distance - PL_SHORTER
 constexpr int MEMO_PL = 4, MEMO_EM = 4;
 // Tests already made for this pixel and frame, by what they aim at: the point
 // light tested at its full distance, point lights tested at distance - 0.001,
@@ -133,12 +134,12 @@ __device__ __forceinline__ void ctx_close(Ctx& c) {
 
 // 1 when the segment is unoccluded (recording: always 1, the value is not used
 // for anything the replay would see differently)
-__device__ __forceinline__ float shadow_test(Ctx& c, V3 o, V3 d, float tmax) {
+__device__ __forceinline__ float shadow_test(Ctx& c, V3 o, V3 d, float tmax, float tmin = SHADOW_TMIN) {
     if (c.k >= c.cap) { c.overflow = true; return 0.0f; }
     const size_t slot = c.base + (size_t)c.k++ * c.stride;
     if (c.rays) {
         c.shadow_rays++;
-        c.rays[2 * slot] = make_float4(o.x, o.y, o.z, SHADOW_TMIN);
+        c.rays[2 * slot] = make_float4(o.x, o.y, o.z, tmin);
         c.rays[2 * slot + 1] = make_float4(d.x, d.y, d.z, tmax);
         return 1.0f;
     }
@@ -158,17 +159,23 @@ __device__ __forceinline__ float memo_answer(Ctx& c, uint32_t code) {
 // segment is part of the longer one: it is free when that is known to be, and the longer
 // one is blocked when the shorter one is known to be (1.0 M of 12.3 M rays of a 1080p
 // frame; two frames 15.64 -> 15.14 ms).  Known are the results of earlier
-// launches, the same in a recording and in its replay.
+// launches, the same in a recording and in its replay.  When the shorter one is known to
+// be free, only the rest of the longer one is traced (the final shading's rays: 15.14 ->
+// 14.84 ms).
 __device__ __forceinline__ float shadow_test_pl(Ctx& c, uint32_t idx, bool minus, V3 o, V3 d, float tmax) {
     Memo* m = c.m;
+    float tmin = SHADOW_TMIN;
     if (m) {
         if (!minus && m->pla_idx == idx) return memo_answer(c, m->pla_code);
         for (uint32_t j = 0; j < m->n_pl; j++)
-            if (m->pl_idx[j] == idx && (minus || m->pl_code[j] == MEMO_KNOWN)) return memo_answer(c, m->pl_code[j]);
+            if (m->pl_idx[j] == idx) {
+                if (minus || m->pl_code[j] == MEMO_KNOWN) return memo_answer(c, m->pl_code[j]);
+                if (m->pl_code[j] == (MEMO_KNOWN | 1u)) tmin = fmax_(tmin, tmax - PL_SHORTER);
+            }
         if (minus && m->pla_idx == idx && m->pla_code == (MEMO_KNOWN | 1u)) return memo_answer(c, m->pla_code);
     }
     const uint32_t k = c.k;
-    const float r = shadow_test(c, o, d, tmax);
+    const float r = shadow_test(c, o, d, tmax, tmin);
     c.last = k;
     if (m && c.k == k + 1) {
         if (!minus) { m->pla_idx = idx; m->pla_code = k; }
@@ -416,7 +423,7 @@ __device__ __forceinline__ void combine(Ctx& c, Reservoir& cur, const Reservoir&
         } else {
             V3 lp = load3(L.pos);
             float ld = length(sub(lp, sh.biased));
-            vis = shadow_test_pl(c, nb.pl_idx, true, sh.biased, divs(sub(lp, sh.biased), ld), ld - 0.001f);
+            vis = shadow_test_pl(c, nb.pl_idx, true, sh.biased, divs(sub(lp, sh.biased), ld), ld - PL_SHORTER);
         }
         float p_hat = len * vis;
         float w = (p_hat * (float)nb.pl_m) * nb.w_pl;

@@ -307,8 +307,7 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
             }
             if (sv0) {   // (the origin's w carries the bits of the contribution entry)
                 const size_t e = b0 + (uint32_t)__popc(m0 & lt);
-                F.shadow_rays[2 * e] = make_float4(so.x, so.y, so.z, __uint_as_float((uint32_t)shadow_entry(F, i, 0)));
-                F.shadow_rays[2 * e + 1] = make_float4(S.dir_light.dir[0], S.dir_light.dir[1], S.dir_light.dir[2], T_FAR);
+                F.shadow_rays[e] = make_float4(so.x, so.y, so.z, __uint_as_float((uint32_t)shadow_entry(F, i, 0)));
             }
             if (sv1) {
                 const size_t e = (size_t)F.n_paths + b1 + (uint32_t)__popc(m1 & lt);

@@ -63,9 +63,9 @@ struct FrameParams {
     HitDev* hits;
     float4* beta;            // per path
     float4* L;               // per path radiance
-    float4* shadow_rays;     // compacted shadow-ray queue of a segment, 2 float4 per ray: (origin, bits of its
-                             // contribution entry), (direction, tmax); directional-light rays from 0,
-                             // local-light rays from n_paths (counts in CNT_SHADOW_Q)
+    float4* shadow_rays;     // compacted shadow-ray queue of a segment (counts in CNT_SHADOW_Q): from 0 a float4
+                             // per directional-light ray, (origin, bits of its contribution entry); from
+                             // 2 n_paths two per local-light ray, the same and (direction, tmax)
     float4* shadow_contrib;  // 1 per shadow entry (shadow_entry): contribution, w = visibility (0: none)
     uint32_t* counters;
     unsigned long long* trav_counters;   // closest: [0] nodes [1] triangles; shadow: [2] [3]

@@ -413,13 +413,12 @@ SNK_HD bool intersect_tri(const WRay& r, V3 org, const float* v0, const float* v
         W = (float)((double)Bx * (double)Ay - (double)By * (double)Ax);
 #endif
     }
-    if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
+    const bool out = (U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f);
     float det = SNK_ADD(SNK_ADD(U, V), W);
-    if (det == 0.0f) return false;
     float Az = SNK_MUL(r.Sz, Akz), Bz = SNK_MUL(r.Sz, Bkz), Cz = SNK_MUL(r.Sz, Ckz);
     float T = SNK_ADD(SNK_ADD(SNK_MUL(U, Az), SNK_MUL(V, Bz)), SNK_MUL(W, Cz));
     float t = SNK_DIV(T, det);
-    if (!(t > tmin && t < tmax)) return false;
+    if (out || det == 0.0f || !(t > tmin && t < tmax)) return false;
     *t_out = t;
     *b1_out = SNK_DIV(V, det);
     *b2_out = SNK_DIV(W, det);

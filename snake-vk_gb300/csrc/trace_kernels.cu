@@ -59,9 +59,8 @@ template <class TV>
 __device__ __forceinline__ bool warp_step(TV& tv, bool active, const SceneDev& S, TraceCounters* ctr,
                                           uint32_t prim_bias) {
     if (active) tv.settle();
-    const bool live = active && !tv.done;
-    const unsigned want_prim = __ballot_sync(0xFFFFFFFFu, live && tv.has_prim());
-    const unsigned want_node = __ballot_sync(0xFFFFFFFFu, live && tv.has_node());
+    const unsigned want_prim = __ballot_sync(0xFFFFFFFFu, active && tv.has_prim());   // (a finished ray has neither)
+    const unsigned want_node = __ballot_sync(0xFFFFFFFFu, active && tv.has_node());
     const bool prims = 4u * (uint32_t)__popc(want_prim) >= prim_bias * (uint32_t)__popc(want_node);
     const uint32_t lane = threadIdx.x & 31u;
     if (prims) {

@@ -86,7 +86,6 @@ __device__ __forceinline__ void res_store(void* base, uint32_t i, const Reservoi
 // queue being recorded.
 constexpr uint32_t MEMO_KNOWN = 0x100;  // answer code: MEMO_KNOWN | visibility, else a slot of the current queue
 constexpr uint32_t MEMO_NONE = 0xFFFF;  // plan code of a test that was not made
-constexpr float PL_SHORTER = 0.001f;    // a combine tests a point light at its distance - PL_SHORTER
 constexpr int MEMO_PL = 4, MEMO_EM = 4;
 // Tests already made for this pixel and frame, by what they aim at: the point
 // light tested at its full distance, point lights tested at distance - 0.001,
@@ -126,21 +125,22 @@ __device__ __forceinline__ void ctx_queue(Ctx& c, const RestirQueue& q, uint32_t
     c.cap = q.per_pixel;
 }
 
-// marks the slots a recording pass left unused as empty (tmax < 0)
+// marks the slots a recording pass left unused as empty
 __device__ __forceinline__ void ctx_close(Ctx& c) {
     if (!c.rays) return;
-    for (uint32_t k = c.k; k < c.cap; k++) c.rays[2 * (c.base + k * c.stride) + 1] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+    for (uint32_t k = c.k; k < c.cap; k++) c.rays[c.base + k * c.stride] = make_float4(0.0f, 0.0f, 0.0f, VIS_EMPTY);
 }
 
-// 1 when the segment is unoccluded (recording: always 1, the value is not used
-// for anything the replay would see differently)
-__device__ __forceinline__ float shadow_test(Ctx& c, V3 o, V3 d, float tmax, float tmin = SHADOW_TMIN) {
+// 1 when the segment from the pixel's biased surface point is unoccluded (recording:
+// always 1, the value is not used for anything the replay would see differently); end: only
+// its last PL_SHORTER.  A segment of no length is unoccluded.
+__device__ __forceinline__ float shadow_test(Ctx& c, V3 d, float tmax, bool end = false) {
     if (c.k >= c.cap) { c.overflow = true; return 0.0f; }
     const size_t slot = c.base + (size_t)c.k++ * c.stride;
     if (c.rays) {
         c.shadow_rays++;
-        c.rays[2 * slot] = make_float4(o.x, o.y, o.z, tmin);
-        c.rays[2 * slot + 1] = make_float4(d.x, d.y, d.z, tmax);
+        const float t = fmax_(tmax, 0.0f);
+        c.rays[slot] = make_float4(d.x, d.y, d.z, end ? -t : t);
         return 1.0f;
     }
     return c.vis[slot] ? 1.0f : 0.0f;
@@ -162,20 +162,20 @@ __device__ __forceinline__ float memo_answer(Ctx& c, uint32_t code) {
 // launches, the same in a recording and in its replay.  When the shorter one is known to
 // be free, only the rest of the longer one is traced (the final shading's rays: 15.14 ->
 // 14.84 ms).
-__device__ __forceinline__ float shadow_test_pl(Ctx& c, uint32_t idx, bool minus, V3 o, V3 d, float tmax) {
+__device__ __forceinline__ float shadow_test_pl(Ctx& c, uint32_t idx, bool minus, V3 d, float tmax) {
     Memo* m = c.m;
-    float tmin = SHADOW_TMIN;
+    bool end = false;
     if (m) {
         if (!minus && m->pla_idx == idx) return memo_answer(c, m->pla_code);
         for (uint32_t j = 0; j < m->n_pl; j++)
             if (m->pl_idx[j] == idx) {
                 if (minus || m->pl_code[j] == MEMO_KNOWN) return memo_answer(c, m->pl_code[j]);
-                if (m->pl_code[j] == (MEMO_KNOWN | 1u)) tmin = fmax_(tmin, tmax - PL_SHORTER);
+                if (m->pl_code[j] == (MEMO_KNOWN | 1u)) end = true;
             }
         if (minus && m->pla_idx == idx && m->pla_code == (MEMO_KNOWN | 1u)) return memo_answer(c, m->pla_code);
     }
     const uint32_t k = c.k;
-    const float r = shadow_test(c, o, d, tmax, tmin);
+    const float r = shadow_test(c, d, tmax, end);
     c.last = k;
     if (m && c.k == k + 1) {
         if (!minus) { m->pla_idx = idx; m->pla_code = k; }
@@ -185,7 +185,7 @@ __device__ __forceinline__ float shadow_test_pl(Ctx& c, uint32_t idx, bool minus
 }
 
 // shadow test toward an emissive sample, reusing an identical earlier test of this pixel
-__device__ __forceinline__ float shadow_test_em(Ctx& c, uint4 key, V3 o, V3 d, float tmax) {
+__device__ __forceinline__ float shadow_test_em(Ctx& c, uint4 key, V3 d, float tmax) {
     Memo* m = c.m;
     if (m)
         for (uint32_t j = 0; j < m->n_em; j++) {
@@ -193,7 +193,7 @@ __device__ __forceinline__ float shadow_test_em(Ctx& c, uint4 key, V3 o, V3 d, f
             if (e.x == key.x && e.y == key.y && e.z == key.z && e.w == key.w) return memo_answer(c, m->em_code[j]);
         }
     const uint32_t k = c.k;
-    const float r = shadow_test(c, o, d, tmax);
+    const float r = shadow_test(c, d, tmax);
     c.last = k;
     if (m && c.k == k + 1 && m->n_em < MEMO_EM) {
         m->em_key[m->n_em] = key;
@@ -308,7 +308,7 @@ __device__ __forceinline__ float tri_shadow(Ctx& c, uint32_t inst, uint32_t tri,
     V3 target = add(p, mul(pn, 0.01f));
     float dist = length(sub(surface_pos, target));
     V3 dir = divs(sub(target, surface_pos), dist);
-    return shadow_test_em(c, key_em(inst, tri, bu, bv), surface_pos, dir, dist);
+    return shadow_test_em(c, key_em(inst, tri, bu, bv), dir, dist);
 }
 
 // ComputeTriangleRadiance without the shadow test: emission of instance inst
@@ -374,7 +374,7 @@ __device__ __forceinline__ V3 tri_radiance(Ctx& c, uint32_t inst, uint32_t tri, 
     V3 target = add(p, mul(pn, 0.01f));
     float dist = length(sub(sh.biased, target));
     V3 dir = divs(sub(target, sh.biased), dist);
-    return mul(rad, shadow_test_em(c, key_em(inst, tri, bu, bv), sh.biased, dir, dist));
+    return mul(rad, shadow_test_em(c, key_em(inst, tri, bu, bv), dir, dist));
 }
 
 // a test whose result changes nothing, in the recording and in the replaying run alike
@@ -417,13 +417,13 @@ __device__ __forceinline__ void combine(Ctx& c, Reservoir& cur, const Reservoir&
             skip_test(c);
         } else if (!FIXED && len * (float)nb.pl_m <= 3.0e38f) {
             // nb's weight is 0 unless its light is free at the full distance, as it then is at the shorter one
-            vis = shadow_test_pl(c, nb.pl_idx, false, none, none, 0.0f);
+            vis = shadow_test_pl(c, nb.pl_idx, false, none, 0.0f);
         } else if (use) {
-            vis = shadow_test_pl(c, nb.pl_idx, true, none, none, 0.0f);
+            vis = shadow_test_pl(c, nb.pl_idx, true, none, 0.0f);
         } else {
             V3 lp = load3(L.pos);
             float ld = length(sub(lp, sh.biased));
-            vis = shadow_test_pl(c, nb.pl_idx, true, sh.biased, divs(sub(lp, sh.biased), ld), ld - PL_SHORTER);
+            vis = shadow_test_pl(c, nb.pl_idx, true, divs(sub(lp, sh.biased), ld), ld - PL_SHORTER);
         }
         float p_hat = len * vis;
         float w = (p_hat * (float)nb.pl_m) * nb.w_pl;
@@ -438,7 +438,7 @@ __device__ __forceinline__ void combine(Ctx& c, Reservoir& cur, const Reservoir&
         V3 rad;
         if (use) {
             const V3 un = v3(cv.y, cv.z, cv.w);
-            rad = mul(un, needed(un) ? shadow_test_em(c, key_em(nb.em_inst, nb.em_tri, nb.em_u, nb.em_v), none, none, 0.0f)
+            rad = mul(un, needed(un) ? shadow_test_em(c, key_em(nb.em_inst, nb.em_tri, nb.em_u, nb.em_v), none, 0.0f)
                                      : 0.0f);
         } else {
             rad = tri_radiance(c, nb.em_inst, nb.em_tri, nb.em_u, nb.em_v, sh, [&](V3 un) {
@@ -629,6 +629,7 @@ __global__ void __launch_bounds__(RBLK, 8) k_restir_initial(FrameParams F, uint3
             float4 gn = R.g_normal[o], ga = R.g_albedo[o], gm = R.g_misc[o];
             V3 nrm = v3(gn.x, gn.y, gn.z);
             Shade sh = shade_of(V.v, v3(gp.x, gp.y, gp.z), nrm, v3(ga.x, ga.y, ga.z), ga.w, gm.x);
+            if (record) R.origin[o] = make_float4(sh.biased.x, sh.biased.y, sh.biased.z, 0.0f);
             // the RIS result of k_restir_ris: reservoir, target values and stream position
             Reservoir Rr = res_load(R.temporal, o);
             const float4 ra = R.ris[2ull * o], rb = R.ris[2ull * o + 1];
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(RBLK, 8) k_restir_initial(FrameParams F, uint3
             if (Rr.pl_idx != INVALID) {
                 V3 lp = load3(S.point_lights[Rr.pl_idx].pos);
                 float dist = length(sub(lp, sh.biased));
-                float vis = shadow_test_pl(c, Rr.pl_idx, false, sh.biased, divs(sub(lp, sh.biased), dist), dist);
+                float vis = shadow_test_pl(c, Rr.pl_idx, false, divs(sub(lp, sh.biased), dist), dist);
                 Rr.w_pl = vis * ((Rr.w_sum_pl / (float)Rr.pl_m) / phat_pl);
             } else {
                 Rr.w_pl = 0.0f;
@@ -788,7 +789,7 @@ __global__ void __launch_bounds__(RBLK, 8) k_restir_spatial(FrameParams F, uint3
                 V3 cdl = calc_directional(load3(S.dir_light.dir), load3(S.dir_light.colour), sh.v, sh.f0, sh.n, sh.rough,
                                           sh.metal, sh.albedo);
                 const bool lit = !(cdl.x == 0.0f && cdl.y == 0.0f && cdl.z == 0.0f);
-                light = mul(cdl, lit ? shadow_test(c, sh.biased, load3(S.dir_light.dir), 1000.0f) : 0.0f);
+                light = mul(cdl, lit ? shadow_test(c, load3(S.dir_light.dir), 1000.0f) : 0.0f);
                 if (!lit) skip_test(c);
             }
             Reservoir Rr;
@@ -844,7 +845,7 @@ __global__ void __launch_bounds__(RBLK, 8) k_restir_spatial(FrameParams F, uint3
                 V3 cpl = calc_pointlight(L, sh.v, sh.f0, sh.ro, sh.n, sh.rough, sh.metal, sh.albedo);
                 float vis;
                 if (phase == 1) {
-                    vis = shadow_test_pl(c, Rr.pl_idx, false, sh.biased, divs(sub(lp, sh.biased), ld), ld);
+                    vis = shadow_test_pl(c, Rr.pl_idx, false, divs(sub(lp, sh.biased), ld), ld);
                     code_pl = c.last;
                 } else {
                     vis = plan_vis(c, plan & 0xFFFFu);

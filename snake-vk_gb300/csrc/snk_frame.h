@@ -129,10 +129,13 @@ cudaError_t launch_trace_closest(const FrameParams& F, uint32_t depth, int grid,
 cudaError_t launch_trace_shadow(const FrameParams& F, uint32_t depth, int grid, bool count, cudaStream_t s);
 cudaError_t launch_trace_rays(const SceneDev& S, const float4* rays, uint32_t n, HitDev* hits, bool any,
                               uint32_t* work_counter, int grid, const TraceTuning& tune, cudaStream_t s);
-// vis[i] = 1 when segment i (origin, tmin | direction, tmax) is unoccluded, 0 when it
-// is not; an empty entry (tmax < 0) is skipped and its vis[i] left as it was
-cudaError_t launch_trace_visibility(const SceneDev& S, const float4* rays, uint32_t n, uint8_t* vis,
-                                    uint32_t* work_counter, int grid, const TraceTuning& tune, cudaStream_t s);
+// vis[i] = 1 when the segment of entry i (RestirQueue; pixel i % pixels) is unoccluded, 0
+// when it is not; an empty entry is skipped and its vis[i] left as it was
+cudaError_t launch_trace_visibility(const SceneDev& S, const float4* rays, const float4* origin, uint32_t pixels,
+                                    uint32_t n, uint8_t* vis, uint32_t* work_counter, int grid,
+                                    const TraceTuning& tune, cudaStream_t s);
+constexpr float PL_SHORTER = 0.001f;    // a ReSTIR combine tests a point light at its distance - PL_SHORTER
+constexpr float VIS_EMPTY = -3.4e38f;
 
 // ReSTIR DI state of one view
 struct RestirView {
@@ -146,6 +149,7 @@ struct RestirView {
     void* spatial;      // final reservoirs of this frame
     float4* ris;        // 2 per pixel: the initial pass's RIS state between its two runs
     uint4* memo_keys;   // 4 per pixel: the initial pass's visibility tests and their results
+    float4* origin;     // per surface pixel: origin of its visibility rays (the biased surface point)
     uint32_t* plan;     // per pixel: how the final shading's two tests are answered (codes, 16 bits each)
     float4* combo;      // unshadowed combine targets, slot-major (slot * pixels + pixel): the temporal
                         // pass's RESTIR_TEMPORAL_COMBOS slots, then the spatial pass's 1 + spatial
@@ -164,8 +168,10 @@ struct RestirSettings {
 };
 
 // Visibility rays of a ReSTIR pass: `per_pixel` slots for each of the view's
-// `pixels` pixels, slot-major: slot k of pixel p is entry k * pixels + p, whose
-// ray is 2 float4 (origin, tmin | direction, tmax) at rays[2 * entry].  Slot k
+// `pixels` pixels, slot-major: slot k of pixel p is entry k * pixels + p, one float4
+// (direction, tmax); all of a pixel's rays start at RestirView::origin and at SHADOW_TMIN,
+// but for those with a negative tmax: the last PL_SHORTER of a segment of length -tmax.
+// VIS_EMPTY as tmax marks an unused slot.  Slot k
 // of neighbouring pixels is written, traced and read together.  A pass either
 // records its rays into `rays` or replays their results from `vis`.
 struct RestirQueue {

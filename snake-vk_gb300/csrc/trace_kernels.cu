@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256) k_accum_shadow(FrameParams F, uint32_t d)
     }
 }
 
-// Ray feed over a queue with empty entries (tmax < 0): the warp takes 32 entries
+// Ray feed over a queue with empty entries (VIS_EMPTY): the warp takes 32 entries
 // at a time from the work counter, keeps the real ones in a per-warp ring in
 // shared memory and hands only those to its idle lanes, so an empty entry costs
 // one 4-byte load instead of a lane's turn.
@@ -355,7 +355,7 @@ struct FilteredFeed {
         const uint32_t nidle = (uint32_t)__popc(idle), lt = (1u << lane) - 1u;
         while (cnt < nidle && !raw.done()) {   // (cnt < 32 here, so the ring of 64 never overflows)
             const uint32_t e = raw.refill(0xFFFFFFFFu, lane, work, n, kn);
-            const bool real = e != INVALID && __ldg(reinterpret_cast<const float*>(rays + 2ull * e + 1) + 3) >= 0.0f;
+            const bool real = e != INVALID && __ldg(reinterpret_cast<const float*>(rays + e) + 3) > VIS_EMPTY;
             const unsigned rm = __ballot_sync(0xFFFFFFFFu, real);
             if (real) ring[(head + cnt + (uint32_t)__popc(rm & lt)) & 63u] = e;
             cnt += (uint32_t)__popc(rm);
@@ -373,16 +373,18 @@ struct FilteredFeed {
     __device__ __forceinline__ bool done() const { return raw.done() && cnt == 0; }
 };
 
-// visibility of a queue of segments: vis[i] = 1 when nothing is hit in (tmin, tmax),
-// 0 when something is; entries with tmax < 0 are empty (skipped, vis[i] not written:
-// the passes never read the result of a slot they did not record).
+// visibility of a queue of segments (RestirQueue): vis[i] = 1 when nothing is hit in (tmin,
+// tmax), 0 when something is; empty entries are skipped, vis[i] not written:
+// the passes never read the result of a slot they did not record.  Origins are kept once
+// per pixel (recip: 2^32 / pixels): the recording passes are bound by the slots' bytes.
 // The ReSTIR passes queue their visibility rays here instead of tracing inline.  (No
 // eight-lane end: these queues are long and their rays short, two 1080p ReSTIR frames
 // took 17.38 ms with it and 17.02 without.)
 template <int MINB, bool SINGLE>
 __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(const __grid_constant__ SceneDev S, const float4* __restrict__ rays,
-                                                                 uint32_t n, uint8_t* vis, uint32_t* work,
-                                                                 TraceTuning tune) {
+                                                                 const float4* __restrict__ origin, uint32_t pixels,
+                                                                 uint32_t recip, uint32_t n, uint8_t* vis,
+                                                                 uint32_t* work, TraceTuning tune) {
     using TV = Traverser<true, false, SINGLE>;
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     __shared__ uint32_t ring[TBLK / 32][64];
@@ -395,8 +397,12 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(const __grid_co
         [&](unsigned idle) { return feed.refill(idle, lane, work, n, kn, rays, ring[threadIdx.x >> 5]); },
         [&] { return feed.done(); },
         [&](TV& tv, uint32_t i, uint2* spill) {
-            const float4 a = __ldg(rays + 2ull * i), b = __ldg(rays + 2ull * i + 1);
-            tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
+            uint32_t o = i - __umulhi(i, recip) * pixels;   // i % pixels, or that + pixels
+            o = o >= pixels ? o - pixels : o;
+            const float4 b = __ldg(rays + i), a = __ldg(origin + o);
+            const float t = fabsf(b.w);
+            tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), b.w < 0.0f ? fmaxf(SHADOW_TMIN, t - PL_SHORTER) : SHADOW_TMIN,
+                    t, sh_stack, spill, threadIdx.x, TBLK);
             return i;
         },
         [&](const TraceResult& r, uint32_t ri) { vis[ri] = r.hit ? 0u : 1u; });
@@ -470,16 +476,18 @@ cudaError_t launch_trace_shadow(const FrameParams& F, uint32_t depth, int grid, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_trace_visibility(const SceneDev& S, const float4* rays, uint32_t n, uint8_t* vis, uint32_t* work,
-                                    int grid, const TraceTuning& tune, cudaStream_t s) {
+cudaError_t launch_trace_visibility(const SceneDev& S, const float4* rays, const float4* origin, uint32_t pixels,
+                                    uint32_t n, uint8_t* vis, uint32_t* work, int grid, const TraceTuning& tune,
+                                    cudaStream_t s) {
+    const uint32_t recip = pixels > 1u ? (uint32_t)(0x100000000ull / pixels) : 0xFFFFFFFFu;
     if (S.single_leaf) {
-        if (tune.variant == 1) k_trace_visibility<8, true><<<grid, TBLK, 0, s>>>(S, rays, n, vis, work, tune);
-        else if (tune.variant == 2) k_trace_visibility<4, true><<<grid, TBLK, 0, s>>>(S, rays, n, vis, work, tune);
-        else k_trace_visibility<6, true><<<grid, TBLK, 0, s>>>(S, rays, n, vis, work, tune);
+        if (tune.variant == 1) k_trace_visibility<8, true><<<grid, TBLK, 0, s>>>(S, rays, origin, pixels, recip, n, vis, work, tune);
+        else if (tune.variant == 2) k_trace_visibility<4, true><<<grid, TBLK, 0, s>>>(S, rays, origin, pixels, recip, n, vis, work, tune);
+        else k_trace_visibility<6, true><<<grid, TBLK, 0, s>>>(S, rays, origin, pixels, recip, n, vis, work, tune);
     } else {
-        if (tune.variant == 1) k_trace_visibility<8, false><<<grid, TBLK, 0, s>>>(S, rays, n, vis, work, tune);
-        else if (tune.variant == 2) k_trace_visibility<4, false><<<grid, TBLK, 0, s>>>(S, rays, n, vis, work, tune);
-        else k_trace_visibility<6, false><<<grid, TBLK, 0, s>>>(S, rays, n, vis, work, tune);
+        if (tune.variant == 1) k_trace_visibility<8, false><<<grid, TBLK, 0, s>>>(S, rays, origin, pixels, recip, n, vis, work, tune);
+        else if (tune.variant == 2) k_trace_visibility<4, false><<<grid, TBLK, 0, s>>>(S, rays, origin, pixels, recip, n, vis, work, tune);
+        else k_trace_visibility<6, false><<<grid, TBLK, 0, s>>>(S, rays, origin, pixels, recip, n, vis, work, tune);
     }
     return cudaGetLastError();
 }

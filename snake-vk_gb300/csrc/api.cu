@@ -97,6 +97,7 @@ struct snk_pt_ctx {
     DBuf<unsigned> d_err;              // [0] the device error word, [1] work counter of the ray queries
     DBuf<unsigned char> q_in, q_in2, q_out, q_out2;   // staging of the particle / contact queries
     DBuf<float4> rq_rays, rq_origin;                   // ReSTIR visibility queue (slots x pixels), origins (pixels)
+    DBuf<uint8_t> rq_counts;                           // slots in use (pixels)
     DBuf<uint8_t> rq_vis_a, rq_vis_b;                  // its results (initial / shading, spatial)
     DBuf<uint32_t> rq_work;                            // work counters of the three visibility traces
     UploadMemo memo[7];                // raw instances, emissive firsts, emissive list, -, -, -, BVH list
@@ -1333,7 +1334,7 @@ int render_impl(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, cons
             s.radius = rs.restir_radius; s.pad = 0;
             // visibility queues: initial (K1 slots per pixel), spatial (K2), final shading (K3)
             const uint32_t K1 = RESTIR_INITIAL_SLOTS, K2 = restir_spatial_slots(s.spatial), K3 = RESTIR_SHADE_SLOTS;
-            if (ctx->rq_rays.reserve((size_t)std::max(K1, K2) * np) || ctx->rq_origin.reserve(np) ||
+            if (ctx->rq_rays.reserve((size_t)std::max(K1, K2) * np) || ctx->rq_origin.reserve(np) || ctx->rq_counts.reserve(np) ||
                 ctx->rq_vis_a.reserve(std::max(K1, K3) * np) ||
                 ctx->rq_vis_b.reserve((size_t)K2 * np) || ctx->rq_work.reserve(3))
                 return fail(ctx, SNK_ERR_OUT_OF_MEMORY, "restir visibility queues");
@@ -1341,8 +1342,9 @@ int render_impl(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, cons
             if (cudaMemsetAsync(ctx->rq_work.p, 0, 3 * sizeof(uint32_t), st) != cudaSuccess)
                 return fail(ctx, SNK_ERR_CUDA, "restir queue reset");
             RV.origin = ctx->rq_origin.p;
-            const RestirQueue q1{ctx->rq_rays.p, ctx->rq_vis_a.p, K1, (uint32_t)np},
-                q2{ctx->rq_rays.p, ctx->rq_vis_b.p, K2, (uint32_t)np}, q3{ctx->rq_rays.p, ctx->rq_vis_a.p, K3, (uint32_t)np};
+            const RestirQueue q1{ctx->rq_rays.p, ctx->rq_vis_a.p, ctx->rq_counts.p, K1, (uint32_t)np},
+                q2{ctx->rq_rays.p, ctx->rq_vis_b.p, ctx->rq_counts.p, K2, (uint32_t)np},
+                q3{ctx->rq_rays.p, ctx->rq_vis_a.p, ctx->rq_counts.p, K3, (uint32_t)np};
             const SceneDev SD = scene_dev(ctx);
             const TraceTuning tt = any_tuning(ctx);
             const int ta = any_grid(ctx);
@@ -1352,7 +1354,7 @@ int render_impl(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, cons
             };
             auto visibility = [&](uint32_t K, uint8_t* vis, int slot) {
                 return staged(ctx, profile, SNK_STAGE_TRACE_SHADOW, [&] {
-                    return launch_trace_visibility(SD, ctx->rq_rays.p, RV.origin, (uint32_t)np, (uint32_t)(K * np), vis, ctx->rq_work.p + slot,
+                    return launch_trace_visibility(SD, ctx->rq_rays.p, RV.origin, ctx->rq_counts.p, (uint32_t)np, (uint32_t)(K * np), vis, ctx->rq_work.p + slot,
                                                    ta, tt, st);
                 });
             };

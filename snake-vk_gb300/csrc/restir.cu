@@ -108,6 +108,7 @@ struct Ctx {
                             // when recording)
     float4* rays;           // recording
     const uint8_t* vis;     // replaying
+    uint8_t* counts;
     size_t base;            // the pixel: slot k is entry base + k * stride
     size_t stride;          // pixels of the view
     uint32_t k, cap;
@@ -119,16 +120,17 @@ struct Ctx {
 __device__ __forceinline__ void ctx_queue(Ctx& c, const RestirQueue& q, uint32_t pixel, bool record) {
     c.rays = record ? q.rays : nullptr;
     c.vis = record ? nullptr : q.vis;
+    c.counts = q.counts;
     c.base = pixel;
     c.stride = q.pixels;
     c.k = 0;
     c.cap = q.per_pixel;
 }
 
-// marks the slots a recording pass left unused as empty
+// how many slots a recording pass has used
 __device__ __forceinline__ void ctx_close(Ctx& c) {
     if (!c.rays) return;
-    for (uint32_t k = c.k; k < c.cap; k++) c.rays[c.base + k * c.stride] = make_float4(0.0f, 0.0f, 0.0f, VIS_EMPTY);
+    c.counts[c.base] = (uint8_t)c.k;
 }
 
 // 1 when the segment from the pixel's biased surface point is unoccluded (recording:

@@ -129,13 +129,12 @@ cudaError_t launch_trace_closest(const FrameParams& F, uint32_t depth, int grid,
 cudaError_t launch_trace_shadow(const FrameParams& F, uint32_t depth, int grid, bool count, cudaStream_t s);
 cudaError_t launch_trace_rays(const SceneDev& S, const float4* rays, uint32_t n, HitDev* hits, bool any,
                               uint32_t* work_counter, int grid, const TraceTuning& tune, cudaStream_t s);
-// vis[i] = 1 when the segment of entry i (RestirQueue; pixel i % pixels) is unoccluded, 0
-// when it is not; an empty entry is skipped and its vis[i] left as it was
-cudaError_t launch_trace_visibility(const SceneDev& S, const float4* rays, const float4* origin, uint32_t pixels,
-                                    uint32_t n, uint8_t* vis, uint32_t* work_counter, int grid,
+// vis[i] = 1 when the segment of entry i (RestirQueue; slot i / pixels of pixel i % pixels)
+// is unoccluded, 0 when it is not; an entry not in use is skipped and its vis[i] left as it was
+cudaError_t launch_trace_visibility(const SceneDev& S, const float4* rays, const float4* origin, const uint8_t* counts,
+                                    uint32_t pixels, uint32_t n, uint8_t* vis, uint32_t* work_counter, int grid,
                                     const TraceTuning& tune, cudaStream_t s);
 constexpr float PL_SHORTER = 0.001f;    // a ReSTIR combine tests a point light at its distance - PL_SHORTER
-constexpr float VIS_EMPTY = -3.4e38f;
 
 // ReSTIR DI state of one view
 struct RestirView {
@@ -171,12 +170,13 @@ struct RestirSettings {
 // `pixels` pixels, slot-major: slot k of pixel p is entry k * pixels + p, one float4
 // (direction, tmax); all of a pixel's rays start at RestirView::origin and at SHADOW_TMIN,
 // but for those with a negative tmax: the last PL_SHORTER of a segment of length -tmax.
-// VIS_EMPTY as tmax marks an unused slot.  Slot k
+// A pixel uses its first counts[p] slots.  Slot k
 // of neighbouring pixels is written, traced and read together.  A pass either
 // records its rays into `rays` or replays their results from `vis`.
 struct RestirQueue {
     float4* rays;
     const uint8_t* vis;
+    uint8_t* counts;
     uint32_t per_pixel;
     uint32_t pixels;
 };

@@ -46,3 +46,20 @@ def test_tests_that_change_nothing(cuda, built_lib, case):
         s = pt.stats()
         assert s["rays_shadow"] + s["shadow_tests_reused"] == int(ctr[2])
         assert s["device_error"] == 0
+
+
+# entries of the visibility queue are split into slot and pixel: the smallest views and odd numbers of pixels
+@pytest.mark.parametrize("W,H,spatial", [(1, 1, 3), (2, 1, 32), (5, 3, 1), (31, 7, 3), (64, 33, 5)])
+def test_small_views(cuda, built_lib, W, H, spatial):
+    sc = scenes.config2(width=W, height=H, frames=2)
+    pt = snkpt.PathTracer(0)
+    pt.load_scene(sc)
+    ors = O.OracleRestir(O.OracleScene(sc), W, H)
+    for f in range(2):
+        st = abi.settings(mode=abi.MODE_RESTIR_DI, frame_index=f, seed=5, restir_spatial=spatial)
+        g = _gpu_frame(pt, [sc.views[f]], st, cuda)[0]
+        ctr = np.zeros(5, np.uint64)
+        r, _ = ors.frame(sc.views[f], st, counters=ctr)
+        _compare(g, r, f"{W}x{H}, frame {f}")
+        s = pt.stats()
+        assert s["rays_shadow"] + s["shadow_tests_reused"] == int(ctr[2]) and s["device_error"] == 0

@@ -174,14 +174,16 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
             float4 so = make_float4(0, 0, 0, 0), sd1 = so;
             float4 q0, q1, q2, q3, qb;
             if (have) {
+                // (loads that depend on the entry or the path alone go first)
                 p = F.path_ids[cur][i];
+                const float4 rd4 = F.rays[cur][2ull * i + 1];
+                const HitDev h = F.hits[i];
+                const float4 b4 = FIRST ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : F.beta[p];
+                const V3 rd = v3(rd4.x, rd4.y, rd4.z);
                 uint32_t gpix, s, vi, x, y;
                 const bool train = decode_path(F, p, &gpix, &s, &vi, &x, &y);
                 const ViewDev& V = F.views[vi];
                 const uint32_t o = y * V.v.width + x;
-                float4 rd4 = F.rays[cur][2ull * i + 1];
-                V3 rd = v3(rd4.x, rd4.y, rd4.z);
-                HitDev h = F.hits[i];
                 Pcg rng = pcg_stream(gpix, s, d, frame_seed(F));
                 if (FIRST) { pcg_next(rng); pcg_next(rng); }
                 const bool gbuf = FIRST && s == 0 && !train;
@@ -197,7 +199,6 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
                     float u_sel = pcg_float(rng), u1 = pcg_float(rng), u2 = pcg_float(rng);
                     float u_rr = pcg_float(rng), u_d1 = pcg_float(rng), u_d2 = pcg_float(rng);
                     float u_lobe = pcg_float(rng);
-                    const float4 b4 = FIRST ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : F.beta[p];
                     V3 beta = v3(b4.x, b4.y, b4.z);
                     bool to_cache = false;
                     if (CACHE) {

@@ -15,10 +15,10 @@ constexpr uint32_t MAX_VIEWS = 64;
 // different parts of the scene, so that a packet visits every ray's nodes and the longest
 // packets end late; and a few packets leave SMs idle.  Frames of two segments, packets
 // and ray by ray: a room of 2,120 triangles (line at 55,000 rays) with 128x72 pixels
-// 157 and 141 us, 320x180 173 and 179, 640x360 244 and 265, 3840x2160 4273 and 4469;
-// spheres and a terrain tile of 387,000 (747,000 rays) 960x540 739 and 649 us, 720p 927
-// and 916, 1080p 1558 and 1654; 64 tiles of 8.6 million (3.5 million rays) 720p 2104 and
-// 1809 us, 1080p 3591 and 3491, 1440p 5715 and 5789, 3840x2160 11516 and 12266.  With
+// 152 and 139 us, 320x180 165 and 178, 640x360 232 and 259, 3840x2160 3970 and 4190;
+// spheres and a terrain tile of 387,000 (747,000 rays) 960x540 672 and 603 us, 720p 857
+// and 856, 1080p 1420 and 1520; 64 tiles of 8.6 million (3.5 million rays) 720p 1926 and
+// 1643 us, 1080p 3251 and 3148, 1440p 5153 and 5195, 3840x2160 10385 and 11028.  With
 // a line at 1280x720 for all scenes a 256x256 room frame of depth 4 took 303 us (296 now),
 // a 1080p terrain frame with the radiance cache 3.91 ms (3.67).  (Packets that hand their
 // tile over to the ray-by-ray kernel after 64 to 512 steps, or when few rays share

@@ -196,7 +196,8 @@ __device__ __forceinline__ void karras_node(int i, const unsigned long long* __r
 // start within the digit.  As it stores an element it counts the element's next digit
 // for the tile it lands in, so a pass needs no counting or scanning launch of its own.
 // Bound by latency at the sizes of a scene: tiles of 1024 put 131,072 elements on 128
-// SMs (tiles of 4096 and three launches per digit before).
+// SMs, nine launches of about 9 us for 132,352 keys of two trees (tiles of 4096 and three
+// launches per digit took 24 launches and 185 us).
 constexpr int SORT_THREADS = 1024;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
 constexpr int SORT_RADIX = 256;
@@ -317,12 +318,14 @@ __global__ void __launch_bounds__(SORT_THREADS, 1) k_sort_pass(const unsigned lo
 }
 
 // One tree of up to SORT_BITONIC_MAX primitives is sorted by one CTA in shared
-// memory with a bitonic network (66 barrier-separated compare-exchange stages for
-// 2048 entries, one launch instead of eight).  The network is not
+// memory with a bitonic network (78 barrier-separated compare-exchange stages for
+// 4096 entries, one launch instead of eight).  The network is not
 // stable by itself, so it orders by (key, value): the values are the primitives'
 // indices 0..n-1 in their input order, which makes the result the stable order.
-// Entries past n are padded with the largest pair.
-constexpr uint32_t SORT_BITONIC_MAX = 2048;
+// Entries past n are padded with the largest pair.  Rebuilding the BVH of 1,100 instances
+// took 187 us with the network and 204 with the radix sort, 2,048 202 and 242, 3,000 240
+// and 252, 4,096 246 and 252; a network of 8,192 has 91 stages of twice the work.
+constexpr uint32_t SORT_BITONIC_MAX = 4096;
 
 __global__ void __launch_bounds__(SORT_THREADS, 1) k_sort_bitonic(unsigned long long* keys, uint32_t* vals,
                                                                 uint32_t n) {

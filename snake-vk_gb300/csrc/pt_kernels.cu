@@ -137,9 +137,9 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
             bool hit = false;
             if (i < n) {
                 hit = F.hits[i].flags != 0u;
-                if (!hit) {   // no shadow rays: zero contributions
-                    F.shadow_contrib[shadow_entry(F, i, 0)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    F.shadow_contrib[shadow_entry(F, i, 1)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (!hit) {   // no shadow rays, no contributions
+                    shadow_vis(F)[shadow_entry(F, i, 0)] = 0u;
+                    shadow_vis(F)[shadow_entry(F, i, 1)] = 0u;
                     if (FIRST) {
                         uint32_t gpix, s, vi, x, y;
                         const bool train = decode_path(F, F.path_ids[cur][i], &gpix, &s, &vi, &x, &y);
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
                     } else if (sf.flags & MAT_EMISSIVE) {
                         if (FIRST && direct && !train) {   // as a visible contribution (a training path's is not used)
                             const V3 c = cmul(beta, sf.albedo);
-                            F.shadow_contrib[shadow_entry(F, i, 0)] = make_float4(c.x, c.y, c.z, 1.0f);
+                            F.shadow_contrib[shadow_entry(F, i, 0)] = make_float4(c.x, c.y, c.z, 0.0f);
                             emits = true;
                         }
                     } else {
@@ -277,10 +277,9 @@ __global__ void __launch_bounds__(BLK, 4) k_shade(FrameParams F, uint32_t d) {
                     }
                 }
             }
-            if (have) {   // zero contribution: no shadow ray of that kind
-                const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (!sv0 && !emits) F.shadow_contrib[shadow_entry(F, i, 0)] = z;
-                if (!sv1) F.shadow_contrib[shadow_entry(F, i, 1)] = z;
+            if (have) {   // without a shadow ray (which writes it): no contribution, or a visible one
+                if (!sv0) shadow_vis(F)[shadow_entry(F, i, 0)] = emits ? 1u : 0u;
+                if (!sv1) shadow_vis(F)[shadow_entry(F, i, 1)] = 0u;
             }
             // warp-ballot compaction of the continuing paths into the next queue and of
             // the shadow rays into their kinds' parts of the shadow queue

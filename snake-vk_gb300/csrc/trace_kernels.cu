@@ -256,8 +256,8 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_packet(FrameParams F, uint
 // shadow rays of segment d: the compacted queue's n0 directional-light rays (origins
 // only: the eight-view terrain batch 36.38 -> 36.26 ms), then its n1 local-light rays
 // (from ray n_paths on).  A ray's origin w holds its
-// contribution entry (shadow_entry); the visibility goes to that contribution's w
-// component, and k_accum_shadow adds the visible contributions in entry order
+// contribution entry (shadow_entry); the visibility goes to that entry's byte
+// (shadow_vis), and k_accum_shadow adds the visible contributions in entry order
 // (the same order as the CPU oracle, so sums are bit-identical).
 template <bool COUNT, int MINB, bool SINGLE>
 __global__ void __launch_bounds__(TBLK, MINB) k_trace_shadow(const __grid_constant__ FrameParams F, uint32_t d) {
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_shadow(const __grid_consta
             tv.init(F.S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), SHADOW_TMIN, b.w, sh_stack, spill, threadIdx.x, TBLK);
             return __float_as_uint(a.w);
         },
-        [&](const TraceResult& r, uint32_t ri) { F.shadow_contrib[ri].w = r.hit ? 0.0f : 1.0f; });
+        [&](const TraceResult& r, uint32_t ri) { shadow_vis(F)[ri] = r.hit ? 0u : 1u; });
     flush_counts<COUNT>(ctr, F.trav_counters ? F.trav_counters + 2 : nullptr);
 }
 
@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(256) k_accum_shadow(FrameParams F, uint32_t d)
     const uint32_t n = F.counters[CNT_QUEUE + d];
     const uint32_t* pids = F.path_ids[d & 1u];
     for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
-        float4 c0 = F.shadow_contrib[shadow_entry(F, i, 0)], c1 = F.shadow_contrib[shadow_entry(F, i, 1)];
-        const bool add = c0.w != 0.0f || c1.w != 0.0f;
+        const bool v0 = shadow_vis(F)[shadow_entry(F, i, 0)] != 0u, v1 = shadow_vis(F)[shadow_entry(F, i, 1)] != 0u;
+        const bool add = v0 || v1;
         uint32_t p = 0;
         bool fin = false;   // (early resolve) the path ends in this segment
         if (F.early_resolve) {
@@ -314,9 +314,11 @@ __global__ void __launch_bounds__(256) k_accum_shadow(FrameParams F, uint32_t d)
             p = pids[i];
         }
         if (!add && !fin && d) continue;
-        float4 l = d ? F.L[p] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (c0.w != 0.0f) l = make_float4(l.x + c0.x, l.y + c0.y, l.z + c0.z, 0.0f);
-        if (c1.w != 0.0f) l = make_float4(l.x + c1.x, l.y + c1.y, l.z + c1.z, 0.0f);
+        float4 l = d ? F.L[p] : make_float4(0.0f, 0.0f, 0.0f, 0.0f), c0 = l, c1 = l;
+        if (v0) c0 = F.shadow_contrib[shadow_entry(F, i, 0)];
+        if (v1) c1 = F.shadow_contrib[shadow_entry(F, i, 1)];
+        if (v0) l = make_float4(l.x + c0.x, l.y + c0.y, l.z + c0.z, 0.0f);
+        if (v1) l = make_float4(l.x + c1.x, l.y + c1.y, l.z + c1.z, 0.0f);
         if (fin) {   // the pixel's outputs, as the resolve pass writes them for one sample
             const uint32_t vi = find_view(F.views, F.nviews, p);   // (one sample: path p is pixel p)
             const ViewDev& V = F.views[vi];
@@ -335,8 +337,8 @@ __global__ void __launch_bounds__(256) k_accum_shadow(FrameParams F, uint32_t d)
         if (F.cache && p >= F.n_render) {   // radiance gathered at this vertex of a training path
             const uint32_t slot = (p - F.n_render) * TRAIN_V + (d < TRAIN_V - 1 ? d : TRAIN_V - 1);
             float4 v = F.train_L[slot];
-            if (c0.w != 0.0f) v = make_float4(v.x + c0.x, v.y + c0.y, v.z + c0.z, 0.0f);
-            if (c1.w != 0.0f) v = make_float4(v.x + c1.x, v.y + c1.y, v.z + c1.z, 0.0f);
+            if (v0) v = make_float4(v.x + c0.x, v.y + c0.y, v.z + c0.z, 0.0f);
+            if (v1) v = make_float4(v.x + c1.x, v.y + c1.y, v.z + c1.z, 0.0f);
             F.train_L[slot] = v;
         }
     }

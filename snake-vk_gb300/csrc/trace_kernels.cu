@@ -220,7 +220,10 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_closest(const __grid_const
             tv.init(F.S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), a.w, b.w, sh_stack, spill, threadIdx.x, TBLK);
             return i;
         },
-        [&](const TraceResult& r, uint32_t ri) { store_hit(F.hits + ri, r); });
+        [&](const TraceResult& r, uint32_t ri) {
+            if (r.hit) store_hit(F.hits + ri, r);
+            else F.hits[ri].flags = 0u;   // (all that is read of a miss)
+        });
     flush_counts<COUNT>(ctr, F.trav_counters);
 }
 
@@ -249,7 +252,8 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_packet(FrameParams F, uint
         tv.run(F.S);
         TraceResult r;
         tv.finish(F.S, r);
-        if (active) store_hit(F.hits + i, r);
+        if (active && r.hit) store_hit(F.hits + i, r);
+        if (active && !r.hit) F.hits[i].flags = 0u;
     }
 }
 

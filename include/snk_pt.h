@@ -281,7 +281,8 @@ typedef struct snk_tuning {
     uint32_t ray_chunk;             /* most rays a warp takes per global work fetch (64); fewer near the end
                                        of a queue and of a small one */
     uint32_t refill_idle;           /* hand new rays to a warp when this many lanes idle (4) */
-    uint32_t prim_bias;             /* warp runs a primitive step if 4*n_prim >= bias*n_node (3) */
+    uint32_t prim_bias;             /* warp runs a primitive step if 4*n_prim >= bias*n_node (3; ReSTIR
+                                       visibility rays 2) */
     uint32_t trace_variant;         /* registers: 0 <= 85 (6 blocks/SM), 1 <= 64, 2 unconstrained */
     uint32_t bvh_treelet_passes;    /* treelet restructuring passes of later mesh BVH builds (3);
                                        SNK_TREELET_PASSES_NONE builds the plain LBVH */

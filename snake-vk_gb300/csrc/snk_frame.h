@@ -45,7 +45,7 @@ static_assert(sizeof(HitDev) == 24, "hit layout");
 struct TraceTuning {
     uint32_t chunk;        // most rays a warp takes per global fetch (default 64)
     uint32_t refill_idle;  // refill a warp when at least this many lanes are idle (default 4)
-    uint32_t prim_bias;    // primitive step when 4 * n_prim >= prim_bias * n_node (default 3)
+    uint32_t prim_bias;    // primitive step when 4 * n_prim >= prim_bias * n_node (default 3; visibility 2)
     uint32_t variant;      // registers: 0 <= 85 (6 blocks / SM), 1 <= 64 (8 blocks), 2 unconstrained
     uint32_t warps;        // warps resident on the GPU with that variant (set by the host)
 };

@@ -36,9 +36,9 @@ struct Knobs {
     float share;      // chunk per ray left
     int refill_idle;
     uint32_t prim_bias;
-    __device__ __forceinline__ Knobs(const TraceTuning& t, uint32_t n)
+    __device__ __forceinline__ Knobs(const TraceTuning& t, uint32_t n, uint32_t bias = 3u)
         : chunk(t.chunk ? t.chunk : CHUNK_MAX), share(0.25f / (float)t.warps),
-          refill_idle(t.refill_idle ? (int)t.refill_idle : 4), prim_bias(t.prim_bias ? t.prim_bias : 3u) {
+          refill_idle(t.refill_idle ? (int)t.refill_idle : 4), prim_bias(t.prim_bias ? t.prim_bias : bias) {
         const uint32_t c = (uint32_t)((float)n * (16.0f * share));
         chunk_min = min(max(c, 1u), min(CHUNK_MIN, chunk));
         few = n <= (uint32_t)COOP_RAYS * t.warps ? max((n + t.warps - 1u) / t.warps, 1u) : 0u;
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(const __grid_co
     using TV = Traverser<true, false, SINGLE>;
     __shared__ uint2 sh_stack[TRACE_SH_ROWS * TBLK];
     __shared__ uint32_t ring[TBLK / 32][64];
-    const Knobs kn(tune, n);
+    const Knobs kn(tune, n, 2u);   // (few triangles a ray: two ReSTIR frames 13.59 ms, 13.68 with 3, 13.62 with 1)
     const uint32_t lane = threadIdx.x & 31u;
     FilteredFeed feed;
     feed.init();

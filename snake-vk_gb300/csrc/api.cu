@@ -1383,8 +1383,8 @@ int render_impl(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, cons
             };
             auto visibility = [&](uint32_t K, uint8_t* vis, int slot) {
                 return staged(ctx, profile, SNK_STAGE_TRACE_SHADOW, [&] {
-                    return launch_trace_visibility(SD, ctx->rq_rays.p, RV.origin, ctx->rq_counts.p, (uint32_t)np, (uint32_t)(K * np), vis, ctx->rq_work.p + slot,
-                                                   ta, tt, st);
+                    return launch_trace_visibility(SD, ctx->rq_rays.p, RV.origin, ctx->rq_counts.p, (uint32_t)np,
+                                                   (uint32_t)(K * np), vis, ctx->rq_work.p + slot, ta, tt, st);
                 });
             };
             // (the first shading pass wrote the G-buffer and the surface records)

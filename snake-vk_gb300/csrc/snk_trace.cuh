@@ -25,6 +25,7 @@
 // warp (PacketTraverser, below), with the same results.
 #pragma once
 #include "snk_device.cuh"
+#include "snk_lane_stack.h"
 
 namespace snk {
 
@@ -506,7 +507,7 @@ __device__ __noinline__ void coop_trace(CoopSlot* slots, uint32_t k_rays, const 
             if (!tv.has_node() && !tv.has_prim()) {
                 if (tv.level == 1 && tv.st.sp == tv.blas_sp) { tv.level = 0; tv.restore_world(); }
                 if (tv.st.sp == 0) break;
-                const uint2 e = entry(g, --tv.st.sp);
+                const uint2 e = lanes_pop<uint2>([&](int k) { return entry(g, k); }, tv.st.sp, [&] { __syncwarp(gm); });
                 if (e.x & PRIM_GROUP) tv.tgroup = make_uint2(e.x & ~PRIM_GROUP, e.y);
                 else tv.ngroup = e;
                 continue;
@@ -617,8 +618,7 @@ __device__ __noinline__ void coop_trace(CoopSlot* slots, uint32_t k_rays, const 
 // most.  Hits equal the per-ray traversal's: boxes only cull, and the closest hit
 // is the minimum over the tested triangles in the same (t, instance, triangle)
 // order.  The group stack is one array of PSTACK entries (base, bits, lane mask)
-// per warp in shared memory; every lane writes the same values, so each lane
-// reads back what it wrote itself.  Each lane's world ray and its node-test
+// per warp in shared memory (lanes_pop).  Each lane's world ray and its node-test
 // set-up wait in shared-memory rows while the lane's ray is in an instance.  For
 // single-primitive-leaf trees only.  A packet that runs past its stack or past
 // 32x the per-ray step cap reports the same error bits as a ray would (all its
@@ -797,7 +797,7 @@ struct PacketTraverser {
             if (tgroup.y <= 0x00FFFFFFu && ngroup.y <= 0x00FFFFFFu) {
                 if (level == 1 && sp == blas_sp) { level = 0; restore_world(); coct = woct; }
                 if (sp == 0) return;
-                const uint4 g = stk[--sp];
+                const uint4 g = lanes_pop<uint4>([&](int k) { return stk[k]; }, sp, [] { __syncwarp(); });
                 if (g.x & PRIM_GROUP) { tgroup = make_uint2(g.x & ~PRIM_GROUP, g.y); tmask = g.z; }
                 else { ngroup = make_uint2(g.x, g.y); nmask = g.z; }
             }

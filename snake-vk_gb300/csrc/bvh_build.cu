@@ -1854,8 +1854,9 @@ __device__ __forceinline__ float reach(const MeshExtents& E, const float* n) {
 // reaches along the box's own directions (26 object-space extents: a rotated mesh that
 // does not fill its box gets a box of its own size, not of the box's corners; a
 // sphere's is 1.1 to 1.2 instead of up to 1.7 times its diameter), with 1 % of the extent
-// to spare for the roundings of the object-space ray (0.1 % to spare gave 0.3 % more on
-// the terrain, 5 % to spare took 1 % back).  A ray that enters an instance and leaves it
+// and 1e-5 of the mesh's coordinates to spare for the roundings of the object-space ray
+// (0.1 % of the extent to spare gave 0.3 % more on the terrain, 5 % to spare took 1 %
+// back).  A ray that enters an instance and leaves it
 // without a hit costs its transform and a walk from the mesh's root: over 4,097 turned
 // spheres, a 1920x1080 path-traced frame 1.997 -> 1.918 ms, one with reservoirs 16.98 ->
 // 16.40 ms, 2^20 device rays 370 -> 347 us; the eight-view terrain (19.2 Mpx) 2.3 % less
@@ -1881,7 +1882,13 @@ __global__ void k_instance_boxes(const uint32_t* __restrict__ list, uint32_t n, 
     for (int a = 0; a < 3; a++) {
         const float up[3] = {I.m[4 * a], I.m[4 * a + 1], I.m[4 * a + 2]}, down[3] = {-up[0], -up[1], -up[2]};
         const float zl = r[a] - reach(E, down), zh = r[a] + reach(E, up);
-        const float spare = 0.01f * (zh - zl);
+        // the extent's share, and what the object-space ray may be off by: its roundings (and
+        // ref's) are some ten of 2^-24 of the mesh's coordinates, which the world box need not
+        // show when the translation takes them back; 1e-5 of them, as the triangles' boxes have
+        // that the corners' box is made of
+        float at = 0.0f;
+        for (int k = 0; k < 3; k++) at += fabsf(up[k]) * fmaxf(fabsf(M.lo[k]), fabsf(M.hi[k]));
+        const float spare = 0.01f * (zh - zl) + 1e-5f * at;
         if (zl - spare > l[a]) l[a] = zl - spare;   // (false for a NaN: the corners' box stays)
         if (zh + spare < h[a]) h[a] = zh + spare;
     }

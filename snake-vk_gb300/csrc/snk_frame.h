@@ -178,7 +178,8 @@ struct RestirSettings {
 // Visibility rays of a ReSTIR pass: `per_pixel` slots for each of the view's
 // `pixels` pixels, slot-major: slot k of pixel p is entry k * pixels + p, one float4
 // (direction, tmax); all of a pixel's rays start at RestirView::origin and at SHADOW_TMIN,
-// but for those with a negative tmax: the last PL_SHORTER of a segment of length -tmax.
+// but for those with a negative tmax: the last PL_SHORTER of a segment of length -tmax,
+// from its end of the shorter segment on.
 // A pixel uses its first counts[p] slots.  Slot k
 // of neighbouring pixels is written, traced and read together.  A pass either
 // records its rays into `rays` or replays their results from `vis`.

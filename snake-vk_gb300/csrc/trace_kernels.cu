@@ -393,6 +393,14 @@ struct FilteredFeed {
     __device__ __forceinline__ bool done() const { return raw.done() && cnt == 0; }
 };
 
+// Where the rest of a segment of length t starts whose first t - PL_SHORTER is free: one
+// float below that, since a test takes neither of its ends and a hit at t - PL_SHORTER is in
+// the whole segment (of a difference of 0 that makes a NaN, of a negative one a negative
+// one: SHADOW_TMIN).
+__device__ __forceinline__ float end_tmin(float t) {
+    return fmaxf(SHADOW_TMIN, __uint_as_float(__float_as_uint(t - PL_SHORTER) - 1u));
+}
+
 // visibility of a queue of segments (RestirQueue): vis[i] = 1 when nothing is hit in (tmin,
 // tmax), 0 when something is; entries not in use are skipped, vis[i] not written:
 // the passes never read the result of a slot they did not record.  Origins are kept once
@@ -424,8 +432,8 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(const __grid_co
             slot_of(i, pixels, recip, &o);
             const float4 b = __ldg(rays + i), a = __ldg(origin + o);
             const float t = fabsf(b.w);
-            tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), b.w < 0.0f ? fmaxf(SHADOW_TMIN, t - PL_SHORTER) : SHADOW_TMIN,
-                    t, sh_stack, spill, threadIdx.x, TBLK);
+            tv.init(S, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), b.w < 0.0f ? end_tmin(t) : SHADOW_TMIN, t, sh_stack, spill,
+                    threadIdx.x, TBLK);
             return i;
         },
         [&](const TraceResult& r, uint32_t ri) { vis[ri] = r.hit ? 0u : 1u; });

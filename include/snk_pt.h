@@ -302,7 +302,10 @@ typedef struct snk_tuning {
                                        (bvh_leaf_max..4; default bvh_leaf_max) */
     uint32_t max_traversal_steps;   /* traversal units (node groups and primitives) one ray may take;
                                        a ray that needs more stops and the next synchronising call
-                                       returns SNK_ERR_LIMIT (0: 65536) */
+                                       returns SNK_ERR_LIMIT (0: 65536).  Below the default of this or
+                                       the next limit every ray is traced by itself; with both
+                                       defaults, packets of rays count theirs in common and rays with
+                                       eight lanes a leaf's primitives as one */
     uint32_t stack_limit;           /* traversal stack entries per ray, 1..64; a deeper stack stops
                                        the ray with SNK_ERR_LIMIT (0: 64) */
     uint32_t shadow_blocks_per_sm;  /* any-hit traversal (shadow and ReSTIR visibility rays): grid =

@@ -678,8 +678,12 @@ int any_grid(snk_pt_ctx* ctx) {
 uint32_t resident_warps(snk_pt_ctx* ctx, uint32_t variant) {
     return (uint32_t)ctx->num_sms * 4u * (variant == 1 ? 8u : (variant == 2 ? 4u : 6u));
 }
+// the bounds of a ray's traversal are the defaults (packets and eight-lane rays, whose steps
+// and entries are not a single ray's, need that)
+bool default_limits(const SceneDev& S) { return S.max_steps == MAX_TRAVERSAL_STEPS && S.stack_max >= STACK_MAX; }
 TraceTuning trace_tuning(snk_pt_ctx* ctx) {
     TraceTuning t;
+    t.default_limits = default_limits(scene_dev(ctx)) ? 1u : 0u;
     t.chunk = ctx->tune.ray_chunk;
     t.refill_idle = ctx->tune.refill_idle;
     t.prim_bias = ctx->tune.prim_bias;
@@ -1118,8 +1122,7 @@ int render_impl(snk_pt_ctx* ctx, const snk_view* views, uint32_t num_views, cons
     F.n_pixels = (uint32_t)n_pixels;
     // camera packets: every view large for its scene, single-primitive leaves, the default
     // traversal bounds (their limits are per ray) and no counting of traversal work
-    F.packet_primary = F.S.single_leaf && !(rs.flags & SNK_RENDER_COUNT_NODES) &&
-                       F.S.max_steps == MAX_TRAVERSAL_STEPS && F.S.stack_max >= STACK_MAX;
+    F.packet_primary = F.S.single_leaf && !(rs.flags & SNK_RENDER_COUNT_NODES) && default_limits(F.S);
     for (uint32_t v = 0; v < num_views; v++) {
         const uint32_t w = views[v].width, h = views[v].height;
         const double rays = (double)((uint64_t)w * h * spp);

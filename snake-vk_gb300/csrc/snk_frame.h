@@ -48,6 +48,7 @@ struct TraceTuning {
     uint32_t prim_bias;    // primitive step when 4 * n_prim >= prim_bias * n_node (default 3; visibility 2)
     uint32_t variant;      // registers: 0 <= 85 (6 blocks / SM), 1 <= 64 (8 blocks), 2 unconstrained
     uint32_t warps;        // warps resident on the GPU with that variant (set by the host)
+    uint32_t default_limits;   // the traversal's step and stack limits are the defaults (set by the host)
 };
 
 struct FrameParams {

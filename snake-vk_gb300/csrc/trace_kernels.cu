@@ -32,16 +32,17 @@ constexpr uint32_t CHUNK_MAX = 64, CHUNK_MIN = 32;
 
 struct Knobs {
     uint32_t chunk, chunk_min;
+    bool coop;        // a warp's last rays may get eight lanes each
     uint32_t few;     // rays per warp of a queue of at most COOP_RAYS rays per resident warp, else 0
     float share;      // chunk per ray left
     int refill_idle;
     uint32_t prim_bias;
     __device__ __forceinline__ Knobs(const TraceTuning& t, uint32_t n, uint32_t bias = 3u)
-        : chunk(t.chunk ? t.chunk : CHUNK_MAX), share(0.25f / (float)t.warps),
+        : chunk(t.chunk ? t.chunk : CHUNK_MAX), coop(t.default_limits != 0u), share(0.25f / (float)t.warps),
           refill_idle(t.refill_idle ? (int)t.refill_idle : 4), prim_bias(t.prim_bias ? t.prim_bias : bias) {
         const uint32_t c = (uint32_t)((float)n * (16.0f * share));
         chunk_min = min(max(c, 1u), min(CHUNK_MIN, chunk));
-        few = n <= (uint32_t)COOP_RAYS * t.warps ? max((n + t.warps - 1u) / t.warps, 1u) : 0u;
+        few = coop && n <= (uint32_t)COOP_RAYS * t.warps ? max((n + t.warps - 1u) / t.warps, 1u) : 0u;
     }
     // eight lanes per ray from the start: a warp takes `few` rays at a time
     __device__ __forceinline__ void take_few() { chunk = chunk_min = few; }
@@ -121,7 +122,9 @@ struct RayFeed {
 // them has taken COOP_STEPS steps: such a ray has a long way behind it and likely more to
 // go, and the queue's end waits for it (short rays, as in a closed room, finish sooner
 // where they are: a 65,536-path room frame 304 us, 328 with all last rays moved).  So do
-// all rays of a queue that gives the resident warps no more than COOP_RAYS each.  The
+// all rays of a queue that gives the resident warps no more than COOP_RAYS each.  (Not with
+// limits of the caller's: eight lanes take a leaf's triangles in one step and keep fewer
+// entries, so that it would depend on a ray's queue whether a limit is reported.)  The
 // 480x270 terrain batch took 1.43 instead of 1.55 ms so, a 480x270 sphere-field frame 0.54
 // and 0.58, a 1080p frame 2.005 and 2.037, 10,000 rays 112 and 129 us, 64 rays 73 and 83 us.
 constexpr uint32_t COOP_STEPS = 48;
@@ -173,7 +176,7 @@ __device__ __forceinline__ void trace_queue(const SceneDev& S, const Knobs& kn, 
                 if (act == 0) continue;
             } else if (act == 0) {
                 break;
-            } else if (COOP && __popc(act) <= COOP_RAYS &&
+            } else if (COOP && kn.coop && __popc(act) <= COOP_RAYS &&
                        __any_sync(0xFFFFFFFFu, active && tv.steps >= COOP_STEPS)) {
                 if (active) coop_save(coop_slots[threadIdx.x >> 5][rank(act)], tv, ri);
                 finish_few((uint32_t)__popc(act));

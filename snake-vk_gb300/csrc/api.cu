@@ -142,7 +142,7 @@ struct snk_pt_ctx {
     uint32_t accum_w = 0, accum_h = 0;
     uint64_t accum_frames = 0;
 
-    DBuf<unsigned char> tr_buf;        // rays (32 B each), then hits of a ray or contact query
+    DBuf<unsigned char> tr_buf;        // rays (32 B each), then hits of a ray query from the host
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool timing_pending = false;
@@ -1778,23 +1778,34 @@ T* stage_out(DBuf<unsigned char>& b, void* dst, size_t bytes, uint32_t memory, S
     if (b.reserve(bytes ? bytes : 1)) { *st = Status::Err(SNK_ERR_OUT_OF_MEMORY, "query staging"); return nullptr; }
     return reinterpret_cast<T*>(b.p);
 }
-// Scratch of a contact query of n items with `per` rays each; queries run in parts of at
-// most CONTACT_RAYS rays (enough to fill the GPU), which bounds it to 59 MB.
-constexpr uint32_t CONTACT_RAYS = 1u << 20;
-Status contact_scratch(snk_pt_ctx* ctx, uint32_t n, uint32_t per, bool own_rays, ContactScratch* c) {
-    const size_t rays = std::min<size_t>((size_t)n * per, CONTACT_RAYS);
-    const size_t ray_bytes = own_rays ? rays * sizeof(snk_ray) : 0;
-    SNK_TRY_CUDA(ctx->tr_buf.reserve(ray_bytes + rays * sizeof(HitDev)));
-    *c = ContactScratch{reinterpret_cast<float4*>(ctx->tr_buf.p), reinterpret_cast<HitDev*>(ctx->tr_buf.p + ray_bytes),
-                        ctx->d_err.p + 1, trace_grid(ctx), trace_tuning(ctx)};
+// Scratch of a contact query of items with `per` rays each, in parts of at most CONTACT_RAYS
+// rays (enough to fill the GPU): memory that the mesh build has left (SCRATCH_BYTES), so that
+// a query allocates nothing, whatever its size and the sizes before it.  (An allocation
+// of its own took 110 us of a context's first query, 330 us for 100,000 particles, and with its exact
+// size again in every step of a system that grows.)  A scene without such a build makes
+// the scratch here; where there is no room for it, the parts are smaller.
+constexpr uint32_t CONTACT_RAYS = 1u << 20, CONTACT_RAYS_MIN = 1u << 10;
+static_assert(CONTACT_RAYS * (sizeof(snk_ray) + sizeof(HitDev)) <= SCRATCH_BYTES, "a part's rays and hits");
+Status contact_scratch(snk_pt_ctx* ctx, uint32_t per, bool own_rays, ContactScratch* c) {
+    DBuf<float>& mem = ctx->scratch.wide_cost;
+    const size_t per_ray = sizeof(HitDev) + (own_rays ? sizeof(snk_ray) : 0);
+    uint32_t rays = CONTACT_RAYS;
+    cudaError_t e;
+    while ((e = mem.reserve(rays * per_ray / sizeof(float))) == cudaErrorMemoryAllocation && rays > CONTACT_RAYS_MIN) {
+        cudaGetLastError();   // (the launches that follow ask for the last error)
+        rays >>= 1;
+    }
+    SNK_TRY_CUDA(e);
+    unsigned char* p = reinterpret_cast<unsigned char*>(mem.p);
+    *c = ContactScratch{reinterpret_cast<float4*>(p), reinterpret_cast<HitDev*>(p + rays * (per_ray - sizeof(HitDev))),
+                        rays / per, ctx->d_err.p + 1, trace_grid(ctx), trace_tuning(ctx)};
     return Status::Ok();
 }
-// calls part(first, count) over [0, n) in parts of at most CONTACT_RAYS / per items
+// calls part(first, count) over [0, n) in the parts that the scratch is made for
 template <class Fn>
-cudaError_t in_parts(uint32_t n, uint32_t per, Fn&& part) {
+cudaError_t in_parts(uint32_t n, const ContactScratch& c, Fn&& part) {
     cudaError_t e = cudaSuccess;
-    for (uint64_t b = 0; b < n && e == cudaSuccess; b += CONTACT_RAYS / per)
-        e = part((uint32_t)b, std::min(n - (uint32_t)b, CONTACT_RAYS / per));
+    for (uint64_t b = 0; b < n && e == cudaSuccess; b += c.items) e = part((uint32_t)b, std::min(n - (uint32_t)b, c.items));
     return e;
 }
 Status download(snk_pt_ctx* ctx, void* dst, const void* src, size_t bytes, uint32_t memory) {
@@ -1817,8 +1828,8 @@ int snk_pt_contact_rays(snk_pt_ctx* ctx, const snk_ray* rays, uint32_t n, float 
     ContactOut* d_out = stage_out<ContactOut>(ctx->q_out, out, sizeof(snk_contact) * (size_t)n, memory, &st);
     if (!st.ok()) return fail(ctx, st);
     ContactScratch sc;
-    API_TRY(contact_scratch(ctx, n, 1, false, &sc));
-    const cudaError_t e = in_parts(n, 1, [&](uint32_t b, uint32_t cnt) {
+    API_TRY(contact_scratch(ctx, 1, false, &sc));
+    const cudaError_t e = in_parts(n, sc, [&](uint32_t b, uint32_t cnt) {
         return launch_contact_rays(scene_dev(ctx), d_rays + 2ull * b, cnt, timestep, d_out + b, sc, ctx->stream);
     });
     if (e != cudaSuccess) return fail(ctx, SNK_ERR_CUDA, std::string("contact_rays: ") + cudaGetErrorString(e));
@@ -1841,8 +1852,8 @@ int snk_pt_particle_probe(snk_pt_ctx* ctx, const snk_particle* particles, uint32
     float* d_g = stage_out<float>(ctx->q_out2, gravity_dv, sizeof(float) * (size_t)n, memory, &st);
     if (!st.ok()) return fail(ctx, st);
     ContactScratch sc;
-    API_TRY(contact_scratch(ctx, n, 4, true, &sc));
-    const cudaError_t e = in_parts(n, 4, [&](uint32_t b, uint32_t cnt) {
+    API_TRY(contact_scratch(ctx, 4, true, &sc));
+    const cudaError_t e = in_parts(n, sc, [&](uint32_t b, uint32_t cnt) {
         return launch_particle_probe(scene_dev(ctx), d_p + b, cnt, timestep, d_c + b, d_g + b, sc, ctx->stream);
     });
     if (e != cudaSuccess) return fail(ctx, SNK_ERR_CUDA, std::string("particle_probe: ") + cudaGetErrorString(e));
@@ -1866,8 +1877,8 @@ int snk_pt_particle_constrain(snk_pt_ctx* ctx, const snk_particle* particles, co
     float* d_out = stage_out<float>(ctx->q_out, out, 3 * sizeof(float) * (size_t)n, memory, &st);
     if (!st.ok()) return fail(ctx, st);
     ContactScratch sc;
-    API_TRY(contact_scratch(ctx, n, 1, true, &sc));
-    const cudaError_t e = in_parts(n, 1, [&](uint32_t b, uint32_t cnt) {
+    API_TRY(contact_scratch(ctx, 1, true, &sc));
+    const cudaError_t e = in_parts(n, sc, [&](uint32_t b, uint32_t cnt) {
         return launch_particle_constrain(scene_dev(ctx), d_p + b, d_off + 3ull * b, cnt, timestep, d_out + 3ull * b, sc,
                                          ctx->stream);
     });

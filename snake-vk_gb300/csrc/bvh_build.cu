@@ -2004,7 +2004,10 @@ Status build_wide_bvhs(BuildScratch& sc, const float4* prim_lo, const float4* pr
     }
     const uint32_t* wide_split = nullptr;
     if (sah_collapse) {   // SAH-optimal choice of each wide node's children over the final binary trees
-        SNK_TRY_CUDA(sc.wide_cost.reserve(8 * (size_t)n));
+        if (sc.wide_cost.reserve(std::max(8 * (size_t)n, SCRATCH_BYTES / sizeof(float))) != cudaSuccess) {
+            cudaGetLastError();
+            SNK_TRY_CUDA(sc.wide_cost.reserve(8 * (size_t)n));
+        }
         SNK_TRY_CUDA(sc.wide_split.reserve(n));
         if (boxes)
             k_collapse_cost<false><<<g, BLK, 0, st>>>((int)n, sorted, prim_lo, prim_hi, sc.children.p, sc.parent.p,

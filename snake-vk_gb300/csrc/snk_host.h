@@ -64,6 +64,9 @@ struct Status {
     } while (0)
 
 // ---- BVH builder ---------------------------------------------------------------
+// Least size of BuildScratch::wide_cost: what a part of a contact query needs.  (An
+// allocation of 59 MB takes no longer than one of 4.)
+constexpr size_t SCRATCH_BYTES = 56ull << 20;
 struct BuildScratch {
     DBuf<unsigned long long> keys, keys_alt;
     DBuf<uint32_t> vals, vals_alt;
@@ -78,7 +81,8 @@ struct BuildScratch {
     DBuf<uint32_t> sort_hist;     // per-tile digit counts of the radix sort, every digit
     DBuf<double> sah;             // SAH accumulator
     DBuf<uint32_t> level_tasks;   // task count per wide level
-    DBuf<float> wide_cost;        // 8 per binary internal node: SAH cost of its subtree in 1..8 wide children
+    DBuf<float> wide_cost;        // 8 per binary internal node: SAH cost of its subtree in 1..8 wide children;
+                                  // between builds the scratch of the contact queries (SCRATCH_BYTES)
     DBuf<uint32_t> wide_split;    // per binary internal node: the split of those children (4-bit fields)
 };
 

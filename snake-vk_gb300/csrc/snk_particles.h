@@ -18,6 +18,7 @@ static_assert(sizeof(ParticleDev) == 48 && sizeof(ContactOut) == 48, "particle r
 struct ContactScratch {
     float4* rays;
     HitDev* hits;
+    uint32_t items;   // of a part at most (particles, offsets or rays)
     uint32_t* work;
     int grid;
     TraceTuning tune;

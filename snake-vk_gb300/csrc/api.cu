@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstddef>
 #include <cstring>
+#include <exception>
 #include <map>
 #include <string>
 #include <vector>
@@ -845,8 +846,13 @@ int snk_pt_get_last_error(const snk_pt_ctx* ctx, char* buf, size_t len) {
 
 int snk_pt_upload_meshes(snk_pt_ctx* ctx, const snk_mesh* meshes, uint32_t num_meshes) {
     if (!ctx || (num_meshes && !meshes)) return fail(ctx, SNK_ERR_INVALID_ARG, "upload_meshes: null argument");
-    std::vector<HostMesh> hm(num_meshes);
+    std::vector<HostMesh> hm;
     size_t nv = 0, nt = 0;
+    try {
+        hm.resize(num_meshes);
+    } catch (const std::exception&) {
+        return fail(ctx, SNK_ERR_OUT_OF_MEMORY, "upload_meshes: host memory");
+    }
     for (uint32_t m = 0; m < num_meshes; m++) {
         const snk_mesh& M = meshes[m];
         if ((M.num_vertices && !M.positions) || (M.num_triangles && !M.indices))
@@ -862,13 +868,18 @@ int snk_pt_upload_meshes(snk_pt_ctx* ctx, const snk_mesh* meshes, uint32_t num_m
         nt += M.num_triangles;
     }
     // all meshes are valid: their arrays take the place of the old ones (one copy here, in
-    // the layout of the device buffers; the vectors keep their memory from load to load)
+    // the layout of the device buffers; the vectors keep their memory from load to load).
+    // Room for them comes first, so that without it the old ones are still there
+    try {
+        ctx->mesh_pos.reserve(3 * nv);
+        ctx->mesh_nrm.reserve(3 * nv);
+        ctx->mesh_idx.reserve(3 * nt);
+    } catch (const std::exception&) {
+        return fail(ctx, SNK_ERR_OUT_OF_MEMORY, "upload_meshes: host memory");
+    }
     ctx->mesh_pos.clear();
     ctx->mesh_nrm.clear();
     ctx->mesh_idx.clear();
-    ctx->mesh_pos.reserve(3 * nv);
-    ctx->mesh_nrm.reserve(3 * nv);
-    ctx->mesh_idx.reserve(3 * nt);
     for (uint32_t m = 0; m < num_meshes; m++) {
         const snk_mesh& M = meshes[m];
         const size_t v3 = 3ull * M.num_vertices;

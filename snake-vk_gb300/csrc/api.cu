@@ -1,5 +1,5 @@
 // api.cu -- the C ABI of include/snk_pt.h: context, scene upload, acceleration
-// structure builds, frame dispatch and the per-ray test hook.
+// structure builds, frame dispatch and the ray and contact queries.
 //
 // Reference boundary: class RT (Core/headers/rendering/Raytracing.h:11-31),
 // RT::Init / RT::RecordRenderCmdBuf (Core/src/rendering/Raytracing.cpp:227-278)

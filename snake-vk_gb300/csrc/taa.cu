@@ -159,9 +159,10 @@ __device__ __forceinline__ float4 resolve_pixel(const float4 cur4, const float* 
 // it points to, with 24 warps per SM to cover both, and runs some 570 instructions (the
 // exact divisions and square roots among them).  So a block asks L2 for the texels of
 // one that runs later, neither index needs a division, and the bounds take three
-// operands at a time: a 1080p resolve 43 us, 50 before (49 without the prefetch), 88 B per
-// pixel at 4.2 TB/s.  (Two pixels per thread need 126 registers and were slower, as were
-// 512-thread blocks; 64 registers changed nothing.)
+// operands at a time: a 1080p resolve whose images are partly in L2 43 us, 50 before (49
+// without the prefetch); after an L2 flush 60 us, 72 before, 88 B per pixel at 3.0 TB/s.  (Two
+// pixels per thread need 126 registers and were slower, as were 512-thread blocks; 64
+// registers changed nothing.)
 __global__ void __launch_bounds__(TX * TY) k_taa_resolve(TaaImages I) {
     __shared__ float4 tile[TY + 2][TX + 2];   // clamped to >= 0, as the neighbourhood takes it
     const int bx = blockIdx.x * TX, by = blockIdx.y * TY;

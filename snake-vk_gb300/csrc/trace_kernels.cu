@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(TBLK, MINB) k_trace_visibility(const __grid_co
         [&](const TraceResult& r, uint32_t ri) { vis[ri] = r.hit ? 0u : 1u; });
 }
 
-// generic trace of an array of rays (the snk_pt_trace_rays test hook)
+// trace of an array of rays: snk_pt_trace_rays, and the rays of the particle and contact queries
 template <bool ANY, bool SINGLE>
 __global__ void __launch_bounds__(TBLK, 6) k_trace_rays(const __grid_constant__ SceneDev S, const float4* __restrict__ rays, uint32_t n,
                                                      HitDev* hits, uint32_t* work, TraceTuning tune) {
